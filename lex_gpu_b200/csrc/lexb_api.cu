@@ -1595,6 +1595,32 @@ static bool is_pinned(const void* p) {
     return at.type == cudaMemoryTypeHost;
 }
 
+// May the call go in parts?  Part 0 of y is stored and copied out before the last part of x is copied in, so nothing the call
+// writes (x_dev, y_dev, y_host) may meet anything else it touches, in host memory or on the device (one address space:
+// a buffer may wrap mapped host memory).  r and y_dev as one buffer stay in parts: a part reads its own tokens of r only.
+// A stream that is being captured keeps the one copy, launch and copy (the wait then fails as it always did).
+static bool host_parts_apply(const lexb_gpu* g, const lexb_pipeline* p, const void* x_host, const lexb_buffer* x_dev, const lexb_buffer* wq,
+                             const lexb_buffer* ws, const lexb_buffer* wg, const lexb_buffer* r, const lexb_buffer* y_dev, const void* y_host) {
+    if (!p->host_part || p->gpu != g || x_dev->gpu != g || y_dev->gpu != g || !wq || !ws || !wg || g->d_trace) return false;
+    const size_t m = p->m, n = p->n, k = p->k;
+    auto range = [](const void* at, size_t bytes) { return Range{static_cast<const char*>(at), static_cast<const char*>(at) + bytes}; };
+    const Range written[3] = {range(x_dev->ptr, m * k * 2), range(y_dev->ptr, m * n * 4), range(y_host, m * n * 4)};
+    const Range read[5] = {range(x_host, m * k * 2), range(wq->ptr, n * k / 2), range(ws->ptr, n * k / 16), range(wg->ptr, n * 4),
+                           r ? range(r->ptr, m * n * 4) : Range{nullptr, nullptr}};
+    for (uint32_t w = 0; w < 3u; w++) {
+        for (uint32_t v = 0; v < w; v++)
+            if (meet(written[w], written[v])) return false;
+        for (uint32_t v = 0; v < 5u; v++)
+            if (meet(written[w], read[v]) && !(w == 1u && v == 4u && r->ptr == y_dev->ptr)) return false;
+    }
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(g->stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return false;
+    }
+    return is_pinned(x_host) && is_pinned(y_host);
+}
+
 // The call below in parts of p->host_part tokens: the copies in, the launches and the copies out on three streams, ordered
 // by events, so that a part is copied out while the next is copied in and multiplied.  The launch stream waits for the last
 // copy, as if it had made them all.  Pinned memory only: copies of pageable memory do not return before they are made.
@@ -1663,7 +1689,7 @@ int lexb_gemm_fp4_run_host(lexb_gpu* g, const lexb_pipeline* p, const void* x_ho
     if (p->x_q16) return fail(LEXB_ERR_UNSUPPORTED, "lexb_gemm_fp4_run_host takes f16 or f32 activations; quantise on the device (lexb_quant16) and launch a step");
     const size_t xb = static_cast<size_t>(p->m) * p->k * (p->x_f32 ? 4 : 2), yb = static_cast<size_t>(p->m) * p->n * 4;
     if (x_dev->bytes < xb || y_dev->bytes < yb) return fail(LEXB_ERR_ARG, "lexb_gemm_fp4_run_host: staging buffers too small");
-    if (p->host_part && p->gpu == g && x_dev->gpu == g && y_dev->gpu == g && !g->d_trace && is_pinned(x_host) && is_pinned(y_host)) {
+    if (host_parts_apply(g, p, x_host, x_dev, wq, ws, wg, r, y_dev, y_host)) {
         if ((rc = run_host_in_parts(g, p, x_host, x_dev, wq, ws, wg, r, y_dev, y_host))) return rc;
         CUDA_TRY(cudaStreamSynchronize(g->stream));
         return LEXB_OK;

@@ -445,6 +445,41 @@ def test_run_host_in_parts(gpu, m, n, residual):
     assert gpu.status_word() == 0
 
 
+@pytest.mark.parametrize("layout", ["y over the last tokens of x", "one place", "x over the last tokens of y"])
+def test_run_host_with_x_and_y_in_one_pinned_arena(gpu, layout):
+    """Host buffers that overlap: x is copied in whole before any of y is copied out, as it is with pageable memory.  (In
+    parts, the first part of y would be on its way out before the last tokens of x are copied in.)"""
+    m, n, k = 1024, 9472, 2048
+    x, wq, ws, wg = inputs.make_case(m, n, k, seed_base=93)
+    q, pipe = L.QBuf(gpu, wq, ws, wg), gpu.plan_gemm_fp4(m, n, k)
+    xd, yd = gpu.alloc(x.nbytes), gpu.alloc(m * n * 4)
+    hx, hy = L.HostBuffer(x.nbytes), L.HostBuffer(m * n * 4)
+    hx.array(np.float16, (m, k))[:] = x
+    gpu.run_host(pipe, hx.ptr, xd, q.wq, q.ws, q.wg, None, yd, hy.ptr)
+    want = hy.array(np.float32, (m, n))
+    x_at, y_at = {"y over the last tokens of x": (0, x.nbytes * 3 // 4), "one place": (0, 0), "x over the last tokens of y": (m * n * 4 - 4096, 0)}[layout]
+    arena = L.HostBuffer(m * n * 4 + x.nbytes)
+    for _ in range(3):
+        arena.array(np.uint8, (arena.nbytes,))[x_at:x_at + x.nbytes] = x.reshape(-1).view(np.uint8)
+        gpu.run_host(pipe, arena.ptr + x_at, xd, q.wq, q.ws, q.wg, None, yd, arena.ptr + y_at)
+        got = arena.array(np.uint8, (arena.nbytes,))[y_at:y_at + m * n * 4].view(np.float32).reshape(m, n)
+        assert np.array_equal(got, want)
+    assert gpu.status_word() == 0
+
+
+def test_run_host_with_the_residual_in_place(gpu):
+    """r and y as one device buffer, the result on top of it: token by token the same in parts as in one launch."""
+    m, n, k = 200, 9600, 512
+    x, wq, ws, wg = inputs.make_case(m, n, k, seed_base=94)
+    r = inputs.make_residual(m, n, seed_base=94)
+    q, pipe = L.QBuf(gpu, wq, ws, wg), gpu.plan_gemm_fp4(m, n, k, residual=True)
+    hx, hy = L.HostBuffer(x.nbytes), L.HostBuffer(m * n * 4)
+    hx.array(np.float16, (m, k))[:] = x
+    xd, yd = gpu.alloc(x.nbytes), gpu.upload(r)
+    gpu.run_host(pipe, hx.ptr, xd, q.wq, q.ws, q.wg, yd, yd, hy.ptr)
+    check(hy.array(np.float32, (m, n)).copy(), O.gemm_fp4(x, wq, ws, wg, r=r))
+
+
 def test_torch_default_stream_is_passed_as_the_legacy_stream(gpu):
     """torch's default stream has the handle 0, which means "the library's own stream" to lexb_set_stream: the
     binding passes cudaStreamLegacy instead, so that launches are ordered with torch's work on that stream.
