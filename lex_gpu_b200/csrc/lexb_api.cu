@@ -101,6 +101,7 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
 
 enum { KERNEL_MATVEC = 1, KERNEL_TCGEN05 = 2, KERNEL_TCGEN05_PAIR = 3, KERNEL_MATMUL_Q = 4 };
 thread_local bool t_plan_q16 = false;      // set by lexb_matmul_int8_plan around its call of lexb_gemm_fp4_plan
+thread_local float* t_plan_partial = nullptr;      // a split-K workspace to borrow instead of allocating one (run_host_in_parts)
 
 }  // namespace
 
@@ -163,7 +164,8 @@ struct lexb_pipeline {
     bool mq_pre = false;        // ... with the tokens' digit rows from the pieces kernel: buffers and their tensor map
     uint8_t* pre_buf = nullptr; // [8 m][k / 2] digit rows, then [k / 256][2048] scale blocks, then [m] magnitudes
     CUtensorMap pre_map{};
-    float* partial = nullptr;   // split-K workspace [k_splits][m][n], owned by the pipeline
+    float* partial = nullptr;   // split-K workspace [k_splits][m][n], owned by the pipeline (a part of run_host's: by the whole's)
+    bool partial_borrowed = false;
     // matvec
     uint32_t sm_warps = 24;     // ... warps per SM the registers are cut to (24 or 16)
     uint32_t kc, cluster = 1, parts = 8;   // ... K columns of x staged at a time, blocks that share a row block's K, parts K has
@@ -1336,12 +1338,15 @@ int lexb_gemm_fp4_plan(lexb_gpu* g, uint32_t m, uint32_t n, uint32_t k, int resi
         splits = (raw_blocks + rb_per_split - 1u) / rb_per_split;          // no empty split
         p->k_splits = splits;
         p->kb_per_split = rb_per_split * (lexb::PAIR_RAW_K / lexb::GEMM_BK);
-        if (splits > 1u) {
+        p->partial_borrowed = splits > 1u && t_plan_partial;
+        if (p->partial_borrowed) {
+            p->partial = t_plan_partial;
+        } else if (splits > 1u) {
             cudaError_t e = x_malloc(&p->partial, sizeof(float) * splits * static_cast<size_t>(m) * n);
             if (e != cudaSuccess) return bail(fail(LEXB_ERR_CUDA, "allocating the split-K workspace: %s", cudaGetErrorString(e)));
         }
         // From host memory: y leaves at 55 GB/s, 10 to 20 times slower than it is made, so it should start to leave early.
-        // Where unsplit tiles of a part's tokens fill at least half of the machine, a part's launch takes less time than its
+        // Where one row of tiles fills at least half of the machine, a part's launch takes less time than its
         // copy out and only the first part's copy in and launch are waited for.
         if (!s.tm && !s.stages && !s.w_stages && !s.k_splits && m >= 192u && 2u * n_pairs >= sm_pairs)
             p->host_part = round_up((m + lexb_gpu::HOST_PARTS - 1u) / lexb_gpu::HOST_PARTS, 64u);
@@ -1472,7 +1477,7 @@ void lexb_pipeline_free(lexb_pipeline* p) {
     for (lexb_pipeline* part : p->host_pipes) lexb_pipeline_free(part);
     if (p->partial || p->pre_buf) {
         cudaSetDevice(p->gpu->device);
-        cudaFree(p->partial);
+        if (!p->partial_borrowed) cudaFree(p->partial);
         cudaFree(p->pre_buf);
     }
     delete p;
@@ -1622,7 +1627,8 @@ static bool host_parts_apply(const lexb_gpu* g, const lexb_pipeline* p, const vo
 }
 
 // The call below in parts of p->host_part tokens: the copies in, the launches and the copies out on three streams, ordered
-// by events, so that a part is copied out while the next is copied in and multiplied.  The launch stream waits for the last
+// by events, so that a part is copied out while the next is copied in and multiplied.  A part has the whole's K split, in the
+// whole's workspace, so y's bits do not depend on the way taken.  The launch stream waits for the last
 // copy, as if it had made them all.  Pinned memory only: copies of pageable memory do not return before they are made.
 static int run_host_in_parts(lexb_gpu* g, const lexb_pipeline* p, const void* x_host, lexb_buffer* x_dev, const lexb_buffer* wq,
                              const lexb_buffer* ws, const lexb_buffer* wg, const lexb_buffer* r, lexb_buffer* y_dev, void* y_host) {
@@ -1647,9 +1653,12 @@ static int run_host_in_parts(lexb_gpu* g, const lexb_pipeline* p, const void* x_
                 if (!part) {
                     lexb_sched s{};
                     s.kernel = KERNEL_TCGEN05_PAIR;
-                    s.k_splits = 1;                                      // (no workspace)
+                    s.k_splits = p->k_splits;                            // the sums of one launch of the whole, bit for bit
                     s.flags = (p->w_const ? LEXB_SCHED_WEIGHTS_CONSTANT : 0u) | (p->w_volatile ? LEXB_SCHED_WEIGHTS_MAY_CHANGE : 0u);
-                    if ((rc = lexb_gemm_fp4_plan(g, tokens, p->n, p->k, p->residual, &s, &part))) return rc;
+                    t_plan_partial = p->partial;                         // (one part at a time, in the launch stream's order)
+                    rc = lexb_gemm_fp4_plan(g, tokens, p->n, p->k, p->residual, &s, &part);
+                    t_plan_partial = nullptr;
+                    if (rc) return rc;
                 }
             }
             const size_t xo = static_cast<size_t>(t0) * p->k * 2, xb = static_cast<size_t>(tokens) * p->k * 2;

@@ -467,6 +467,28 @@ def test_run_host_with_x_and_y_in_one_pinned_arena(gpu, layout):
     assert gpu.status_word() == 0
 
 
+@pytest.mark.parametrize("m,n,k,splits", [(200, 9472, 4096, 2), (200, 9600, 8192, 3), (600, 9472, 1024, 1)])
+def test_run_host_gives_the_bits_of_a_launch(gpu, m, n, k, splits):
+    """One plan, K split or not: y from pinned host memory (in parts), from pageable memory and from a launch on the device
+    are the same bits."""
+    x, wq, ws, wg = inputs.make_case(m, n, k, seed_base=95)
+    q, pipe = L.QBuf(gpu, wq, ws, wg), gpu.plan_gemm_fp4(m, n, k)
+    assert pipe.describe().k_splits == splits
+    hx, hy = L.HostBuffer(x.nbytes), L.HostBuffer(m * n * 4)
+    hx.array(np.float16, (m, k))[:] = x
+    xd, yd = gpu.upload(x), gpu.alloc(m * n * 4)
+    gpu.run(pipe, q.bind(xd, None, yd))
+    want = gpu.download(yd, np.float32, (m, n))
+    pageable = np.empty((m, n), np.float32)
+    for _ in range(2):
+        gpu.memset(yd, 0xFF)
+        gpu.run_host(pipe, hx.ptr, xd, q.wq, q.ws, q.wg, None, yd, hy.ptr)
+        assert np.array_equal(hy.array(np.float32, (m, n)), want)
+        gpu.run_host(pipe, x.ctypes.data, xd, q.wq, q.ws, q.wg, None, yd, pageable.ctypes.data)
+        assert np.array_equal(pageable, want)
+    assert gpu.status_word() == 0
+
+
 def test_run_host_with_the_residual_in_place(gpu):
     """r and y as one device buffer, the result on top of it: token by token the same in parts as in one launch."""
     m, n, k = 200, 9600, 512
