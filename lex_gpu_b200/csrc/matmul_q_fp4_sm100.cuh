@@ -272,7 +272,6 @@ matmul_q_fp4_kernel(const __grid_constant__ CUtensorMap tmap_wq, const __grid_co
         tmem_alloc(smem_u32(tmem_slot), MQ_TMEM_COLS);
         tmem_relinquish();
     }
-    if (warp != 0) allow_dependents();
     // Warp 0 has set up every barrier itself and needs nothing from the others: it announces that and
     // goes on to its loads, the other warps meet here (named barrier 2).
     uint32_t tmem_base = 0;
@@ -281,6 +280,7 @@ matmul_q_fp4_kernel(const __grid_constant__ CUtensorMap tmap_wq, const __grid_co
     } else {
         tc_fence_before_sync();
         asm volatile("bar.sync 2, %0;" ::"r"(NTHREADS) : "memory");
+        allow_dependents();                  // (not before this block holds its columns: see tmem_alloc; warp 0 does not know)
         tc_fence_after_sync();
         tmem_base = *tmem_slot;
     }
@@ -334,7 +334,6 @@ matmul_q_fp4_kernel(const __grid_constant__ CUtensorMap tmap_wq, const __grid_co
                 }
                 mbar_arrive_expect_tx(raw_full(s), MQ_CODE_BYTES + (PRE ? b_bytes + sfb_bytes : 0u));
                 tma_load_2d(codes_of(s), &tmap_wq, (int)((kb0 + kb) * (MQ_STAGE_K / 2)), (int)n0, raw_full(s));
-                if (kb + 1u == S || kb + 1u == KB) allow_dependents();       // the ring is filled (once is enough; twice is harmless)
                 if (PRE) {
                     // The digit rows are written by the launch ahead (the pieces kernel): the first ring of
                     // weights goes out before that launch is waited for, the digit rows of those stages after.
