@@ -343,7 +343,9 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
     return r;
 }
 // All threads of both CTAs: nobody passes until everybody has arrived.
+// (the aligned form wants the warp together, which lane-divergent code ahead of it does not promise)
 __device__ __forceinline__ void cluster_sync_all() {
+    __syncwarp();
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 __device__ __forceinline__ float ld_shared_cluster_f32(uint32_t cluster_addr) {

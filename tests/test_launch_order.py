@@ -29,3 +29,13 @@ def test_dependents_go_only_once_the_block_holds_its_tensor_memory(name, barrier
     if name == "matmul_q_fp4_sm100.cuh":
         copy_warp = kernels[0][kernels[0].index("tma_load_2d"):kernels[0].index("umma_idesc")]
         assert "allow_dependents" not in copy_warp
+
+
+def test_the_cluster_barrier_brings_the_warp_together_first():
+    """barrier.cluster.*.aligned must be executed by all lanes of a warp at once; the matvec meets it behind code whose lanes
+    part (tokens that do not exist, outputs that do not divide by the threads)."""
+    for name in ("sm100_ptx.cuh", "matvec_fp4_sm100.cuh", "gemm_fp4_sm100_pair.cuh"):
+        for at in re.finditer(r"barrier\.cluster\.(?:arrive|wait)[\w.]*\.aligned", code(name)):
+            ahead = code(name)[:at.start()]
+            last = max(ahead.rfind("__syncwarp()"), ahead.rfind("barrier.cluster"))
+            assert last > ahead.rfind("__device__"), name
