@@ -599,8 +599,11 @@ int launch_one(lexb_gpu* g, const lexb_pipeline* p, const lexb_buffer* x, const 
         a.r = r ? static_cast<const float*>(r->ptr) : nullptr;
         a.y = static_cast<float*>(y->ptr);
         a.m = p->m; a.n = p->n; a.k = p->k; a.kc = p->kc;
-        a.cluster = p->cluster;
-        a.parts = p->parts;
+        auto log2u = [](uint32_t v) { uint32_t l = 0; while (v >>= 1) l++; return l; };
+        a.log_cluster = log2u(p->cluster);
+        a.log_parts = log2u(p->parts);
+        a.log_group = log2u(p->threads / 32u * p->cluster / p->parts);
+        a.log_tokens = log2u(std::min(p->threads / 32u, 2u * p->m - 1u));
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3(p->grid);
         cfg.blockDim = dim3(p->threads);

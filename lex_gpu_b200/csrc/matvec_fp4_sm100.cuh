@@ -58,8 +58,11 @@ struct MatvecArgs {
     float* y;             // [m, n]
     uint32_t m, n, k;
     uint32_t kc;          // K columns of x staged per chunk: multiple of MV_ROUND
-    uint32_t cluster;     // blocks that share the parts of K: 1, 2, 4 or 8
-    uint32_t parts;       // parts that K has: 8, or 4, 2, 1 if that is as many as it has slices
+    // powers of two, as their logarithms (a division by a run-time number costs a short launch more than its multiply)
+    uint32_t log_cluster; // blocks that share the parts of K: 1, 2, 4 or 8
+    uint32_t log_parts;   // parts that K has: 8, or 4, 2, 1 if that is as many as it has slices
+    uint32_t log_group;   // row blocks a cluster works on at once: its warps / parts
+    uint32_t log_tokens;  // tokens a block's warps stage at once: m rounded up, at most the block's warps
 };
 
 // token pitch in bytes: kc/32 runs of 72 bytes, padded to 32 (mod 128)
@@ -110,44 +113,47 @@ __global__ void __launch_bounds__(MV_THREADS, WARPS / MV_WARPS) matvec_fp4_kerne
     uint8_t* const ring = mv_smem + 2u * warps * RED * 4u;              // [warp][MV_DEPTH] stages of packed weights
     uint8_t* const zeros = ring + (RING ? warps * MV_DEPTH * MV_STAGE_BYTES : 0u);   // 128 bytes: x of a token that does not exist
     uint8_t* const xs = zeros + 128u;
-    // launched with programmatic stream serialization: the blocks are in place when the launch ahead ends
-    allow_dependents();
-    const uint32_t C = a.cluster, rank = C > 1u ? cluster_ctarank() : 0u;
-    const uint32_t parts = a.parts, PP = parts / C;                     // parts of K in this block
-    const uint32_t R = warps / PP;                                      // row blocks the cluster works on at once: a group
-    const uint32_t part = rank * PP + (warp & (PP - 1u)), sub = warp / PP;           // this warp's part of K, and its row block of the group
+    const uint32_t lc = a.log_cluster, lp = a.log_parts, lr = a.log_group, lpp = lp - lc;
+    const uint32_t C = 1u << lc, rank = C > 1u ? cluster_ctarank() : 0u;
+    const uint32_t parts = 1u << lp, PP = 1u << lpp;                    // parts of K, of them in this block
+    const uint32_t R = 1u << lr;                                        // row blocks the cluster works on at once: a group
+    const uint32_t part = (rank << lpp) + (warp & (PP - 1u)), sub = warp >> lpp;     // this warp's part of K, and its row block of the group
     const uint32_t k = a.k, kc = a.kc;
-    const uint32_t pitch = matvec_x_pitch(kc / C);
+    const uint32_t pitch = matvec_x_pitch(kc >> lc);
     const uint32_t slices = (k + MV_SLICE - 1u) / MV_SLICE;             // per row block
-    const uint32_t row_blocks = a.n / MV_ROWS, groups = (row_blocks + R - 1u) / R;
-    const uint32_t first_group = blockIdx.x / C, group_step = gridDim.x / C;
+    const uint32_t row_blocks = a.n / MV_ROWS, groups = (row_blocks + R - 1u) >> lr;
+    const uint32_t first_group = blockIdx.x >> lc, group_step = gridDim.x >> lc;
     const bool resident = kc >= k;                                      // all of x staged once
 
+    // Launched with programmatic stream serialization: the blocks are in place when the launch ahead ends.  The next launch's
+    // blocks are let in only then.  Let in earlier, they gather, as many as fit, on the SMs that this launch has left free, and
+    // its own turn then waits for the fullest SM (1024x4096, m = 1, back to back: 5.1 us; 4.0 like this).
     grid_dependency_wait();
+    allow_dependents();
 
     // lanes whose token does not exist (and lanes past the end of K) read the zero block instead
     const bool have_lo = g < a.m, have_hi = HI && (g + 8u) < a.m;
 
     // this block's parts of x[:, k0:k1] -> shared memory, asynchronously and 8 bytes at a time (coalesced in,
-    // conflict-free out): slice s of the chunk is the block's slice (s / 8) * PP + s % PP
+    // conflict-free out): slice s of the chunk is the block's slice (s / 8) * PP + s % PP.  A warp takes a token's slice at a
+    // time, 256 bytes; the warps are dealt to the tokens, and within a token to its slices.
     auto stage_x = [&](uint32_t k0, uint32_t k1) {
-        const uint32_t sc = (k1 - k0 + MV_SLICE - 1u) / MV_SLICE, rem = sc & (parts - 1u), p0 = rank * PP;
-        const uint32_t mine = sc / parts * PP + (rem <= p0 ? 0u : (rem - p0 < PP ? rem - p0 : PP));
-        for (uint32_t tok = 0; tok < a.m; tok++) {
+        const uint32_t sc = (k1 - k0 + MV_SLICE - 1u) / MV_SLICE, rem = sc & (parts - 1u), p0 = rank << lpp;
+        const uint32_t mine = ((sc >> lp) << lpp) + (rem <= p0 ? 0u : (rem - p0 < PP ? rem - p0 : PP));
+        const uint32_t lt = a.log_tokens, per_token = warps >> lt;
+        for (uint32_t tok = warp & ((1u << lt) - 1u); tok < a.m; tok += 1u << lt) {
             const __half* src = a.x + (size_t)tok * k + k0;
-            const uint32_t dst = smem_u32(xs) + tok * pitch;
-            for (uint32_t u = tid; u < mine * 32u; u += nthreads) {     // 8-byte units
-                const uint32_t j = u >> 5, v = u & 31u;
-                const uint32_t col = ((j / PP) * parts + p0 + (j & (PP - 1u))) * MV_SLICE + 4u * v;
-                if (!RAGGED || k0 + col < k1) cp_async_8(dst + (j * 4u + (v >> 3)) * 72u + (v & 7u) * 8u, src + col, 8u);
+            const uint32_t dst = smem_u32(xs) + tok * pitch + (lane >> 3) * 72u + (lane & 7u) * 8u;
+            for (uint32_t j = warp >> lt; j < mine; j += per_token) {
+                const uint32_t col = (((j >> lpp) << lp) + p0 + (j & (PP - 1u))) * MV_SLICE + 4u * lane;
+                if (!RAGGED || k0 + col < k1) cp_async_8(dst + j * 288u, src + col, 8u);
             }
         }
         if (tid < 16u) *reinterpret_cast<uint2*>(zeros + tid * 8u) = make_uint2(0u, 0u);
-        cp_async_commit();
     };
 
     // This warp's slices of a row block: part, part + 8, ... (fewer parts: one slice, or none)
-    const uint32_t my_slices = part < slices ? (slices - part + parts - 1u) / parts : 0u;
+    const uint32_t my_slices = part < slices ? (slices - part + parts - 1u) >> lp : 0u;
     const size_t q_row = k / 2u, s_row = k / 16u, q_pitch8 = 8u * q_row;
     // The copy cursor: this lane's codes of the next slice to be asked for (row g; row g + 8 is q_pitch8 further) and its
     // scale bytes - in the ring lanes t = 0 and 1 of a quad copy the quad's 8 of row g and of row g + 8.
@@ -174,27 +180,35 @@ __global__ void __launch_bounds__(MV_THREADS, WARPS / MV_WARPS) matvec_fp4_kerne
     // This warp's ring.  Stage layout: [codes of row g: 32 lanes x 16 B][codes of row g + 8][scales: 16 rows x 8 B].
     uint8_t* const my_ring = ring + warp * (MV_DEPTH * MV_STAGE_BYTES);
     uint32_t st_c = 0, st = 0;                                          // byte offsets of the stages: next to fill, next to use
-    // asynchronous copies of the next slice (one commit group, also when there is none: the groups are counted)
-    auto issue_next = [&]() {
+    // asynchronous copies of the next slice (a commit group of its own, also when there is none: the groups are counted)
+    uint32_t scales = 0, scales_b = 0, scales_at = 0;                   // (RAGGED) loaded scale bytes and the stage they belong to
+    auto issue_copies = [&]() {
+        if (RAGGED) {
+            uint8_t* sdst = my_ring + scales_at + 1024u + g * 8u + 2u * t;
+            *reinterpret_cast<unsigned short*>(sdst) = static_cast<unsigned short>(scales);
+            *reinterpret_cast<unsigned short*>(sdst + 64u) = static_cast<unsigned short>(scales_b);
+        }
         if (rb_c < row_blocks && my_slices != 0u) {
             const uint32_t in_k = cursor_in_k() ? 1u : 0u;              // zeros past the end of K
             const uint32_t dst = smem_u32(my_ring) + st_c + lane * 16u;
             cp_async_16(dst, in_k ? q_next : a.wq, 16u * in_k);
             cp_async_16(dst + 512u, in_k ? q_next + q_pitch8 : a.wq, 16u * in_k);
             if (RAGGED) {
-                // k % 128 != 0: a row's scale bytes are not 8-byte aligned, so each lane fetches its own two
-                // (plain loads; these shapes are small)
-                uint8_t* sdst = my_ring + st_c + 1024u + g * 8u + 2u * t;
-                *reinterpret_cast<unsigned short*>(sdst) = in_k ? __ldg(reinterpret_cast<const unsigned short*>(s_next)) : (unsigned short)0;
-                *reinterpret_cast<unsigned short*>(sdst + 64u) =
-                    in_k ? __ldg(reinterpret_cast<const unsigned short*>(s_next + 8u * s_row)) : (unsigned short)0;
+                // k % 128 != 0: a row's scale bytes are not 8-byte aligned, so each lane loads its own two of both rows
+                // and stores them when the next slice is asked for, not waiting for them here
+                scales = in_k ? __ldg(reinterpret_cast<const unsigned short*>(s_next)) : 0u;
+                scales_b = in_k ? __ldg(reinterpret_cast<const unsigned short*>(s_next + 8u * s_row)) : 0u;
+                scales_at = st_c;
             } else if (t < 2u) {
                 cp_async_8(smem_u32(my_ring) + st_c + 1024u + (g + 8u * t) * 8u, s_next, 8u);
             }
             cursor_step();
         }
-        cp_async_commit();
         st_c = st_c == (MV_DEPTH - 1u) * MV_STAGE_BYTES ? 0u : st_c + MV_STAGE_BYTES;
+    };
+    auto issue_next = [&]() {
+        issue_copies();
+        cp_async_commit();
     };
     // the register path (RING = false): this lane's loads for the next slice
     auto load_next = [&]() {
@@ -230,19 +244,21 @@ __global__ void __launch_bounds__(MV_THREADS, WARPS / MV_WARPS) matvec_fp4_kerne
     };
     load_row_scales(rb_c);
 
-    // (x first: its copies are the oldest group.)  The copies run MV_DEPTH slices ahead of the decode, in the same
-    // order: this warp's slices of a row block, then those of its next one.
-    if (resident) stage_x(0, k);
+    // The first weights go out before x (they come from HBM, x mostly from L2) and are waited for with it.  The copies run
+    // MV_DEPTH slices ahead of the decode, in the same order: this warp's slices of a row block, then those of its next one.
     MvLoad nxt{};
+    if constexpr (RING) issue_copies();
+    else nxt = load_next();
+    if (resident) stage_x(0, k);
+    cp_async_commit();
     if constexpr (RING) {
 #pragma unroll
-        for (uint32_t d = 0; d < MV_DEPTH; d++) issue_next();
-    } else {
-        nxt = load_next();
+        for (uint32_t d = 1; d < MV_DEPTH; d++) issue_next();
     }
-
+    // (the row scales are on their way since before the copies: what follows from them is worked out under the wait)
+    RowScale ga = make_row_scale(wg_a), gb = make_row_scale(wg_b);
     if (resident) {
-        cp_async_wait<RING ? MV_DEPTH : 0u>();
+        cp_async_wait<RING ? MV_DEPTH - 1u : 0u>();
         __syncthreads();
     }
 
@@ -253,7 +269,6 @@ __global__ void __launch_bounds__(MV_THREADS, WARPS / MV_WARPS) matvec_fp4_kerne
     for (uint32_t grp_i = first_group; grp_i < groups; grp_i += group_step, parity ^= 1u) {
         const uint32_t rb = grp_i * R + sub;                            // (>= row_blocks in the last group: this warp has no rows)
         const bool have_rb = rb < row_blocks;
-        const RowScale ga = make_row_scale(wg_a), gb = make_row_scale(wg_b);
         load_row_scales(rb + group_step * R);                           // (in flight during this row block)
         // rows g and g + 8 are decoded side by side: their scale bytes share a word, g's in the low half
         const uint32_t below = prmt(ga.below, gb.below, 0x5410u), above = prmt(ga.above, gb.above, 0x5410u);
@@ -267,6 +282,7 @@ __global__ void __launch_bounds__(MV_THREADS, WARPS / MV_WARPS) matvec_fp4_kerne
                 const uint32_t k1 = (k0 + kc < k) ? (k0 + kc) : k;
                 __syncthreads();                                        // previous chunk fully consumed
                 stage_x(k0, k1);
+                cp_async_commit();
                 cp_async_wait<0>();
                 __syncthreads();
                 here = min(left, kc / MV_ROUND);                        // (all chunks but the last are whole rounds)
@@ -358,26 +374,32 @@ __global__ void __launch_bounds__(MV_THREADS, WARPS / MV_WARPS) matvec_fp4_kerne
         }
         if (C > 1u) cluster_sync_all();
         else __syncthreads();
-        // outputs of the group: m tokens x R * 16 rows, shared out over the cluster's threads
-        for (uint32_t o_i = rank * nthreads + tid; o_i < a.m * R * MV_ROWS; o_i += C * nthreads) {
-            const uint32_t tok = o_i / (R * MV_ROWS), ri = o_i - tok * (R * MV_ROWS);
-            const uint32_t row = grp_i * R * MV_ROWS + ri;
+        // outputs of the group: m tokens x R * 16 rows, four rows a thread, shared out over the cluster's threads
+        const uint32_t log_quads = lr + 2u;
+        for (uint32_t o_i = rank * nthreads + tid; o_i < (a.m << log_quads); o_i += nthreads << lc) {
+            const uint32_t tok = o_i >> log_quads, ri = (o_i & ((1u << log_quads) - 1u)) * 4u;
+            const uint32_t row = (grp_i << (lr + 4u)) + ri;
             if (row >= a.n) continue;
-            const float* rp = red + (parity * warps + (ri >> 4) * PP) * RED + tok * MV_RED_PITCH + (ri & 15u);
-            float s = 0.f;
+            const float* rp = red + (parity * warps + ((ri >> 4) << lpp)) * RED + tok * MV_RED_PITCH + (ri & 15u);
+            float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+            auto add = [&](const float4& v) { s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w; };
             if (C > 1u) {
                 const uint32_t rp_u32 = smem_u32(rp);
 #pragma unroll
                 for (uint32_t p = 0; p < MV_PARTS; p++)
-                    if (p < parts) s += ld_shared_cluster_f32(map_to_cta(rp_u32 + (p & (PP - 1u)) * (RED * 4u), p / PP));
+                    if (p < parts) add(ld_shared_cluster_f32x4(map_to_cta(rp_u32 + (p & (PP - 1u)) * (RED * 4u), p >> lpp)));
             } else {
 #pragma unroll
                 for (uint32_t p = 0; p < MV_PARTS; p++)
-                    if (p < parts) s += rp[p * RED];
+                    if (p < parts) add(*reinterpret_cast<const float4*>(rp + p * RED));
             }
-            const size_t o = (size_t)tok * a.n + row;
-            if (a.r) s = s + __ldg(a.r + o);
-            a.y[o] = s;
+            const size_t o = (size_t)tok * a.n + row;                       // (n % 16 == 0: rows of whole 16-byte quads)
+            if (a.r) add(__ldg(reinterpret_cast<const float4*>(a.r + o)));
+            *reinterpret_cast<float4*>(a.y + o) = s;
+        }
+        if (grp_i + group_step < groups) {
+            ga = make_row_scale(wg_a);
+            gb = make_row_scale(wg_b);
         }
     }
     if (C > 1u) cluster_sync_all();                                     // a block's sums are read by the others until here

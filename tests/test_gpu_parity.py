@@ -133,6 +133,17 @@ def test_matvec_over_a_cluster(gpu, n, k):
         assert np.array_equal(L.gemm_fp4(gpu, x[:m].copy(), wq, ws, wg, r=r[:m].copy()), y16[:m]), m
 
 
+@pytest.mark.parametrize("m", [1, 3, 8, 13])
+@pytest.mark.parametrize("n,k", [(16, 32), (48, 64), (1040, 96), (4112, 128), (2064, 160), (1040, 224), (4112, 288), (2064, 480), (528, 544), (16, 1056), (272, 2080)])
+def test_matvec_short_and_ragged_k(gpu, m, n, k):
+    """Few parts of K (1, 2, 4, 8), k that ends inside a slice, blocks of 4 warps with several row blocks, the last one alone."""
+    x, wq, ws, wg = inputs.make_case(m, n, k, seed_base=73)
+    r = inputs.make_residual(m, n, seed_base=73)
+    got = L.gemm_fp4(gpu, x, wq, ws, wg, r=r, kernel=1)
+    check(got, O.gemm_fp4(x, wq, ws, wg, r=r, bk=32))
+    assert np.array_equal(got[:1], L.gemm_fp4(gpu, x[:1].copy(), wq, ws, wg, r=r[:1].copy(), kernel=1))
+
+
 # ---------------------------------------------------------------- tcgen05 path (m > 16)
 
 def test_gemm_config0_readme_example(gpu):
