@@ -150,6 +150,21 @@ LEXB_API int lexb_gemm_fp4_plan(lexb_gpu* gpu, uint32_t m, uint32_t n, uint32_t 
 LEXB_API void lexb_pipeline_free(lexb_pipeline* p);                                /* Pipeline::drop */
 LEXB_API int lexb_pipeline_describe(const lexb_pipeline* p, lexb_lowered* out);
 
+/* How a pipeline's work is laid out beyond its launch descriptor, for tests and for callers that want to see it; no
+ * counterpart in the reference. */
+typedef struct lexb_route {
+    uint32_t cluster;        /* matvec: blocks that share a row block's K (1 otherwise) */
+    uint32_t parts;          /* matvec: parts K is summed in, a warp each */
+    uint32_t groups;         /* matvec: groups of row blocks each block (cluster) works through */
+    uint32_t kc;             /* matvec: K columns of x staged at a time, over the cluster's blocks; less than k: in chunks */
+    uint32_t blocks, threads;
+    uint32_t host_part;      /* tokens of a part of lexb_gemm_fp4_run_host from pinned memory; 0: always whole */
+} lexb_route;
+LEXB_API int lexb_pipeline_route(const lexb_pipeline* p, lexb_route* out);
+/* The matvec's route for a B200 with `sms` SMs, by host arithmetic only (needs no GPU; the number of clusters that a device
+ * holds at once is estimated). */
+LEXB_API int lexb_matvec_route(uint32_t sms, uint32_t m, uint32_t n, uint32_t k, uint32_t kc, lexb_route* out);
+
 /* One Step, asynchronous on the gpu's stream: Gpu::run, crates/lex-cuda/src/device.rs:629-648.
  * Buffers in the order [x, wq, ws, wg, (r), y]; r must be null exactly when the pipeline
  * was planned without a residual. */

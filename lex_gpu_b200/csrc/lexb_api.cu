@@ -8,6 +8,7 @@
 
 #include <algorithm>
 #include <chrono>
+#include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
@@ -144,6 +145,16 @@ struct lexb_buffer {
     bool owned;
 };
 
+// How the matvec's launch is laid out (plan_matvec).
+struct MatvecShape {
+    uint32_t parts = 8;         // parts that K is summed in
+    uint32_t cluster = 1;       // blocks that share a row block's K
+    uint32_t warps = 8;         // per block
+    uint32_t sm_warps = 24;     // warps per SM the registers are cut to (24 or 16)
+    uint32_t kc = 0, smem = 0;  // K columns of x staged at a time, shared memory per block
+    uint32_t clusters = 0, per = 0;   // clusters (blocks, without clusters) of the launch, groups of row blocks each works through
+};
+
 struct lexb_pipeline {
     lexb_gpu* gpu;
     uint32_t kernel;
@@ -167,8 +178,8 @@ struct lexb_pipeline {
     float* partial = nullptr;   // split-K workspace [k_splits][m][n], owned by the pipeline (a part of run_host's: by the whole's)
     bool partial_borrowed = false;
     // matvec
-    uint32_t sm_warps = 24;     // ... warps per SM the registers are cut to (24 or 16)
-    uint32_t kc, cluster = 1, parts = 8;   // ... K columns of x staged at a time, blocks that share a row block's K, parts K has
+    MatvecShape mv;
+    uint32_t kc;                // ... K columns of x staged at a time
     uint32_t grid, threads, smem;
     char entry[96];
     // tensor maps of x, keyed by the device pointer they were encoded for
@@ -428,6 +439,77 @@ uint32_t matvec_clusters(MatvecKernel kernel, uint32_t c, uint32_t threads, uint
     return static_cast<uint32_t>(clusters);
 }
 
+// The matvec's launch.  K is summed in 8 parts (4, 2 or 1 if it has no more slices; a row's result depends on k alone), held
+// by one block or by a cluster of 2, 4 or 8; blocks have 8 warps or 4, and as many row blocks at a time as their warps
+// hold all of their parts.  A cluster divides the staged x, so that a long k at several tokens still leaves room for enough
+// warps per SM (m = 4, k = 17408: 157 KB of x in one block, 20 KB each in eight); it costs a barrier across the cluster.
+// A short k puts several row blocks in a block, which leaves SMs idle where there are few of them: hence blocks of 4 warps.
+//
+// Every form is priced in us, with figures fitted to 12,600 launches on a B200 (m = 1-16, n = 128-28672, k = 64-17408, back to
+// back on one stream; the form chosen takes 1.3 % more than the fastest in the mean, 8 % at the 95th percentile): the slices of the
+// fullest SM at its rate, or a warp's own chain of them, the first three of which are in flight together (`three`, then
+// `slice`); per group of row blocks `group` for its sums and `output` per turn of the threads over its outputs; `cluster`
+// and `cluster_group` for the barriers; x from the L2; a chunked x per wave of blocks.  `uneven`: where more blocks fit an
+// SM than its even share, the fullest one gets more.
+template <typename Held>
+bool plan_matvec(uint32_t m, uint32_t n, uint32_t k, uint32_t kc_asked, uint32_t sms, size_t smem_optin, size_t smem_sm, Held held, MatvecShape* out) {
+    struct Price { double rate24, rate16, three, slice, group, output, cluster, cluster_group, x, chunk, uneven; };
+    static const Price UP_TO_8 = {0.053, 0.044, 0.50, 0.45, 0.13, 0.22, 2.1, 1.1, 6.2e-5, 2.1, 0.58},
+                       PAST_8 = {0.043, 0.043, 0.017, 0.71, 0.23, 0.45, 2.4, 2.3, 7.5e-5, 1.8, 0.98};
+    const bool ring = m <= 8u;
+    const Price& f = ring ? UP_TO_8 : PAST_8;
+    const uint32_t row_blocks = n / lexb::MV_ROWS, slices = (k + lexb::MV_SLICE - 1u) / lexb::MV_SLICE;
+    uint32_t parts = lexb::MV_PARTS;
+    while (parts / 2u >= slices) parts /= 2u;                            // (a short k leaves no warp without a slice)
+    const uint32_t part_slices = (slices + parts - 1u) / parts;
+    double best = 1e30;
+    for (uint32_t c = 1; c <= parts; c *= 2u) {
+        const uint32_t pp = parts / c;
+        for (uint32_t warps = 8; warps >= 4u && warps >= pp; warps /= 2u) {
+            for (uint32_t sm_warps = 24; sm_warps >= (ring ? 16u : 24u); sm_warps -= 8u) {
+                uint32_t kc = kc_asked;
+                if (!kc) {
+                    // the whole of K if a block's share of x fits in 96 KiB of shared memory (blocks are then persistent
+                    // and stage x once), else the largest multiple of 1024 columns that does
+                    const uint32_t budget = 98304u;
+                    kc = round_up(k, lexb::MV_SLICE * parts);
+                    while (kc > lexb::MV_ROUND && m * lexb::matvec_x_pitch(kc / c) > budget) kc -= lexb::MV_ROUND;
+                }
+                const uint32_t smem = lexb::matvec_smem_bytes(m, kc, warps, c, ring);
+                if (smem > smem_optin) continue;
+                const uint32_t per_sm = std::min(static_cast<uint32_t>(smem_sm / (smem + 1024u)), sm_warps / warps);
+                const uint32_t at_once = warps / pp, groups = (row_blocks + at_once - 1u) / at_once;      // row blocks a cluster works on at once: a group
+                MatvecShape v{parts, c, warps, sm_warps, kc, smem, 0, 0};
+                auto price = [&](uint32_t resident) {
+                    const uint32_t most = std::max(1u, std::min(groups, resident));
+                    v.per = kc < k ? 1u : (groups + most - 1u) / most;
+                    v.clusters = (groups + v.per - 1u) / v.per;
+                    const uint32_t blocks = v.clusters * c;
+                    double deep = (blocks + sms - 1u) / sms;                              // blocks of the fullest SM
+                    const double crowd = std::min<double>(per_sm, 2.0 * deep);
+                    if (crowd > deep) deep += f.uneven * (crowd - deep);
+                    const double chain = v.per * part_slices, busy = (sm_warps == 24u ? f.rate24 : f.rate16) * deep * warps * chain;
+                    const double alone = f.three * std::min(chain, 3.0) + f.slice * std::max(chain - 3.0, 0.0);
+                    return std::cbrt(busy * busy * busy + alone * alone * alone) + v.per * (f.group + f.output * ((m * at_once + 8u * warps - 1u) / (8u * warps))) +
+                           (c > 1u ? f.cluster + f.cluster_group * v.per : 0.0) + f.x * deep * m * k / c +
+                           (kc < k ? f.chunk * ((blocks + sms * per_sm - 1u) / (sms * per_sm)) : 0.0);
+                };
+                const uint32_t room = sms * per_sm / c;
+                double us = price(room);
+                if (us < best && c > 1u) {                               // (the device holds fewer clusters than its blocks make up)
+                    const uint32_t fit = held(c, warps, sm_warps, smem);
+                    us = fit ? price(std::min(room, fit)) : 1e30;
+                }
+                if (us < best) {
+                    best = us;
+                    *out = v;
+                }
+            }
+        }
+    }
+    return best != 1e30;
+}
+
 int launch_one(lexb_gpu* g, const lexb_pipeline* p, const lexb_buffer* x, const lexb_buffer* wq, const lexb_buffer* ws,
                const lexb_buffer* wg, const lexb_buffer* r, lexb_buffer* y, const lexb::GatherDst* gather = nullptr,
                const NextWeights* next = nullptr, Order order = Order{}, lexb_buffer* act = nullptr,
@@ -600,10 +682,10 @@ int launch_one(lexb_gpu* g, const lexb_pipeline* p, const lexb_buffer* x, const 
         a.y = static_cast<float*>(y->ptr);
         a.m = p->m; a.n = p->n; a.k = p->k; a.kc = p->kc;
         auto log2u = [](uint32_t v) { uint32_t l = 0; while (v >>= 1) l++; return l; };
-        a.log_cluster = log2u(p->cluster);
-        a.log_parts = log2u(p->parts);
-        a.log_group = log2u(p->threads / 32u * p->cluster / p->parts);
-        a.log_tokens = log2u(std::min(p->threads / 32u, 2u * p->m - 1u));
+        a.log_cluster = log2u(p->mv.cluster);
+        a.log_parts = log2u(p->mv.parts);
+        a.log_group = log2u(p->mv.warps * p->mv.cluster / p->mv.parts);
+        a.log_tokens = log2u(std::min(p->mv.warps, 2u * p->m - 1u));
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3(p->grid);
         cfg.blockDim = dim3(p->threads);
@@ -615,15 +697,15 @@ int launch_one(lexb_gpu* g, const lexb_pipeline* p, const lexb_buffer* x, const 
             attr[attrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
             attr[attrs++].val.programmaticStreamSerializationAllowed = 1;
         }
-        if (p->cluster > 1u) {
+        if (p->mv.cluster > 1u) {
             attr[attrs].id = cudaLaunchAttributeClusterDimension;
-            attr[attrs].val.clusterDim.x = p->cluster;
+            attr[attrs].val.clusterDim.x = p->mv.cluster;
             attr[attrs].val.clusterDim.y = 1;
             attr[attrs++].val.clusterDim.z = 1;
         }
         cfg.attrs = attr;
         cfg.numAttrs = attrs;
-        const auto kernel = matvec_kernel(p->m, p->k, p->sm_warps);
+        const auto kernel = matvec_kernel(p->m, p->k, p->mv.sm_warps);
         LAUNCH_TRY(cudaLaunchKernelEx(&cfg, kernel, a));
     }
     CUDA_TRY(cudaGetLastError());
@@ -1361,58 +1443,14 @@ int lexb_gemm_fp4_plan(lexb_gpu* g, uint32_t m, uint32_t n, uint32_t k, int resi
         if (n % lexb::MV_ROWS) return bail(fail(LEXB_ERR_SHAPE, "gemm_fp4 (matvec): %u rows per block do not divide n = %u", lexb::MV_ROWS, n));
         if (k % 32u) return bail(fail(LEXB_ERR_SHAPE, "gemm_fp4 (matvec): 32 does not divide k = %u", k));
         if (s.kc % lexb::MV_ROUND) return bail(fail(LEXB_ERR_ARG, "kc = %u is not a multiple of %u", s.kc, lexb::MV_ROUND));
-        // K is always summed in 8 parts (a row's result depends on k alone), held by one block or by a cluster of 2, 4 or
-        // 8; blocks have 8 warps or 4.  A cluster divides the staged x, so that a long k at several tokens still leaves
-        // room for enough warps per SM (m = 4, k = 17408: 157 KB of x in one block, 20 KB each in eight), and puts more
-        // SMs on a matrix with few rows; it costs a barrier across the cluster.  Priced in us, fitted
-        // to a few launches: a slice of 16 x 128 weights takes an SM 0.053 with registers for 24 warps, 0.046 with registers for
-        // 16 (see the kernel), and a warp 0.73 from one to the next; 0.3 for the sums of a group; the cluster's barriers; x from
-        // the L2.  A later choice must win by 3 %.
-        const uint32_t row_blocks = n / lexb::MV_ROWS, slices = (k + lexb::MV_SLICE - 1u) / lexb::MV_SLICE;
-        uint32_t parts = lexb::MV_PARTS;
-        while (parts / 2u >= slices) parts /= 2u;                        // (a short k leaves no warp without a slice)
-        p->parts = parts;
-        const uint32_t part_slices = (slices + parts - 1u) / parts;
-        const uint32_t sms = static_cast<uint32_t>(g->prop.multiProcessorCount);
-        const bool ring = m <= 8u;
-        double best = 1e30;
-        for (uint32_t c = 1; c <= parts; c *= 2u) {
-            for (uint32_t warps = 8; warps >= 4u; warps /= 2u)
-            for (uint32_t sm_warps = 24; sm_warps >= (ring ? 16u : 24u); sm_warps -= 8u) {
-                const uint32_t pp = parts / c;
-                if (warps < pp) continue;
-                uint32_t kc = s.kc;
-                if (!kc) {
-                    // the whole of K if a block's share of x fits in 96 KiB of shared memory (blocks are then persistent
-                    // and stage x once), else the largest multiple of 1024 columns that does
-                    const uint32_t budget = 98304u;
-                    kc = round_up(k, lexb::MV_ROUND);
-                    while (kc > lexb::MV_ROUND && m * lexb::matvec_x_pitch(kc / c) > budget) kc -= lexb::MV_ROUND;
-                }
-                const uint32_t smem = lexb::matvec_smem_bytes(m, kc, warps, c, ring);
-                if (smem > g->smem_optin) continue;
-                uint32_t per_sm = static_cast<uint32_t>(g->prop.sharedMemPerMultiprocessor / (smem + 1024u));
-                per_sm = std::min(per_sm, sm_warps / warps);
-                const uint32_t groups = (row_blocks + warps / pp - 1u) / (warps / pp);      // of the row blocks a cluster works on at once
-                uint32_t clusters = std::max(1u, std::min(groups, sms * per_sm / c));
-                if (c > 1u) {
-                    const uint32_t held = matvec_clusters(matvec_kernel(m, k, sm_warps), c, 32u * warps, smem);
-                    if (!held) continue;
-                    clusters = std::min(clusters, held);
-                }
-                const uint32_t per = kc < k ? 1u : (groups + clusters - 1u) / clusters;
-                clusters = (groups + per - 1u) / per;
-                const uint32_t deep = (clusters * c + sms - 1u) / sms;                       // blocks of the fullest SM
-                const double us = std::max((sm_warps == 24u ? 0.053 : 0.046) * deep * per * warps * part_slices, 0.73 * per * part_slices) + 0.3 * per + (c > 1u ? 1.0 + 0.1 * per : 0.0) +
-                                  2e-5 * deep * m * k / c + (kc < k ? 5.0 : 0.0);
-                if (us < best * 0.97) {
-                    best = us;
-                    p->kc = kc; p->cluster = c; p->sm_warps = sm_warps; p->threads = 32u * warps; p->smem = smem; p->grid = clusters * c;
-                }
-            }
-        }
-        if (best == 1e30)
-            return bail(fail(LEXB_ERR_UNSUPPORTED, "kc = %u needs %u bytes of shared memory", s.kc, lexb::matvec_smem_bytes(m, s.kc, 4, 8, ring)));
+        auto held = [&](uint32_t c, uint32_t warps, uint32_t sm_warps, uint32_t smem) {
+            return matvec_clusters(matvec_kernel(m, k, sm_warps), c, 32u * warps, smem);
+        };
+        MatvecShape v;
+        if (!plan_matvec(m, n, k, s.kc, static_cast<uint32_t>(g->prop.multiProcessorCount), g->smem_optin, g->prop.sharedMemPerMultiprocessor, held, &v))
+            return bail(fail(LEXB_ERR_UNSUPPORTED, "kc = %u needs %u bytes of shared memory", s.kc, lexb::matvec_smem_bytes(m, s.kc, 4, 8, m <= 8u)));
+        p->mv = v;
+        p->kc = v.kc; p->threads = 32u * v.warps; p->smem = v.smem; p->grid = v.clusters * v.cluster;
         snprintf(p->entry, sizeof p->entry, "%s_%u_%u_%u_%u_%u_%u", stem, m, n, k, m, lexb::MV_ROWS, lexb::MV_SLICE);
     }
     *out = p;
@@ -1510,6 +1548,39 @@ int lexb_pipeline_describe(const lexb_pipeline* p, lexb_lowered* out) {
     } else {
         out->bm = p->m; out->bn = lexb::MV_ROWS; out->bk = lexb::MV_SLICE; out->stages = 1;
     }
+    return LEXB_OK;
+}
+
+static lexb_route matvec_route(const MatvecShape& v) {
+    lexb_route r{};
+    r.cluster = v.cluster; r.parts = v.parts; r.groups = v.per; r.kc = v.kc;
+    r.blocks = v.clusters * v.cluster; r.threads = 32u * v.warps;
+    return r;
+}
+
+int lexb_pipeline_route(const lexb_pipeline* p, lexb_route* out) {
+    if (!p || !out) return fail(LEXB_ERR_ARG, "lexb_pipeline_route: null argument");
+    *out = lexb_route{};
+    if (p->kernel == KERNEL_MATVEC) *out = matvec_route(p->mv);
+    else {
+        out->cluster = 1; out->blocks = p->grid; out->threads = p->threads;
+    }
+    out->host_part = p->host_part;
+    return LEXB_OK;
+}
+
+int lexb_matvec_route(uint32_t sms, uint32_t m, uint32_t n, uint32_t k, uint32_t kc, lexb_route* out) {
+    if (!out) return fail(LEXB_ERR_ARG, "lexb_matvec_route: null out");
+    *out = lexb_route{};
+    if (sms == 0 || m == 0 || m > 16u || n == 0 || n % lexb::MV_ROWS || k == 0 || k % 32u || kc % lexb::MV_ROUND)
+        return fail(LEXB_ERR_SHAPE, "the matvec takes m <= 16, n %% %u == 0, k %% 32 == 0, kc %% %u == 0; not m=%u n=%u k=%u kc=%u", lexb::MV_ROWS, lexb::MV_ROUND, m, n, k, kc);
+    const size_t smem_optin = 227u * 1024u, smem_sm = 228u * 1024u;
+    auto held = [&](uint32_t c, uint32_t warps, uint32_t sm_warps, uint32_t smem) {      // (about four fifths: see matvec_clusters)
+        return sms * std::min(static_cast<uint32_t>(smem_sm / (smem + 1024u)), sm_warps / warps) * 4u / (5u * c);
+    };
+    MatvecShape v;
+    if (!plan_matvec(m, n, k, kc, sms, smem_optin, smem_sm, held, &v)) return fail(LEXB_ERR_UNSUPPORTED, "kc = %u leaves no room in shared memory", kc);
+    *out = matvec_route(v);
     return LEXB_OK;
 }
 

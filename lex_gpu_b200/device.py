@@ -25,7 +25,7 @@ SYMBOLS = [
     "lexb_last_error", "lexb_version", "lexb_open", "lexb_close", "lexb_info", "lexb_set_stream", "lexb_get_stream",
     "lexb_sync", "lexb_alloc", "lexb_zeroed", "lexb_wrap", "lexb_free", "lexb_buffer_ptr", "lexb_buffer_bytes",
     "lexb_upload", "lexb_download", "lexb_memset", "lexb_host_alloc", "lexb_host_free", "lexb_gemm_fp4_plan",
-    "lexb_pipeline_free", "lexb_pipeline_describe", "lexb_gemm_fp4_launch", "lexb_gemm_fp4_run_host",
+    "lexb_pipeline_free", "lexb_pipeline_describe", "lexb_pipeline_route", "lexb_matvec_route", "lexb_gemm_fp4_launch", "lexb_gemm_fp4_run_host",
     "lexb_gemm_fp4_enqueue_host",
     "lexb_run_launches", "lexb_list_runs", "lexb_run_each_timed", "lexb_time_launches", "lexb_status_word",
     "lexb_selftest_bounded_wait", "lexb_dequant_fp4_f16", "lexb_shard_rows", "lexb_trace_enable", "lexb_trace_read",
@@ -64,6 +64,11 @@ class Lowered(ctypes.Structure):
                 ("m", c_uint32), ("n", c_uint32), ("k", c_uint32), ("residual", c_uint32),
                 ("bm", c_uint32), ("bn", c_uint32), ("bk", c_uint32), ("stages", c_uint32),
                 ("k_splits", c_uint32), ("scratch_bytes", c_uint64)]
+
+
+class Route(ctypes.Structure):
+    _fields_ = [("cluster", c_uint32), ("parts", c_uint32), ("groups", c_uint32), ("kc", c_uint32), ("blocks", c_uint32),
+                ("threads", c_uint32), ("host_part", c_uint32)]
 
 
 class StepStruct(ctypes.Structure):
@@ -111,6 +116,8 @@ def load_library() -> ctypes.CDLL:
     L.lexb_pipeline_free.argtypes = [vp]
     L.lexb_pipeline_free.restype = None
     L.lexb_pipeline_describe.argtypes = [vp, POINTER(Lowered)]
+    L.lexb_pipeline_route.argtypes = [vp, POINTER(Route)]
+    L.lexb_matvec_route.argtypes = [u32, u32, u32, u32, u32, POINTER(Route)]
     L.lexb_gemm_fp4_launch.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp]
     L.lexb_gemm_fp4_run_host.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp]
     L.lexb_gemm_fp4_enqueue_host.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp]
@@ -147,6 +154,13 @@ def debug_fail_next(site: int, nth: int = 1, cuda_error: int = 0) -> None:
     """Tests of the error paths: the nth call from now that reaches `site` (SITE_ALLOC, SITE_COPY, SITE_LAUNCH,
     SITE_ENCODE) reports a CUDA error instead of being made; site 0 disarms everything."""
     _check(load_library().lexb_debug_fail_next(site, nth, cuda_error))
+
+
+def matvec_route(m: int, n: int, k: int, kc: int = 0, sms: int = 148) -> Route:
+    """How the matvec would lay out a shape on a B200 (host arithmetic only; needs no GPU)."""
+    out = Route()
+    _check(load_library().lexb_matvec_route(sms, m, n, k, kc, byref(out)))
+    return out
 
 
 def prefill_chunks(tokens: int, limit: int = 0, gemm_ok: bool = True) -> list[int]:
@@ -212,6 +226,11 @@ class Pipeline:
     def describe(self) -> Lowered:
         out = Lowered()
         _check(load_library().lexb_pipeline_describe(self.handle, byref(out)))
+        return out
+
+    def route(self) -> Route:
+        out = Route()
+        _check(load_library().lexb_pipeline_route(self.handle, byref(out)))
         return out
 
     def close(self) -> None:

@@ -133,6 +133,21 @@ def test_matvec_over_a_cluster(gpu, n, k):
         assert np.array_equal(L.gemm_fp4(gpu, x[:m].copy(), wq, ws, wg, r=r[:m].copy()), y16[:m]), m
 
 
+@pytest.mark.parametrize("m,n,k,kc,want", [(8, 5136, 17408, 0, "groups"), (8, 17424, 8192, 0, "groups"), (12, 17424, 4096 + 32, 0, "groups"),
+                                           (8, 1040, 17408, 8192, "chunks"), (5, 528, 8192 + 96, 4096, "chunks"), (3, 144, 17408, 2048, "chunks"),
+                                           (16, 5136, 17408, 8192, "chunks")])
+def test_matvec_clusters_with_several_groups_and_with_x_in_chunks(gpu, m, n, k, kc, want):
+    """A cluster that works through several groups of row blocks (the last one not whole), whose sums the other blocks read
+    from alternating buffers; and a cluster that stages x chunk by chunk."""
+    x, wq, ws, wg = inputs.make_case(m, n, k, seed_base=72)
+    route = gpu.plan_gemm_fp4(m, n, k, kernel=1, kc=kc).route()
+    assert route.cluster > 1 and (route.groups > 1 if want == "groups" else route.kc < k)
+    got = L.gemm_fp4(gpu, x, wq, ws, wg, kernel=1, kc=kc)
+    check(got, O.gemm_fp4(x, wq, ws, wg, bk=32))
+    one = L.gemm_fp4(gpu, x[-1:].copy(), wq, ws, wg, kernel=1)            # the same bits by another route
+    assert np.array_equal(got[-1:], one)
+
+
 @pytest.mark.parametrize("m", [1, 3, 8, 13])
 @pytest.mark.parametrize("n,k", [(16, 32), (48, 64), (1040, 96), (4112, 128), (2064, 160), (1040, 224), (4112, 288), (2064, 480), (528, 544), (16, 1056), (272, 2080)])
 def test_matvec_short_and_ragged_k(gpu, m, n, k):
