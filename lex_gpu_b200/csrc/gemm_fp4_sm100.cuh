@@ -127,10 +127,10 @@ gemm_fp4_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const GemmAr
     if (warp == GEMM_WARP_MMA) {
         tmem_alloc(smem_u32(tmem_slot), a.tmem_cols);
         tmem_relinquish();
+        allow_dependents();                                     // (not before this block holds its columns: see tmem_alloc)
     }
     tc_fence_before_sync();
     __syncthreads();
-    allow_dependents();                                         // (not before this block holds its columns: see tmem_alloc)
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
     // (launched with programmatic stream serialization: all of the above runs while the launch ahead drains)

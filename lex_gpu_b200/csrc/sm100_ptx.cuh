@@ -149,8 +149,8 @@ __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* map) {
 
 // ---- tcgen05 / TMEM ---------------------------------------------------------------
 // The allocation waits, without a limit, for columns that another block of the SM holds, and the holder may be a later launch
-// only if it can finish on its own.  So a block lets dependents go (allow_dependents) only behind the barrier that follows
-// its allocation: else the next launch could start beside it, take the columns it is waiting for, and wait for it in turn.
+// only if it can finish on its own.  So a block lets dependents go (allow_dependents) only once it has its columns - in the
+// warp that allocates, or behind the barrier that follows: else the next launch could start beside it, take the columns it is waiting for, and wait for it in turn.
 // With that order every block that is waiting for columns belongs to the newest launch of its stream.
 __device__ __forceinline__ void tmem_alloc(uint32_t smem_result, uint32_t ncols) {   // whole warp
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_result), "r"(ncols)

@@ -23,8 +23,9 @@ def test_dependents_go_only_once_the_block_holds_its_tensor_memory(name, barrier
     for k in kernels:
         alloc = k.index("tmem_alloc")
         held = k.index(barrier, alloc)
-        assert "allow_dependents" in k[held:]
-        assert "allow_dependents" not in k[:held]
+        assert "allow_dependents" not in k[:alloc] and "allow_dependents" in k[alloc:]
+        if "allow_dependents" in k[:held]:                       # then it is the allocating warp itself that does it
+            assert "}" not in k[alloc:k.index("allow_dependents")]
     # the warp that does not meet that barrier (the block-scaled kernel's copy warp) leaves it to the others
     if name == "matmul_q_fp4_sm100.cuh":
         copy_warp = kernels[0][kernels[0].index("tma_load_2d"):kernels[0].index("umma_idesc")]
