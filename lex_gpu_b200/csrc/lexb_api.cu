@@ -405,9 +405,12 @@ struct NextWeights {
 // it has finished (the caller declared them constant, or the step list shows that nothing in flight writes them).
 // `fence`: launched without programmatic stream serialization, so that it starts only when everything ahead of it
 // in the stream is done - the first launch of a step list, behind which the list's own launches overlap one another only.
+// `in_order`: launched with it, but every read waits for the launches ahead, that of weights declared constant too.
 struct Order {
     bool early_weights = false;
     bool fence = false;
+    bool in_order = false;
+    bool early(const lexb_pipeline* p) const { return !in_order && (p->w_const || (early_weights && !p->w_volatile)); }
 };
 
 using MatvecKernel = void (*)(const lexb::MatvecArgs);
@@ -568,7 +571,7 @@ int launch_one(lexb_gpu* g, const lexb_pipeline* p, const lexb_buffer* x, const 
         a.tm = p->tm; a.stages = p->stages; a.w_stages = p->w_stages; a.raw_stages = p->raw_stages; a.k_sub = p->k_sub; a.x_rows = p->x_rows;
         // bit 0: operand-collector hint; bit 1 (two-CTA kernel): the packed weights are constant - declared, or
         // proven from the step list - so their copy and decode may run ahead of the stream's order
-        a.flags = p->flags | ((p->w_const || (order.early_weights && !p->w_volatile)) ? 2u : 0u);
+        a.flags = p->flags | (order.early(p) ? 2u : 0u);
         a.k_splits = p->k_splits; a.kb_per_split = p->kb_per_split; a.partial = p->partial; a.tok_blocks = p->tok_blocks;
         a.tmem_cols = p->tmem_cols; a.m_tiles = p->m_tiles; a.n_acc = p->n_acc;
         a.x_tx_bytes = p->kernel == KERNEL_TCGEN05_PAIR ? (p->m < p->x_rows ? p->m : p->x_rows) * 128u
@@ -626,7 +629,7 @@ int launch_one(lexb_gpu* g, const lexb_pipeline* p, const lexb_buffer* x, const 
         a.m = p->m; a.n = p->n; a.k = p->k; a.stages = p->stages;
         a.k_splits = p->k_splits; a.kb_per_split = p->kb_per_split;
         a.ws_pitch = p->ws_pitch;
-        a.flags = (p->w_const || (order.early_weights && !p->w_volatile)) ? 1u : 0u;
+        a.flags = order.early(p) ? 1u : 0u;
         lexb_pipeline::MapEntry nmaps = maps;         // placeholders when there is no hint (next_grid = 0)
         if (next && next->pipe && next->pipe->kernel == KERNEL_MATMUL_Q && next->pipe->gpu == g && next->wq && next->ws &&
             next->x && (a.flags & 1u) && get_maps(next->pipe, next->x->ptr, next->wq->ptr, next->ws->ptr, &nmaps) == LEXB_OK) {
@@ -968,7 +971,8 @@ int launch_step(lexb_gpu* g, const lexb_step& s, const lexb_step* following = nu
 
 // Issues the steps of a list once, in order, forming runs; `proof` and `first` carry over between the passes of
 // lexb_time_launches.  `first`: nothing of this call has been launched yet - that launch is the call's fence.
-// `lone`: a single step, issued once.  Nothing follows that could use a fence, and behind the launch ahead its set-up is hidden.
+// `lone`: a single step, issued once.  Nothing follows that could use a fence: the launch's set-up is hidden behind the launch
+// ahead, but like a fence it reads nothing before all earlier work of the stream is done, whatever was declared constant.
 int issue_list(lexb_gpu* g, const lexb_step* steps, size_t nsteps, ListProof& proof, bool& first, const lexb_step* after_last, bool lone = false) {
     int rc;
     for (size_t i = 0; i < nsteps;) {
@@ -982,7 +986,8 @@ int issue_list(lexb_gpu* g, const lexb_step* steps, size_t nsteps, ListProof& pr
         const StepRanges sr = step_ranges(steps[i]);
         Order order;
         order.fence = first && !lone;
-        order.early_weights = !lone && sr.valid && proof.weights_untouched(sr);
+        order.in_order = lone;
+        order.early_weights = sr.valid && proof.weights_untouched(sr);
         const lexb_step* following = i + 1 < nsteps ? &steps[i + 1] : after_last;
         if ((rc = launch_step(g, steps[i], following, order))) return rc;
         if (sr.valid) proof.add(sr);

@@ -593,3 +593,32 @@ def test_a_step_whose_weights_an_earlier_step_of_the_list_writes(gpu):
         assert np.array_equal(np.isnan(got), np.isnan(want)) and np.array_equal(np.nan_to_num(got), np.nan_to_num(want))
     assert np.abs(np.nan_to_num(want)).max() > 0
     assert gpu.status_word() == 0
+
+
+@pytest.mark.parametrize("kind", ["block-scaled", "digit rows ahead", "two-CTA"])
+def test_a_list_of_one_step_waits_for_the_work_ahead_of_it(gpu, kind):
+    """lexb_run_launches promises that a call's first launch waits for all earlier work of the stream; so does the only launch
+    of a call, also with weights declared constant: here the launch ahead, which leaves SMs free for the step's blocks,
+    writes the step's packed weights."""
+    n, k = 1024, 4096
+    m = {"block-scaled": 1, "digit rows ahead": 8, "two-CTA": 32}[kind]
+    x, wq, ws, wg = inputs.make_case(m, n, k, seed_base=171)
+    ma, na, ka = 64, n * k // 2 // (64 * 4), 17408
+    xa, wqa, wsa, wga = inputs.make_case(ma, na, ka, seed_base=172)
+    qa, q = L.QBuf(gpu, wqa, wsa, wga), L.QBuf(gpu, wq, ws, wg)
+    ahead = gpu.plan_gemm_fp4(ma, na, ka)
+    assert ahead.describe().grid < 148
+    pipe = gpu.plan_gemm_fp4(m, n, k, weights_constant=True) if kind == "two-CTA" else gpu.plan_matmul_fp4(m, n, k, weights_constant=True)
+    xab, xb, y = gpu.upload(xa), gpu.upload(x), gpu.alloc(4 * m * n)
+    steps = L.StepList([(pipe, q.bind(xb, None, y))])
+    gpu.run(ahead, qa.bind(xab, None, q.wq))                      # (once for all: the codes the step is to read)
+    gpu.sync()
+    gpu.run_launches(steps)
+    want = gpu.download(y, np.float32, (m, n))
+    for _ in range(5):
+        gpu.write(q.wq, 0, wq)
+        gpu.sync()
+        gpu.run(ahead, qa.bind(xab, None, q.wq))
+        gpu.run_launches(steps)
+        assert np.array_equal(gpu.download(y, np.float32, (m, n)), want, equal_nan=True)
+    assert gpu.status_word() == 0
