@@ -1287,9 +1287,14 @@ int lexb_gemm_fp4_plan(lexb_gpu* g, uint32_t m, uint32_t n, uint32_t k, int resi
         }
         // From 5 tokens on the digit rows are derived once per launch by a small kernel ahead of this one
         // (each block deriving them itself is what bounds the kernel there); LEXB_MQ_PRE=0/1 forces either way.
-        // (past 16 tokens there is no in-block path)
+        // (past 16 tokens there is no in-block path.)  Of int16 activations every value is widened in both walks over them, all
+        // of a token for its magnitude and the block's own K range for the digits, so up to 4 tokens the length of the two
+        // decides: in the block against ahead, quant16 and product a call, 28672x4096 at t = 1 / 2 / 3 / 4: -2.5 / -0.9 / +0.8 /
+        // +2.0 us (lengths 32 to 128), 5120x17408: -1.5 / +0.2 / +1.3 / +2.3 (91 to 364), 4096x4096: -1.9 to -1.1 (20 to 80).
         p->x_q16 = t_plan_q16;
-        p->mq_pre = m > 16u || env_u32("LEXB_MQ_PRE", m > 4u ? 1u : 0u) != 0;
+        const uint32_t walk = m * (kb_all + per);
+        const bool ahead = m > 4u || (p->x_q16 && m > 1u && walk > (m == 2u ? 150u : 95u));
+        p->mq_pre = m > 16u || env_u32("LEXB_MQ_PRE", ahead ? 1u : 0u) != 0;
         if (p->mq_pre) {
             const size_t pieces_bytes = static_cast<size_t>(m) * 8u * (k / 2u), sfb_bytes = static_cast<size_t>(kb_all) * lexb::matmul_q_sfb_bytes(m);
             const size_t total = pieces_bytes + sfb_bytes + 4u * lexb::MQ_MAX_TOKENS;

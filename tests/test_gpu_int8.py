@@ -135,11 +135,12 @@ def test_int8_pipeline_describes_itself_and_checks_its_bindings(gpu):
 
 @pytest.mark.parametrize("m,n,k", [(1, 128, 256), (3, 256, 1280), (4, 384, 8448)])
 def test_digit_rows_in_the_block_are_those_of_the_pieces_kernel(gpu, monkeypatch, m, n, k):
-    """Up to 4 tokens every block derives the digit rows of int16 activations itself (one K range per block, or several); a plan
-    that asks for the kernel ahead instead gives the same bits."""
+    """Up to 4 tokens a block may derive the digit rows of int16 activations itself (one K range per block, or several), where
+    they are few; a plan that asks for it, one that asks for the kernel ahead and one that chooses give the same bits."""
     x, wq, ws, wg = inputs.make_case(m, n, k, seed_base=640)
     x = x.astype(np.float32)
     r = inputs.make_residual(m, n, seed_base=640)
-    own = int8_matmul(gpu, x, wq, ws, wg, r)[0]
-    monkeypatch.setenv("LEXB_MQ_PRE", "1")
-    assert np.array_equal(own, int8_matmul(gpu, x, wq, ws, wg, r)[0])
+    chosen = int8_matmul(gpu, x, wq, ws, wg, r)[0]
+    for way in ("0", "1"):
+        monkeypatch.setenv("LEXB_MQ_PRE", way)
+        assert np.array_equal(chosen, int8_matmul(gpu, x, wq, ws, wg, r)[0])
