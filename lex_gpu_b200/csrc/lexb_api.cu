@@ -629,7 +629,9 @@ int launch_one(lexb_gpu* g, const lexb_pipeline* p, const lexb_buffer* x, const 
         a.m = p->m; a.n = p->n; a.k = p->k; a.stages = p->stages;
         a.k_splits = p->k_splits; a.kb_per_split = p->kb_per_split;
         a.ws_pitch = p->ws_pitch;
-        a.flags = order.early(p) ? 1u : 0u;
+        // a step on its own: the pieces kernel can be what it waits behind, and the weights are loaded beside that kernel
+        const uint32_t pieces_fence = p->mq_pre && order.in_order ? 1u : 0u;
+        a.flags = order.early(p) || (pieces_fence && !p->w_volatile) ? 1u : 0u;
         lexb_pipeline::MapEntry nmaps = maps;         // placeholders when there is no hint (next_grid = 0)
         if (next && next->pipe && next->pipe->kernel == KERNEL_MATMUL_Q && next->pipe->gpu == g && next->wq && next->ws &&
             next->x && (a.flags & 1u) && get_maps(next->pipe, next->x->ptr, next->wq->ptr, next->ws->ptr, &nmaps) == LEXB_OK) {
@@ -660,9 +662,9 @@ int launch_one(lexb_gpu* g, const lexb_pipeline* p, const lexb_buffer* x, const 
             pc.numAttrs = pdl ? 1 : 0;
             uint32_t* amax_w = reinterpret_cast<uint32_t*>(p->pre_buf + pieces_bytes + sfb_bytes);
             const float* no_xs = nullptr;
-            if (p->x_q16) LAUNCH_TRY(cudaLaunchKernelEx(&pc, lexb::matmul_q_pieces_kernel<2>, static_cast<const void*>(x->ptr), p->k, p->pre_buf, p->pre_buf + pieces_bytes, amax_w, static_cast<const float*>(xs_q16->ptr)));
-            else if (p->x_f32) LAUNCH_TRY(cudaLaunchKernelEx(&pc, lexb::matmul_q_pieces_kernel<1>, static_cast<const void*>(x->ptr), p->k, p->pre_buf, p->pre_buf + pieces_bytes, amax_w, no_xs));
-            else LAUNCH_TRY(cudaLaunchKernelEx(&pc, lexb::matmul_q_pieces_kernel<0>, static_cast<const void*>(x->ptr), p->k, p->pre_buf, p->pre_buf + pieces_bytes, amax_w, no_xs));
+            if (p->x_q16) LAUNCH_TRY(cudaLaunchKernelEx(&pc, lexb::matmul_q_pieces_kernel<2>, static_cast<const void*>(x->ptr), p->k, p->pre_buf, p->pre_buf + pieces_bytes, amax_w, static_cast<const float*>(xs_q16->ptr), pieces_fence));
+            else if (p->x_f32) LAUNCH_TRY(cudaLaunchKernelEx(&pc, lexb::matmul_q_pieces_kernel<1>, static_cast<const void*>(x->ptr), p->k, p->pre_buf, p->pre_buf + pieces_bytes, amax_w, no_xs, pieces_fence));
+            else LAUNCH_TRY(cudaLaunchKernelEx(&pc, lexb::matmul_q_pieces_kernel<0>, static_cast<const void*>(x->ptr), p->k, p->pre_buf, p->pre_buf + pieces_bytes, amax_w, no_xs, pieces_fence));
         }
         const CUtensorMap& bmap = p->mq_pre ? p->pre_map : maps.map_wq;      // a placeholder without the pieces kernel
 #define LEXB_MQ_LAUNCH(TR, XF, PR) LAUNCH_TRY(cudaLaunchKernelEx(&cfg, lexb::matmul_q_fp4_kernel<TR, XF, PR>, maps.map_wq, maps.map_ws, nmaps.map_wq, nmaps.map_ws, bmap, a))
@@ -890,8 +892,8 @@ int launch_chain(lexb_gpu* g, const lexb_step* steps, size_t count, bool fence) 
                 pdl_next = g->pdl;
                 uint32_t* amax_w = reinterpret_cast<uint32_t*>(buf + pieces_bytes + sfb_bytes);
                 const float* no_xs = nullptr;
-                if (p0->x_f32) LAUNCH_TRY(cudaLaunchKernelEx(&pc, lexb::matmul_q_pieces_kernel<1>, static_cast<const void*>(x->ptr), p0->k, buf, buf + pieces_bytes, amax_w, no_xs));
-                else LAUNCH_TRY(cudaLaunchKernelEx(&pc, lexb::matmul_q_pieces_kernel<0>, static_cast<const void*>(x->ptr), p0->k, buf, buf + pieces_bytes, amax_w, no_xs));
+                if (p0->x_f32) LAUNCH_TRY(cudaLaunchKernelEx(&pc, lexb::matmul_q_pieces_kernel<1>, static_cast<const void*>(x->ptr), p0->k, buf, buf + pieces_bytes, amax_w, no_xs, 0u));
+                else LAUNCH_TRY(cudaLaunchKernelEx(&pc, lexb::matmul_q_pieces_kernel<0>, static_cast<const void*>(x->ptr), p0->k, buf, buf + pieces_bytes, amax_w, no_xs, 0u));
             }
         }
         const uint32_t job_tiles = (p->n + lexb::MQ_ROWS - 1u) / lexb::MQ_ROWS;

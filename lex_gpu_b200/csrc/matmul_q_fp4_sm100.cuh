@@ -759,21 +759,23 @@ matmul_q_fp4_kernel(const __grid_constant__ CUtensorMap tmap_wq, const __grid_co
 //   sfb    [k / 256][2048 or 4096] bytes: per stage the scale blocks of B (rows past 8 m stay zero);
 //   amax   [m]: the token's largest magnitude as f32 bits.
 // It follows the previous launch of the same pipeline in the stream, which may still be reading these
-// buffers: nothing is written before grid_dependency_wait().
+// buffers: nothing is written before grid_dependency_wait().  With `fence` the launch behind it starts only once everything
+// ahead of this one is done, and may then load what this one does not write (the weights) at once.
 // XMODE: 0 = f16 activations, 1 = f32, 2 = int16 activations with one f32 scale per 16 values (`xs`), as
 // lex_msl::int8::quant16 leaves them (crates/lex-msl/src/int8.rs:47-114): the value is q * xs in f32.
 template <int XMODE>
 __global__ void __launch_bounds__(1024, 1)
 matmul_q_pieces_kernel(const void* __restrict__ x, uint32_t k, uint8_t* __restrict__ pieces, uint8_t* __restrict__ sfb,
-                       uint32_t* __restrict__ amax, const float* __restrict__ xs) {
+                       uint32_t* __restrict__ amax, const float* __restrict__ xs, uint32_t fence) {
     constexpr bool XF32 = XMODE == 1, Q16 = XMODE == 2;
     const bool wide = gridDim.x > 16u;                        // tokens = gridDim.x
     const uint32_t sfb_stage = matmul_q_sfb_bytes(gridDim.x);
     __shared__ uint32_t s_amax;
     const uint32_t tok = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
     if (tid == 0) s_amax = 0;
-    allow_dependents();
+    if (!fence) allow_dependents();
     grid_dependency_wait();
+    if (fence) allow_dependents();
     __syncthreads();
     const uint4* xr = XF32 ? reinterpret_cast<const uint4*>(static_cast<const float*>(x) + (size_t)tok * k)
                            : reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(x) + (size_t)tok * k);
