@@ -650,18 +650,16 @@ matmul_q_fp4_kernel(const __grid_constant__ CUtensorMap tmap_wq, const __grid_co
         }
         // ---------------------------------------------------------------- epilogue (warps 2-5)
         if (set == 0u) {
-        // What the epilogue reads from global memory is asked for four tokens at a time (the first four before the
-        // accumulators are complete), and so are the partial products below: one trip to L2 each instead of one per value.
+        // What the epilogue reads from global memory is asked for ahead: the tokens' magnitudes, one a lane, and the residual
+        // four tokens at a time, the first of it before the accumulators are complete.  So are the partial products below: one
+        // trip to L2 each instead of one per value.
         const bool to_partial = a.k_splits > 1u;
+        const uint32_t te_lane = PRE && lane < a.m ? __ldg(a.pre_amax + lane) >> 23 : 0u;      // (at most 32 tokens)
         float r4[4] = {0.f, 0.f, 0.f, 0.f};
-        uint32_t te4[4] = {0, 0, 0, 0};
         auto load4 = [&](uint32_t t0) {
 #pragma unroll
-            for (uint32_t i = 0; i < 4; i++) {
-                if (t0 + i >= a.m) continue;
-                if (PRE) te4[i] = __ldg(a.pre_amax + t0 + i) >> 23;
-                if (a.r && !to_partial) r4[i] = __ldg(a.r + (size_t)(t0 + i) * a.n + n0 + row);
-            }
+            for (uint32_t i = 0; i < 4; i++)
+                if (t0 + i < a.m && a.r && !to_partial) r4[i] = __ldg(a.r + (size_t)(t0 + i) * a.n + n0 + row);
         };
         load4(0);
         uint32_t go = 0;
@@ -680,7 +678,8 @@ matmul_q_fp4_kernel(const __grid_constant__ CUtensorMap tmap_wq, const __grid_co
             const bool two_acc = !wide && KB > 1u;
             float* const out = to_partial ? a.partial + (size_t)split * a.m * a.n : a.y;
             for (uint32_t t0 = 0; t0 < a.m; t0 += 4u) {
-            if (t0) load4(t0);
+            const float r_now[4] = {r4[0], r4[1], r4[2], r4[3]};
+            load4(t0 + 4u);
 #pragma unroll
             for (uint32_t i = 0; i < 4; i++) {
                 const uint32_t t = t0 + i;
@@ -696,12 +695,12 @@ matmul_q_fp4_kernel(const __grid_constant__ CUtensorMap tmap_wq, const __grid_co
                     if (two_acc) c += __uint_as_float(d1[pc]);
                     v += c;
                 }
-                const uint32_t te = PRE ? te4[i] : tok_amax[t] >> 23;
+                const uint32_t te = PRE ? __shfl_sync(0xFFFFFFFFu, te_lane, t) : tok_amax[t] >> 23;
                 const float tscale = te >= 16u ? __uint_as_float((te - 8u) << 23) : 0.0f;   // 2^G, G = E_token - 8
                 v = v * tscale * g;
                 if (row_nan || te == 255u) v = __uint_as_float(0x7FC00000u);
                 const size_t o = (size_t)t * a.n + n0 + row;
-                if (!to_partial && a.r) v += r4[i];
+                if (!to_partial && a.r) v += r_now[i];
                 out[o] = v;
             }
             }
