@@ -271,6 +271,7 @@ matmul_q_fp4_kernel(const __grid_constant__ CUtensorMap tmap_wq, const __grid_co
     if (warp == 1) {
         tmem_alloc(smem_u32(tmem_slot), MQ_TMEM_COLS);
         tmem_relinquish();
+        allow_dependents();                                   // (not before this block holds its columns: see tmem_alloc)
     }
     // Warp 0 has set up every barrier itself and needs nothing from the others: it announces that and
     // goes on to its loads, the other warps meet here (named barrier 2).
@@ -280,7 +281,6 @@ matmul_q_fp4_kernel(const __grid_constant__ CUtensorMap tmap_wq, const __grid_co
     } else {
         tc_fence_before_sync();
         asm volatile("bar.sync 2, %0;" ::"r"(NTHREADS) : "memory");
-        allow_dependents();                  // (not before this block holds its columns: see tmem_alloc; warp 0 does not know)
         tc_fence_after_sync();
         tmem_base = *tmem_slot;
     }
