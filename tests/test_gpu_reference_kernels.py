@@ -19,7 +19,7 @@ import pytest
 
 import lex_gpu_b200 as L
 from lex_gpu_b200 import inputs
-from oracle import oracle as O
+from oracle import build_ref, oracle as O
 from oracle import refkernels as R
 
 pytestmark = pytest.mark.gpu
@@ -43,7 +43,9 @@ def of_scale(got, want):
 
 def need(entry):
     if not R.available(entry):
-        pytest.fail(f"oracle/_ref/{entry}.so is missing: run `python oracle/build_ref.py` where the reference tree is present")
+        say = f"oracle/_ref/{entry}.so is missing: run `python oracle/build_ref.py` where the reference tree is present"
+        # a run that stops at the first failure is to reach the files after this one where the kernels cannot be built
+        (pytest.skip if build_ref.reference_root(None) is None else pytest.fail)(say)
 
 
 # ---------------------------------------------------------------- the emitted decode matvec (f32 x)
