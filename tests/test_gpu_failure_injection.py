@@ -7,6 +7,8 @@ Nothing on the device fails, traps or hangs.  Each case checks that the entry po
 a message, that the device memory it had taken is back (cudaMemGetInfo), and that the next ordinary call on
 the same handle passes parity.
 """
+import time
+
 import numpy as np
 import pytest
 
@@ -93,6 +95,39 @@ def test_copy_failure_in_upload_download_and_the_host_call(gpu):
     gpu.run_host(pipe, hx.ptr, xd, q.wq, q.ws, q.wg, None, yd, hy.ptr)
     err, scale, rel = O.err_of_scale(hy.array(np.float32, (m, n)).copy(), O.gemm_fp4(x, wq, ws, wg))
     assert scale > 1e-3 and err <= 2e-3 and rel <= 2e-3
+    assert gpu.status_word() == 0
+
+
+@pytest.mark.parametrize("site,count", [(D.SITE_COPY, 6), (D.SITE_LAUNCH, 3), (D.SITE_ENCODE, 6)])
+def test_failure_in_every_part_of_the_host_call(gpu, site, count):
+    """The host call in three parts (two pipelines' tensor maps, three copies each way, three launches): whichever of them
+    fails, the call returns an error with nothing of it in flight any more, and the next one is right."""
+    m, n, k = 520, 9472, 512
+    x, wq, ws, wg = inputs.make_case(m, n, k, seed_base=9)
+    q = L.QBuf(gpu, wq, ws, wg)
+    hx, hy = L.HostBuffer(x.nbytes), L.HostBuffer(m * n * 4)
+    xd, yd = gpu.alloc(x.nbytes), gpu.alloc(m * n * 4)
+    y = hy.array(np.float32, (m, n))
+    hx.array(np.float16, (m, k))[:] = x
+    whole = gpu.plan_gemm_fp4(m, n, k)
+    gpu.write(xd, 0, x)
+    gpu.run(whole, q.bind(xd, None, yd))
+    want = gpu.download(yd, np.float32, (m, n))
+    for nth in range(1, count + 1):
+        pipe = gpu.plan_gemm_fp4(m, n, k)                         # (nothing cached yet)
+        assert pipe.route().host_part == 192
+        D.debug_fail_next(site, nth=nth)
+        with pytest.raises(L.LexbError) as e:
+            gpu.run_host(pipe, hx.ptr, xd, q.wq, q.ws, q.wg, None, yd, hy.ptr)
+        assert e.value.code == ERR_CUDA and "injected" in e.value.message
+        y[:] = -1.0
+        hx.array(np.uint8, (x.nbytes,))[:] = 0xFF                # a copy still in flight would read this or undo that
+        gpu.sync()
+        time.sleep(0.02)
+        assert (y == -1.0).all()
+        hx.array(np.float16, (m, k))[:] = x
+        gpu.run_host(pipe, hx.ptr, xd, q.wq, q.ws, q.wg, None, yd, hy.ptr)
+        assert np.array_equal(y, want)
     assert gpu.status_word() == 0
 
 

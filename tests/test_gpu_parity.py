@@ -434,6 +434,33 @@ def test_run_launches_and_timing_entry_points(gpu):
     assert gpu.status_word() == 0
 
 
+def test_one_cta_launches_of_many_shapes_behind_one_another(gpu):
+    """Short rings leave room for several launches' blocks on one SM, with tensor memory for one or two of them: launches
+    of different tiles, depths and row counts queued without a wait in between give what each gives alone."""
+    shapes = [(144, 128, 128), (17, 256, 64), (160, 384, 64), (256, 128, 192), (64, 640, 64), (144, 1280, 128), (33, 128, 320), (150, 256, 128)]
+    runs = []
+    for i, (m, n, k) in enumerate(shapes):
+        x, wq, ws, wg = inputs.make_case(m, n, k, seed_base=300 + i)
+        q, pipe = L.QBuf(gpu, wq, ws, wg), gpu.plan_gemm_fp4(m, n, k, kernel=2)
+        y = gpu.alloc(4 * m * n)
+        runs.append((pipe, q, gpu.upload(x), y, (m, n)))
+        gpu.run(pipe, q.bind(runs[-1][2], None, y))
+        runs[-1] += (gpu.download(y, np.float32, (m, n)),)
+        check(runs[-1][5], O.gemm_fp4(x, wq, ws, wg))
+    rng = np.random.Generator(np.random.PCG64(5))
+    for _ in range(4):
+        for _, _, _, y, (m, n), _ in runs:
+            gpu.memset(y, 0xFF)
+        for i in rng.integers(0, len(runs), 200):
+            pipe, q, xb, y = runs[i][:4]
+            gpu.run(pipe, q.bind(xb, None, y))
+        for pipe, q, xb, y, _, _ in runs:
+            gpu.run(pipe, q.bind(xb, None, y))
+        for _, _, _, y, shape, want in runs:
+            assert np.array_equal(gpu.download(y, np.float32, shape), want)
+    assert gpu.status_word() == 0
+
+
 def test_run_host_copies_in_and_out(gpu):
     m, n, k = 64, 256, 512
     x, wq, ws, wg = inputs.make_case(m, n, k, seed_base=8)
@@ -456,6 +483,7 @@ def test_run_host_in_parts(gpu, m, n, residual):
     r = inputs.make_residual(m, n, seed_base=91) if residual else None
     q, rb = L.QBuf(gpu, wq, ws, wg), gpu.upload(r) if residual else None
     pipe = gpu.plan_gemm_fp4(m, n, k, residual=residual)
+    assert 64 <= pipe.route().host_part < m
     hx, hy = L.HostBuffer(x.nbytes), L.HostBuffer(m * n * 4)
     xd, yd = gpu.alloc(x.nbytes), gpu.alloc(m * n * 4)
     for xi in (x, np.ascontiguousarray(x[::-1])):
@@ -499,7 +527,7 @@ def test_run_host_gives_the_bits_of_a_launch(gpu, m, n, k, splits):
     are the same bits."""
     x, wq, ws, wg = inputs.make_case(m, n, k, seed_base=95)
     q, pipe = L.QBuf(gpu, wq, ws, wg), gpu.plan_gemm_fp4(m, n, k)
-    assert pipe.describe().k_splits == splits
+    assert pipe.describe().k_splits == splits and 64 <= pipe.route().host_part < m
     hx, hy = L.HostBuffer(x.nbytes), L.HostBuffer(m * n * 4)
     hx.array(np.float16, (m, k))[:] = x
     xd, yd = gpu.upload(x), gpu.alloc(m * n * 4)
