@@ -205,7 +205,9 @@ LEXB_API int lexb_interleave_rows(lexb_gpu* gpu, const lexb_buffer* a, const lex
                                   lexb_buffer* out);
 
 /* The call a runtime makes per prefill chunk with host activations: copy x from host memory
- * into x_dev, launch, copy y_dev back into y_host, wait.  The weights stay resident, as
+ * into x_dev, launch, copy y_dev back into y_host, wait.  From and to pinned memory, with a wide n and many tokens, it does
+ * so part by part of the tokens (lexb_route.host_part), y leaving while x still arrives; y is the same bits either way.
+ * Buffers that overlap (x and y in one host arena) are always copied in whole before any of y is copied out.  The weights stay resident, as
  * lex-rt keeps them (Runner::forward_with writes only per-step inputs,
  * crates/lex-rt/src/qwen_run.rs:2348-2373, and downloads the result, :2401-2404). */
 LEXB_API int lexb_gemm_fp4_run_host(lexb_gpu* gpu, const lexb_pipeline* p, const void* x_host, lexb_buffer* x_dev,

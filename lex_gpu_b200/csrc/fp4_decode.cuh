@@ -23,10 +23,12 @@
 // (e = 0.5, 1, 2, 4: e A + e d rounds to e A, because |e d| is less than half a unit of e A; e = 1.5, 3, 6: e A is within
 // 1.5 units of B and e d decides between its two neighbours the right way; the u taken off and put back keeps the
 // addend's sign that of the code, so that code 8 gives -0.)  e * (u + d) is exact in f16 for A >= 2^-10.  Checked against
-// the table method for every mantissa of wg, all scale bytes and codes.  Per weight: half a conversion of two codes
+// the table method for every mantissa of wg, all scale bytes and codes, once; tests/test_fp4_products.py restates it for a
+// spread of mantissas and those beside a tie.  Per weight: half a conversion of two codes
 // (`cvt.rn.f16x2.e2m1x2`, integer pipe) and one FP16 multiply and one fused multiply-add per two weights (the FP16
-// pipe, idle otherwise), 2.3 instructions in all, where the table takes 5.7, most of them in the integer pipe:
-// 39 weights per clock and SM against 21.5.
+// pipe, idle otherwise), 2.4 instructions in all with the factors, where the table takes 5.7, most of them in the integer
+// pipe.  Measured, 16 warps that store what they decode to shared memory: 33 weights per clock and SM with the choice
+// between the methods in place (49, what the stores allow, without it) against 21.5 by the table.
 //
 // Table (when a scale or row scale is outside the range of the products: see RowScale).  A group of 16 weights
 // shares its scale, so it has only 8 distinct magnitudes.  They are computed once per group (16 f32 multiplies, 4 packed

@@ -757,7 +757,7 @@ StepRanges step_ranges(const lexb_step& s) {
 }
 
 // What the steps of one lexb_run_launches / lexb_time_launches call have written so far.  The call's first launch
-// is a fence (it starts when all earlier work of the stream is done), so a later step whose packed weights meet
+// is a fence (it starts when all earlier work of the stream is done; the only launch of a call reads nothing before that), so a later step whose packed weights meet
 // none of these ranges reads weights that nothing in flight writes: its kernel may load them ahead of the
 // stream's order.  That is proven here from the list, as the reference's in-order contract
 // (crates/lex-cuda/src/device.rs:629-672) leaves no other way to know it.
@@ -1355,11 +1355,13 @@ int lexb_gemm_fp4_plan(lexb_gpu* g, uint32_t m, uint32_t n, uint32_t k, int resi
         // each split takes whole blocks of 256 columns (at least 4) and writes a partial product that a second
         // launch sums.  Smaller tiles: more of them; every weight is decoded once per tile of tokens, but a tile's
         // partial product and its store shrink with it and fewer splits are needed.  (Below 256 tokens a K step
-        // costs the same: it is the decode that bounds it, not the MMAs.)
-        // Every (tile, splits) pair is priced with figures fitted to 159 launches timed on a B200 (us; rms error
-        // 4 %): 4.5 overall; per wave of tiles 8.05 / 5.3 / 4.0 / 4.1 for a block's start and its store of a
-        // 512 / 256 / 128 / 64-token tile and 0.559 / 0.311 / 0.310 / 0.304 per K step; for the reduction launch its
-        // bytes at 3.33 TB/s minus 1.1.  The cheapest wins; a smaller tile or a further split must win by 2 %.
+        // costs about the same: it is the decode that bounds it, not the MMAs.)
+        // Every (tile, splits) pair is priced with figures fitted to 159 launches timed on a B200 (us): 4.5 overall; per
+        // wave of tiles 8.05 / 5.3 / 4.0 / 4.1 for a block's start and its store of a 512 / 256 / 128 / 64-token tile and
+        // 0.559 / 0.311 / 0.310 / 0.304 per K step; for the reduction launch its bytes at 3.33 TB/s minus 1.1.  The cheapest
+        // wins; a smaller tile or a further split must win by 2 %.  The fit (rms error 4 %) is that of the table decode: with
+        // the products a K step of the tiles up to 128 tokens takes 0.20-0.31 (17408 rows, k = 2048 to 8192), so they and
+        // their splits are priced up to a third too dear.
         const uint32_t sm_pairs = static_cast<uint32_t>(g->prop.multiProcessorCount) / 2u;
         const uint32_t raw_blocks = k / lexb::PAIR_RAW_K;
         uint32_t splits = s.k_splits ? s.k_splits : 1u;

@@ -11,8 +11,7 @@
 // The tensor core does the whole decode: `tcgen05.mma.kind::mxf4nvf4.block_scale` multiplies packed
 // E2M1 codes by a UE4M3 scale per 16 values of K, which is exactly how wq and ws are stored.  The
 // packed codes go from global memory to shared memory by TMA and are never touched by a thread; the
-// integer pipe, which bounds the table-lookup decode of `matvec_fp4_kernel`, is idle here and the
-// kernel streams at memory speed.
+// issue slots that the decode of `matvec_fp4_kernel` takes are idle here and the kernel streams at memory speed.
 //
 // The activations have to be E2M1 as well.  Each token (f16, or f32) is split into MQ_PIECES = 8 rows of
 // 2-bit digits: inside a group of 16 values with largest exponent E, a value is sign * I * 2^(E-15) with a
@@ -197,7 +196,7 @@ __device__ __forceinline__ uint32_t mq_sfb_offset(uint32_t n, uint32_t grp, bool
 }
 
 // PRE = false: 576 threads, piece warps 10-17 derive the tokens' digit rows in every block (no second launch:
-// best for up to 4 tokens).  PRE = true: 320 threads, the digit rows were written by matmul_q_pieces_kernel
+// best for up to 4 tokens, of int16 ones where they are short).  PRE = true: 320 threads, the digit rows were written by matmul_q_pieces_kernel
 // and the copy engine brings each stage's part of them with the weights.
 // XMODE: 0 = f16 activations, 1 = f32, 2 = int16 with one f32 scale per 16 values (the value is q * xs in f32).
 template <bool TRACE, int XMODE, bool PRE>

@@ -7,12 +7,13 @@
 // quantises x to int16; crates/lex-front/src/llama.rs:444-499 keeps weights in f32); this
 // one keeps gemm_fp4's semantics so one oracle covers every m.
 //
-// K is summed in 8 parts, slices of 128 columns dealt out in turns (part p: slices p, p + 8, ...), a warp each.  A
-// block of 8 warps has all parts of 16 rows at a time, so that it reads 512 contiguous bytes of each row per round; or a
-// cluster of 2, 4 or 8 blocks shares the parts, each block with as many more row blocks, and adds them up through
-// distributed shared memory, always in the order of the parts.  What the cluster divides is the staged x: m = 4 at
-// k = 17408 is 157 KB of it, one block an SM with x read twice over by each; divided by 8, five blocks of 4 warps
-// (5120x17408 on a B200: 57.4 -> 23.5 us, back to back with other weights each time; W alone takes 7.5 at the copy rate).
+// K is summed in 8 parts, slices of 128 columns dealt out in turns (part p: slices p, p + 8, ...), a warp each; a k of 4
+// slices or fewer in 4, 2 or 1.  A block of 8 warps has all parts of 16 rows at a time, so that it reads 512 contiguous
+// bytes of each row per round; or a cluster of 2, 4 or 8 blocks shares the parts, each block with as many more row blocks,
+// and adds them up through distributed shared memory, always in the order of the parts.  What the cluster divides is the
+// staged x: m = 4 at k = 17408 is 157 KB of it, one block an SM with x read twice over by each; divided by 8, four blocks of
+// 4 warps or two of 8 (5120x17408 on a B200: 57.4 -> 22.1 us, back to back with other weights each time; W alone takes 7.7
+// at the copy rate).
 // Inside a slice, lane (g = lane/4, t = lane%4) owns rows g and g+8 and the two groups of 16
 // columns 32t..32t+31: one 16-byte load of codes per row, two scale bytes, the factors of two
 // groups per row.  The multiply-accumulate runs on the tensor cores (mma.sync m16n8k16,
@@ -44,7 +45,7 @@ constexpr uint32_t MV_RED_PITCH = 20;
 __host__ __device__ constexpr uint32_t matvec_red_floats(uint32_t m) { return (m <= 8u ? 8u : 16u) * MV_RED_PITCH; }
 // The packed weights come through a ring in shared memory filled by asynchronous copies (cp.async): a warp keeps
 // MV_DEPTH slices in flight, each lane copying exactly the 2 x 16 bytes of codes it will decode itself (so the ring
-// is a per-lane FIFO and its reads are conflict-free) and one lane of each quad the quad's 2 x 8 scale bytes.
+// is a per-lane FIFO and its reads are conflict-free) and two lanes of each quad the quad's 2 x 8 scale bytes.
 // With the loads in registers one slice ahead, the warps spent most of their time waiting for memory.
 constexpr uint32_t MV_DEPTH = 3;
 constexpr uint32_t MV_STAGE_BYTES = 2u * 512u + 128u;              // codes of row g, codes of row g + 8, scale bytes
@@ -99,9 +100,10 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 
 // HI: m > 8, a second group of 8 tokens, whose staged x leaves no room for the ring: the weights come through registers,
 // one slice ahead.  RAGGED: k % 128 != 0.
-// WARPS: warps per SM the registers are cut to, 24 (80 registers a thread) or 16 (128).  Held to 64 registers (32 warps) the
-// loop spills; with 16 warps the compiler overlaps the decode of one word with the next and with the multiply, which is worth
-// more than the other warps (17408x5120, m = 1: 21.4 us with 32 warps, 19.1 with 16) wherever the row blocks divide as well.
+// WARPS: warps per SM the registers are cut to, 24 (80 registers a thread) or 16 (128).  With 16 the compiler overlaps the
+// decode of one word with the next and with the multiply, which is worth more than the other warps (17408x5120, m = 1: 18.8 us
+// with 16; 21.4 with 32, whose 64 registers spill) wherever the row blocks divide as well.  At 80 registers only the instance
+// for m > 8 with a ragged k spills (20 bytes).
 template <bool HI, bool RAGGED, uint32_t WARPS>
 __global__ void __launch_bounds__(MV_THREADS, WARPS / MV_WARPS) matvec_fp4_kernel(const MatvecArgs a) {
     constexpr bool RING = !HI;
