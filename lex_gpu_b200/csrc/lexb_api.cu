@@ -24,6 +24,7 @@
 #include "../../include/lexb.h"
 #include "gemm_fp4_sm100.cuh"
 #include "gemm_fp4_sm100_pair.cuh"
+#include "gemm_fp4_few_sm100.cuh"
 #include "matvec_fp4_sm100.cuh"
 #include "matmul_q_fp4_sm100.cuh"
 #include "matmul_q_chain_sm100.cuh"
@@ -100,7 +101,8 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-enum { KERNEL_MATVEC = 1, KERNEL_TCGEN05 = 2, KERNEL_TCGEN05_PAIR = 3, KERNEL_MATMUL_Q = 4 };
+// (KERNEL_FEW: what a launch of a pipeline of kernel 1 or 3 may run instead; no selector)
+enum { KERNEL_MATVEC = 1, KERNEL_TCGEN05 = 2, KERNEL_TCGEN05_PAIR = 3, KERNEL_MATMUL_Q = 4, KERNEL_FEW = 5 };
 thread_local bool t_plan_q16 = false;      // set by lexb_matmul_int8_plan around its call of lexb_gemm_fp4_plan
 thread_local float* t_plan_partial = nullptr;      // a split-K workspace to borrow instead of allocating one (run_host_in_parts)
 
@@ -129,6 +131,8 @@ struct lexb_gpu {
     cudaDeviceProp prop{};
     EncodeTiledFn encode_tiled = nullptr;
     size_t smem_optin = 0;
+    std::mutex held_lock;
+    uint32_t held[lexb::FEW_MAX_CLUSTER + 1u] = {};      // clusters of that many blocks the device holds (held_clusters)
     // lexb_gemm_fp4_run_host in parts: one copy stream each way beside the launch stream
     static constexpr uint32_t HOST_PARTS = 4;
     struct HostPath {
@@ -189,6 +193,9 @@ struct lexb_pipeline {
     };
     mutable std::vector<MapEntry> maps;
     mutable std::mutex maps_lock;
+    // few tokens: what a launch without a gather runs instead (gemm_fp4_few_kernel)
+    lexb_pipeline* few = nullptr;
+    uint32_t cluster = 1;
     // lexb_gemm_fp4_run_host in parts: tokens of a part (0: whole), the pipelines of a part and of a shorter last one
     uint32_t host_part = 0;
     mutable lexb_pipeline* host_pipes[2] = {nullptr, nullptr};
@@ -362,7 +369,7 @@ int encode_2d(const lexb_pipeline* p, CUtensorMap* map, CUtensorMapDataType dt, 
 // Tensor maps for one binding, cached by the device pointers they were encoded for.
 int get_maps(const lexb_pipeline* p, const void* x, const void* wq, const void* ws, lexb_pipeline::MapEntry* out) {
     std::lock_guard<std::mutex> lk(p->maps_lock);
-    const bool pair = p->kernel == KERNEL_TCGEN05_PAIR || p->kernel == KERNEL_MATMUL_Q;
+    const bool pair = p->kernel == KERNEL_TCGEN05_PAIR || p->kernel == KERNEL_MATMUL_Q || p->kernel == KERNEL_FEW;
     for (const auto& e : p->maps)
         if (e.x == x && (!pair || (e.wq == wq && e.ws == ws))) {
             *out = e;
@@ -412,6 +419,12 @@ struct Order {
     bool in_order = false;
     bool early(const lexb_pipeline* p) const { return !in_order && (p->w_const || (early_weights && !p->w_volatile)); }
 };
+
+using FewKernel = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const lexb::FewArgs);
+FewKernel few_kernel(uint32_t m) {
+    const uint32_t cols = lexb::few_cols(m);
+    return cols == 16u ? lexb::gemm_fp4_few_kernel<16> : cols == 32u ? lexb::gemm_fp4_few_kernel<32> : lexb::gemm_fp4_few_kernel<64>;
+}
 
 using MatvecKernel = void (*)(const lexb::MatvecArgs);
 MatvecKernel matvec_kernel(uint32_t m, uint32_t k, uint32_t sm_warps) {
@@ -513,6 +526,65 @@ bool plan_matvec(uint32_t m, uint32_t n, uint32_t k, uint32_t kc_asked, uint32_t
     return best != 1e30;
 }
 
+// Clusters of c blocks that the device holds at once with one block an SM, asked for once per handle.
+uint32_t held_clusters(lexb_gpu* g, uint32_t c) {
+    const uint32_t sms = static_cast<uint32_t>(g->prop.multiProcessorCount);
+    if (c == 1u) return sms;
+    std::lock_guard<std::mutex> lk(g->held_lock);
+    uint32_t& held = g->held[c];
+    if (!held) {
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(c);
+        cfg.blockDim = dim3(lexb::FEW_THREADS);
+        cfg.dynamicSmemBytes = static_cast<unsigned>(g->smem_optin);
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = c;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int clusters = 0;
+        if (cudaOccupancyMaxActiveClusters(&clusters, lexb::gemm_fp4_few_kernel<16>, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            clusters = 0;
+        }
+        held = clusters > 0 ? std::min(static_cast<uint32_t>(clusters), sms / c) : ~0u;
+    }
+    return held == ~0u ? 0u : held;
+}
+
+// The few-token kernel's launch for a pipeline, if it takes the shape.
+int plan_few(lexb_gpu* g, lexb_pipeline* p) {
+    const uint32_t m = p->m, n = p->n, k = p->k;
+    if (m > lexb::FEW_MAX_TOKENS || n % lexb::FEW_ROWS || k % lexb::FEW_K) return LEXB_OK;
+    const uint32_t tiles = n / lexb::FEW_ROWS, U = k / lexb::FEW_K;
+    const uint32_t forced = env_u32("LEXB_FEW_C", 0);
+    uint32_t best_c = 0, best_clusters = 0;
+    double best = 1e30;
+    for (uint32_t c = 1; c <= lexb::FEW_MAX_CLUSTER; c++) {
+        if (forced && c != forced) continue;
+        const uint32_t clusters = std::min(held_clusters(g, c), tiles);
+        if (!clusters || (tiles / clusters) * U < c) continue;
+        const uint32_t blocks = ((tiles + clusters - 1u) / clusters * U + c - 1u) / c;
+        const double us = blocks * 0.4 + (c > 1u ? 1.0 : 0.0);
+        if (us < best) { best = us; best_c = c; best_clusters = clusters; }
+    }
+    if (!best_c) return LEXB_OK;
+    lexb_pipeline* f = new (std::nothrow) lexb_pipeline();
+    if (!f) return fail(LEXB_ERR_ARG, "out of host memory");
+    f->gpu = g;
+    f->kernel = KERNEL_FEW;
+    f->m = m; f->n = n; f->k = k; f->tm = m;
+    f->residual = p->residual; f->w_const = p->w_const; f->w_volatile = p->w_volatile;
+    f->cluster = best_c; f->grid = best_c * best_clusters; f->threads = lexb::FEW_THREADS;
+    f->stages = env_u32("LEXB_FEW_SX", m <= 32u ? 4u : 3u); f->raw_stages = env_u32("LEXB_FEW_SR", m <= 32u ? 5u : 4u);
+    f->smem = lexb::few_smem_bytes(m, f->stages, f->raw_stages);
+    if (f->smem > g->smem_optin) { delete f; return LEXB_OK; }
+    p->few = f;
+    return LEXB_OK;
+}
+
 int launch_one(lexb_gpu* g, const lexb_pipeline* p, const lexb_buffer* x, const lexb_buffer* wq, const lexb_buffer* ws,
                const lexb_buffer* wg, const lexb_buffer* r, lexb_buffer* y, const lexb::GatherDst* gather = nullptr,
                const NextWeights* next = nullptr, Order order = Order{}, lexb_buffer* act = nullptr,
@@ -522,6 +594,8 @@ int launch_one(lexb_gpu* g, const lexb_pipeline* p, const lexb_buffer* x, const 
     const bool silu = act != nullptr || (gather && gather->silu);
     if (!p) return fail(LEXB_ERR_ARG, "null pipeline");
     if (p->gpu != g) return fail(LEXB_ERR_ARG, "pipeline was planned on another gpu handle");
+    const bool fuses_silu = p->kernel == KERNEL_TCGEN05_PAIR && !p->residual;
+    if (p->few && !gather) p = p->few;
     const size_t m = p->m, n = p->n, k = p->k;
     int rc;
     if ((rc = check_buf(x, g, m * k * (p->x_f32 ? 4 : 2), p->x_q16 ? "xq" : "x"))) return rc;
@@ -534,7 +608,7 @@ int launch_one(lexb_gpu* g, const lexb_pipeline* p, const lexb_buffer* x, const 
     if ((rc = check_buf(ws, g, n * k / 16, "ws"))) return rc;
     if ((rc = check_buf(wg, g, n * 4, "wg"))) return rc;
     if (silu) {
-        if (p->kernel != KERNEL_TCGEN05_PAIR || p->residual)
+        if (!fuses_silu)
             return fail(LEXB_ERR_UNSUPPORTED, "silu(gate) * up is fused into the two-CTA GEMM only (m > 8, n %% 128 == 0, k %% 256 == 0, no residual)");
         if (act && (rc = check_buf(act, g, m * (n / 2) * 2, "act"))) return rc;
     } else if (!gather && (rc = check_buf(y, g, m * n * 4, "y"))) return rc;
@@ -613,6 +687,33 @@ int launch_one(lexb_gpu* g, const lexb_pipeline* p, const lexb_buffer* x, const 
             launch.cfg.dynamicSmemBytes = p->smem;
             LAUNCH_TRY(cudaLaunchKernelEx(&launch.cfg, lexb::gemm_fp4_tcgen05_kernel, maps.map, a));
         }
+    } else if (p->kernel == KERNEL_FEW) {
+        lexb_pipeline::MapEntry maps;
+        if ((rc = get_maps(p, x->ptr, wq->ptr, ws->ptr, &maps))) return rc;
+        lexb::FewArgs a{};
+        a.wg = static_cast<const float*>(wg->ptr);
+        a.r = r ? static_cast<const float*>(r->ptr) : nullptr;
+        a.y = y ? static_cast<float*>(y->ptr) : nullptr;
+        a.act = act ? static_cast<uint16_t*>(act->ptr) : nullptr;
+        a.status = g->d_status;
+        a.m = p->m; a.n = p->n; a.k = p->k;
+        a.cluster = p->cluster; a.x_stages = p->stages; a.raw_stages = p->raw_stages;
+        a.flags = order.early(p) ? 2u : 0u;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(p->grid);
+        cfg.blockDim = dim3(p->threads);
+        cfg.dynamicSmemBytes = p->smem;
+        cfg.stream = g->stream;
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = p->cluster;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = pdl ? 2 : 1;
+        LAUNCH_TRY(cudaLaunchKernelEx(&cfg, few_kernel(p->m), maps.map, maps.map_wq, maps.map_ws, a));
     } else if (p->kernel == KERNEL_MATMUL_Q) {
         lexb_pipeline::MapEntry maps;
         if ((rc = get_maps(p, x->ptr, wq->ptr, ws->ptr, &maps))) return rc;
@@ -1041,6 +1142,9 @@ int lexb_open(int device, lexb_gpu** out) {
     if (cudaFuncSetAttribute(lexb::gemm_fp4_tcgen05_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem) != cudaSuccess ||
         cudaFuncSetAttribute(lexb::gemm_fp4_tcgen05_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem) != cudaSuccess ||
         cudaFuncSetAttribute(lexb::gemm_fp4_tcgen05_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem) != cudaSuccess ||
+        cudaFuncSetAttribute(lexb::gemm_fp4_few_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem) != cudaSuccess ||
+        cudaFuncSetAttribute(lexb::gemm_fp4_few_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem) != cudaSuccess ||
+        cudaFuncSetAttribute(lexb::gemm_fp4_few_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem) != cudaSuccess ||
         cudaFuncSetAttribute(lexb::matvec_fp4_kernel<true, true, 24>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem) != cudaSuccess ||
         cudaFuncSetAttribute(lexb::matvec_fp4_kernel<true, false, 24>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem) != cudaSuccess ||
         cudaFuncSetAttribute(lexb::matvec_fp4_kernel<false, true, 24>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem) != cudaSuccess ||
@@ -1467,6 +1571,7 @@ int lexb_gemm_fp4_plan(lexb_gpu* g, uint32_t m, uint32_t n, uint32_t k, int resi
         p->kc = v.kc; p->threads = 32u * v.warps; p->smem = v.smem; p->grid = v.clusters * v.cluster;
         snprintf(p->entry, sizeof p->entry, "%s_%u_%u_%u_%u_%u_%u", stem, m, n, k, m, lexb::MV_ROWS, lexb::MV_SLICE);
     }
+    if (!s.kernel && !s.tm && !s.stages && !s.kc && !s.w_stages && !s.k_splits && env_u32("LEXB_FEW", 0u) && (rc = plan_few(g, p))) return bail(rc);
     *out = p;
     return LEXB_OK;
 }
@@ -1530,6 +1635,7 @@ int lexb_quant16(lexb_gpu* g, uint32_t m, uint32_t k, int x_half, const lexb_buf
 void lexb_pipeline_free(lexb_pipeline* p) {
     if (!p) return;
     for (lexb_pipeline* part : p->host_pipes) lexb_pipeline_free(part);
+    delete p->few;
     if (p->partial || p->pre_buf) {
         cudaSetDevice(p->gpu->device);
         if (!p->partial_borrowed) cudaFree(p->partial);

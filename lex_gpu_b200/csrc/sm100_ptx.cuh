@@ -264,6 +264,14 @@ __device__ __forceinline__ void umma2_ts_flag(uint32_t d_tmem, uint32_t a_tmem, 
                  ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(idesc), "r"(UMMA_DESC_HI_SW128), "r"(accumulate)
                  : "memory");
 }
+// ... of one CTA: M = 128
+__device__ __forceinline__ void umma1_ts_flag(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 db;\n\tsetp.ne.b32 p, %5, 0;\n\t"
+                 "mov.b64 db, {%2, %4};\n\t"
+                 "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, p;\n\t}"
+                 ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(idesc), "r"(UMMA_DESC_HI_SW128), "r"(accumulate)
+                 : "memory");
+}
 // Each lane of the warp writes 32 consecutive 32-bit columns of its own TMEM lane (the warp's lane quarter).
 __device__ __forceinline__ void tmem_st_32x32b_x32(uint32_t taddr, const uint32_t (&v)[32]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
