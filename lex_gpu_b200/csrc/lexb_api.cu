@@ -15,6 +15,7 @@
 #include <cstring>
 #include <mutex>
 #include <new>
+#include <queue>
 #include <map>
 #include <string>
 #include <tuple>
@@ -118,13 +119,20 @@ struct lexb_gpu {
     // Job tables of chained runs, kept by content: a decode loop issues the same lists token after token, and a
     // table found here needs no copy in front of its launch (a copy would put the launch behind the whole
     // kernel before it).  A table is never written again once copied.
-    struct ChainTable { std::vector<lexb::MqChainJob> host; lexb::MqChainJob* dev; };
+    // (the jobs, then the table of tiles, which follows from them and the device)
+    struct ChainTable { std::vector<lexb::MqChainJob> host; std::vector<lexb::MqChainTile> tiles; uint32_t grid; lexb::MqChainJob* dev; };
     std::unordered_multimap<uint64_t, ChainTable> chain_tables;
     // Digit rows of a run's activations (matmul_q_pieces_kernel's output: [8 m][k / 2] digit rows, [k / 256][2048]
-    // scale blocks, [m] magnitudes), one buffer per activation buffer, shape and stream: rewritten by every run that
-    // reads that x, in stream order.
-    struct ChainPre { uint8_t* buf; CUtensorMap map; };
-    std::map<std::tuple<const void*, uint32_t, uint32_t, bool, cudaStream_t>, ChainPre> chain_pre;
+    // scale blocks, [m] magnitudes per activation buffer), one arena per stream: every run on that stream writes its
+    // buffers' digit rows into it from the start, in stream order.  An arena that has become too small is replaced by one
+    // of at least twice its size and kept until the handle closes (launches in flight may read it).
+    struct ChainArena {
+        uint8_t* buf = nullptr;
+        size_t bytes = 0;
+        std::map<std::tuple<size_t, uint32_t, uint32_t>, CUtensorMap> maps;      // of the digit rows at an offset, by tokens and K
+    };
+    std::map<cudaStream_t, ChainArena> chain_arenas;
+    std::vector<uint8_t*> retired_arenas;
     unsigned long long* d_trace = nullptr;   // phase timers of the last two-CTA launch, when tracing is on
     size_t trace_ctas = 0;
     uint32_t trace_toggle = 0;
@@ -176,6 +184,7 @@ struct lexb_pipeline {
     bool w_const = false;       // the caller declared wq/ws constant (LEXB_SCHED_WEIGHTS_CONSTANT): loaded ahead of the stream's order
                                 // by the kernels that can (block-scaled kernel, two-CTA GEMM)
     bool w_volatile = false;    // ... or said they may change (LEXB_SCHED_WEIGHTS_MAY_CHANGE): never loaded early, not even in a list
+    bool splits_asked = false;  // ... whose K split the caller gave
     bool mq_pre = false;        // ... with the tokens' digit rows from the pieces kernel: buffers and their tensor map
     uint8_t* pre_buf = nullptr; // [8 m][k / 2] digit rows, then [k / 256][2048] scale blocks, then [m] magnitudes
     CUtensorMap pre_map{};
@@ -424,6 +433,11 @@ using FewKernel = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorM
 FewKernel few_kernel(uint32_t m) {
     const uint32_t cols = lexb::few_cols(m);
     return cols == 16u ? lexb::gemm_fp4_few_kernel<16> : cols == 32u ? lexb::gemm_fp4_few_kernel<32> : lexb::gemm_fp4_few_kernel<64>;
+}
+
+using PiecesKernel = void (*)(const lexb::MqPiecesList, uint32_t);
+PiecesKernel pieces_kernel(int xmode) {
+    return xmode == 2 ? lexb::matmul_q_pieces_kernel<2> : xmode == 1 ? lexb::matmul_q_pieces_kernel<1> : lexb::matmul_q_pieces_kernel<0>;
 }
 
 using MatvecKernel = void (*)(const lexb::MatvecArgs);
@@ -751,7 +765,7 @@ int launch_one(lexb_gpu* g, const lexb_pipeline* p, const lexb_buffer* x, const 
         cfg.attrs = attr;
         cfg.numAttrs = (g->pdl && (!order.fence || p->mq_pre)) ? 1 : 0;      // (behind the pieces kernel, that one is the fence)
         a.trace = (g->d_trace && p->grid <= g->trace_ctas) ? g->d_trace : nullptr;
-        const size_t pieces_bytes = static_cast<size_t>(p->m) * 8u * (p->k / 2u), sfb_bytes = static_cast<size_t>(p->k / lexb::MQ_STAGE_K) * lexb::matmul_q_sfb_bytes(p->m);
+        const size_t pieces_bytes = lexb::matmul_q_pieces_bytes(p->m, p->k), sfb_bytes = lexb::matmul_q_sfb_total(p->m, p->k);
         if (p->mq_pre) {
             a.pre_sfb = p->pre_buf + pieces_bytes;
             a.pre_amax = reinterpret_cast<const uint32_t*>(p->pre_buf + pieces_bytes + sfb_bytes);
@@ -761,11 +775,9 @@ int launch_one(lexb_gpu* g, const lexb_pipeline* p, const lexb_buffer* x, const 
             pc.stream = g->stream;
             pc.attrs = attr;
             pc.numAttrs = pdl ? 1 : 0;
-            uint32_t* amax_w = reinterpret_cast<uint32_t*>(p->pre_buf + pieces_bytes + sfb_bytes);
-            const float* no_xs = nullptr;
-            if (p->x_q16) LAUNCH_TRY(cudaLaunchKernelEx(&pc, lexb::matmul_q_pieces_kernel<2>, static_cast<const void*>(x->ptr), p->k, p->pre_buf, p->pre_buf + pieces_bytes, amax_w, static_cast<const float*>(xs_q16->ptr), pieces_fence));
-            else if (p->x_f32) LAUNCH_TRY(cudaLaunchKernelEx(&pc, lexb::matmul_q_pieces_kernel<1>, static_cast<const void*>(x->ptr), p->k, p->pre_buf, p->pre_buf + pieces_bytes, amax_w, no_xs, pieces_fence));
-            else LAUNCH_TRY(cudaLaunchKernelEx(&pc, lexb::matmul_q_pieces_kernel<0>, static_cast<const void*>(x->ptr), p->k, p->pre_buf, p->pre_buf + pieces_bytes, amax_w, no_xs, pieces_fence));
+            lexb::MqPiecesList list{};
+            list.job[0] = lexb::MqPiecesJob{x->ptr, a.xs, p->pre_buf, p->k};
+            LAUNCH_TRY(cudaLaunchKernelEx(&pc, pieces_kernel(p->x_q16 ? 2 : p->x_f32 ? 1 : 0), list, pieces_fence));
         }
         const CUtensorMap& bmap = p->mq_pre ? p->pre_map : maps.map_wq;      // a placeholder without the pieces kernel
 #define LEXB_MQ_LAUNCH(TR, XF, PR) LAUNCH_TRY(cudaLaunchKernelEx(&cfg, lexb::matmul_q_fp4_kernel<TR, XF, PR>, maps.map_wq, maps.map_ws, nmaps.map_wq, nmaps.map_ws, bmap, a))
@@ -878,13 +890,22 @@ struct ListProof {
 
 bool chain_member(const lexb_gpu* g, const lexb_step& s, const lexb_pipeline* first) {
     const lexb_pipeline* p = s.pipeline;
-    if (!p || !s.buffers || p->gpu != g || p->kernel != KERNEL_MATMUL_Q || p->x_q16 || p->m > chain_max_m() || p->k_splits != 1u) return false;
+    if (!p || !s.buffers || p->gpu != g || p->kernel != KERNEL_MATMUL_Q || p->x_q16 || p->m > chain_max_m() || (p->k_splits != 1u && p->splits_asked)) return false;
     if (p->mq_pre != (p->m > 4u)) return false;                                      // (a plan forced the other way by LEXB_MQ_PRE stays as planned)
     if (p->w_volatile || s.nbuffers != (p->residual ? 6u : 5u)) return false;
+    if (p->k / lexb::MQ_STAGE_K > 0xFFFFu) return false;
     if ((p->k / lexb::MQ_STAGE_K) % lexb::MQ_WS_GROUP == 1u) return false;          // a scale-byte group of one stage is seen by half the scale warps only
     if (p->stages != (p->m <= 4u ? lexb::MQ_MAX_STAGES : 7u) || lexb::matmul_q_chain_smem_bytes(p->stages, p->m) > g->smem_optin) return false;
-    return !first || (p->m == first->m && p->k == first->k && p->x_f32 == first->x_f32 && p->stages == first->stages &&
-                      p->ws_pitch == first->ws_pitch);
+    return !first || (p->m == first->m && p->x_f32 == first->x_f32 && p->stages == first->stages);
+}
+// The digit rows of a run come from the pieces kernel: from 3 tokens on, past 4 in any case, and wherever the steps differ in K
+// or a plan splits it (the in-block derivation walks one K, in one part).
+bool chain_pre(const lexb_step* steps, size_t count) {
+    const lexb_pipeline* p0 = steps[0].pipeline;
+    if (p0->m >= chain_pre_min_m() || p0->m > 4u) return true;
+    for (size_t i = 0; i < count; i++)
+        if (steps[i].pipeline->k != p0->k || steps[i].pipeline->k_splits != 1u) return true;
+    return false;
 }
 
 // Length of the run of steps starting at i that one persistent kernel can take (0: step i is launched on its own).
@@ -909,9 +930,14 @@ size_t chain_run(const lexb_gpu* g, const lexb_step* steps, size_t nsteps, size_
         return false;
     };
     size_t len = 1;
-    while (i + len < nsteps && len < 4096 && chain_member(g, steps[i + len], steps[i].pipeline)) {
+    bool alike = true;                           // (steps of several lengths: their tiles are dealt out one by one, once per list)
+    while (i + len < nsteps && len < (alike ? 4096u : 64u) && chain_member(g, steps[i + len], steps[i].pipeline)) {
         const StepRanges c = step_ranges(steps[i + len]);
         if (!c.valid || conflicts(c, steps[i + len].pipeline->w_const)) break;
+        if (steps[i + len].pipeline->k != steps[i].pipeline->k) {
+            if (len >= 64u) break;
+            alike = false;
+        }
         in_run.push_back(c);
         len++;
     }
@@ -920,28 +946,72 @@ size_t chain_run(const lexb_gpu* g, const lexb_step* steps, size_t nsteps, size_
     // block set-ups (n = 28672: 224 tiles)
     static const bool single = env_u32("LEXB_CHAIN_SINGLE", 1) != 0;
     const uint32_t tiles = (steps[i].pipeline->n + lexb::MQ_ROWS - 1u) / lexb::MQ_ROWS;
-    return single && tiles > static_cast<uint32_t>(g->prop.multiProcessorCount) ? 1 : 0;
+    return single && steps[i].pipeline->k_splits == 1u && tiles > static_cast<uint32_t>(g->prop.multiProcessorCount) ? 1 : 0;
+}
+
+// The table of a run's row tiles: block b works through entries b, b + grid, ...; a row of entries without a job ends it.  Tiles go
+// to the block with the fewest stages so far, the longest tiles first, so that steps of several K end together.
+std::vector<lexb::MqChainTile> chain_tiles(const lexb_step* steps, size_t count, uint32_t sms, uint32_t* grid_out) {
+    std::vector<std::pair<uint32_t, uint32_t>> order;            // (stages of a tile, step), longest first
+    uint32_t total = 0;
+    for (size_t i = 0; i < count; i++) {
+        const lexb_pipeline* p = steps[i].pipeline;
+        order.emplace_back(p->k / lexb::MQ_STAGE_K, static_cast<uint32_t>(i));
+        total += p->n / lexb::MQ_ROWS;
+    }
+    std::stable_sort(order.begin(), order.end(), [](const auto& a, const auto& b) { return a.first > b.first; });
+    const uint32_t grid = std::min(total, sms);
+    const bool alike = order.front().first == order.back().first;
+    std::vector<std::vector<lexb::MqChainTile>> of(grid);
+    using Load = std::pair<uint64_t, uint32_t>;                  // (stages, block)
+    std::priority_queue<Load, std::vector<Load>, std::greater<Load>> least;
+    if (!alike)
+        for (uint32_t b = 0; b < grid; b++) least.emplace(0, b);
+    uint32_t turn = 0;
+    for (const auto& e : order) {
+        const lexb_pipeline* p = steps[e.second].pipeline;
+        for (uint32_t n0 = 0; n0 < p->n; n0 += lexb::MQ_ROWS) {
+            uint32_t b = turn;
+            if (alike) {
+                turn = turn + 1u == grid ? 0u : turn + 1u;
+            } else {
+                const Load l = least.top();
+                least.pop();
+                b = l.second;
+                least.emplace(l.first + e.first, b);
+            }
+            of[b].push_back(lexb::MqChainTile{e.second, n0, e.first | (p->ws_pitch << 16), p->k_splits == 1u ? e.first : p->kb_per_split});
+        }
+    }
+    size_t rows = 0;
+    for (const auto& v : of) rows = std::max(rows, v.size());
+    std::vector<lexb::MqChainTile> out((rows + 1u) * grid, lexb::MqChainTile{lexb::MQC_NO_JOB, 0, 0, 0});
+    for (uint32_t b = 0; b < grid; b++)
+        for (size_t t = 0; t < of[b].size(); t++) out[t * grid + b] = of[b][t];
+    *grid_out = grid;
+    return out;
 }
 
 int launch_chain(lexb_gpu* g, const lexb_step* steps, size_t count, bool fence) {
     bool pdl_next = g->pdl && !fence;            // the run's first kernel launch is the fence, when one is asked for
     const lexb_pipeline* p0 = steps[0].pipeline;
+    const uint32_t m = p0->m;
     std::vector<lexb::MqChainJob> jobs(count);
-    uint32_t tiles = 0, jobs_first_tiles = 0;        // (the latter: every step's tile count if they all agree, else 0)
     int rc;
-    const bool pre = p0->m >= chain_pre_min_m() || p0->m > 4u;       // (the piece warps of a block take up to 4 tokens)
-    std::vector<const void*> pre_done;               // activation buffers whose digit rows this run has asked for
+    const bool pre = chain_pre(steps, count);
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
-    const size_t pieces_bytes = static_cast<size_t>(p0->m) * 8u * (p0->k / 2u);
-    const size_t sfb_bytes = static_cast<size_t>(p0->k / lexb::MQ_STAGE_K) * lexb::MQ_SF_BYTES;
+    struct Act { const void* x; uint32_t k; size_t offset; };    // PRE: the run's distinct activation buffers and their place in the arena
+    std::vector<Act> acts;
+    std::vector<uint32_t> act_of(pre ? count : 0);
+    size_t arena_need = 0;
     for (size_t i = 0; i < count; i++) {
         const lexb_pipeline* p = steps[i].pipeline;
         lexb_buffer* const* b = steps[i].buffers;
         const lexb_buffer *x = b[0], *wq = b[1], *ws = b[2], *wg = b[3], *r = p->residual ? b[4] : nullptr;
         const lexb_buffer* y = p->residual ? b[5] : b[4];
-        const size_t m = p->m, n = p->n, k = p->k;
+        const size_t n = p->n, k = p->k;
         if ((rc = check_buf(x, g, m * k * (p->x_f32 ? 4 : 2), "x"))) return rc;
         if ((rc = check_buf(wq, g, n * k / 2, "wq"))) return rc;
         if ((rc = check_buf(ws, g, n * k / 16, "ws"))) return rc;
@@ -957,86 +1027,124 @@ int launch_chain(lexb_gpu* g, const lexb_step* steps, size_t count, bool fence) 
         jobs[i].r = r ? static_cast<const float*>(r->ptr) : nullptr;
         jobs[i].y = static_cast<float*>(y->ptr);
         jobs[i].n = p->n;
+        jobs[i].k = p->k;
         if (pre) {
-            const auto key = std::make_tuple(static_cast<const void*>(x->ptr), p0->m, p0->k, p0->x_f32 != 0, g->stream);
-            auto it = g->chain_pre.find(key);
-            if (it == g->chain_pre.end()) {
-                if (g->chain_pre.size() >= 256 && pre_done.empty()) {
-                    // activation buffers come and go: start over (buffers of launches in flight are freed after them;
-                    // not in the middle of a run, whose earlier jobs point into these buffers)
-                    CUDA_TRY(cudaDeviceSynchronize());
-                    for (auto& e : g->chain_pre) cudaFree(e.second.buf);
-                    g->chain_pre.clear();
-                }
-                lexb_gpu::ChainPre cp{};
-                const size_t total = pieces_bytes + sfb_bytes + 4u * lexb::MQ_MAX_TOKENS;
-                CUDA_TRY(x_malloc(&cp.buf, total));
-                cudaError_t e = cudaMemsetAsync(cp.buf, 0, total, g->stream);      // scale rows nobody writes stay zero
-                int erc = e == cudaSuccess ? encode_2d(p, &cp.map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, cp.buf, p0->k / 2u, 8u * p0->m, 128u,
-                                                      8u * p0->m, CU_TENSOR_MAP_SWIZZLE_128B, "digit rows of a run")
-                                           : fail(LEXB_ERR_CUDA, "clearing the digit-row buffers: %s", cudaGetErrorString(e));
-                if (erc) { cudaFree(cp.buf); return erc; }
-                it = g->chain_pre.emplace(key, cp).first;
+            size_t e = 0;
+            while (e < acts.size() && (acts[e].x != x->ptr || acts[e].k != p->k)) e++;
+            if (e == acts.size()) {
+                acts.push_back(Act{x->ptr, p->k, arena_need});
+                arena_need += (lexb::matmul_q_pre_bytes(m, p->k) + 255u) / 256u * 256u;
             }
-            uint8_t* buf = it->second.buf;
-            jobs[i].pre = it->second.map;
-            jobs[i].pre_sfb = buf + pieces_bytes;
-            jobs[i].pre_amax = reinterpret_cast<const uint32_t*>(buf + pieces_bytes + sfb_bytes);
-            if (std::find(pre_done.begin(), pre_done.end(), x->ptr) == pre_done.end()) {
-                pre_done.push_back(x->ptr);
-                cudaLaunchConfig_t pc{};
-                pc.gridDim = dim3(p0->m, (p0->k / lexb::MQ_STAGE_K + 31u) / 32u);      // a warp per stage
-                pc.blockDim = dim3(1024);
-                pc.stream = g->stream;
-                pc.attrs = attr;
-                pc.numAttrs = pdl_next ? 1 : 0;
-                pdl_next = g->pdl;
-                uint32_t* amax_w = reinterpret_cast<uint32_t*>(buf + pieces_bytes + sfb_bytes);
-                const float* no_xs = nullptr;
-                if (p0->x_f32) LAUNCH_TRY(cudaLaunchKernelEx(&pc, lexb::matmul_q_pieces_kernel<1>, static_cast<const void*>(x->ptr), p0->k, buf, buf + pieces_bytes, amax_w, no_xs, 0u));
-                else LAUNCH_TRY(cudaLaunchKernelEx(&pc, lexb::matmul_q_pieces_kernel<0>, static_cast<const void*>(x->ptr), p0->k, buf, buf + pieces_bytes, amax_w, no_xs, 0u));
-            }
+            act_of[i] = static_cast<uint32_t>(e);
         }
-        const uint32_t job_tiles = (p->n + lexb::MQ_ROWS - 1u) / lexb::MQ_ROWS;
-        if (i == 0) jobs_first_tiles = job_tiles;
-        else if (job_tiles != jobs_first_tiles) jobs_first_tiles = 0;
-        tiles += job_tiles;
-        jobs[i].tile_end = tiles;
+    }
+    if (pre) {
+        if (g->chain_arenas.size() >= 64 && !g->chain_arenas.count(g->stream)) {
+            // streams come and go: start over (nothing in flight may still read the arenas)
+            CUDA_TRY(cudaDeviceSynchronize());
+            for (auto& e : g->chain_arenas) cudaFree(e.second.buf);
+            for (uint8_t* b : g->retired_arenas) cudaFree(b);
+            g->chain_arenas.clear();
+            g->retired_arenas.clear();
+        }
+        lexb_gpu::ChainArena& arena = g->chain_arenas[g->stream];
+        if (arena.bytes < arena_need) {
+            const size_t bytes = std::max(arena_need, 2u * arena.bytes);
+            uint8_t* buf = nullptr;
+            CUDA_TRY(x_malloc(&buf, bytes));
+            if (arena.buf) g->retired_arenas.push_back(arena.buf);
+            arena.buf = buf;
+            arena.bytes = bytes;
+            arena.maps.clear();
+        }
+        if (arena.maps.size() + acts.size() > 4096u) arena.maps.clear();
+        std::vector<const CUtensorMap*> act_map(acts.size());
+        for (size_t e = 0; e < acts.size(); e++) {
+            const auto key = std::make_tuple(acts[e].offset, m, acts[e].k);
+            auto it = arena.maps.find(key);
+            if (it == arena.maps.end()) {
+                CUtensorMap map;
+                if ((rc = encode_2d(p0, &map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, arena.buf + acts[e].offset, acts[e].k / 2u, 8u * m, 128u, 8u * m,
+                                    CU_TENSOR_MAP_SWIZZLE_128B, "digit rows of a run")))
+                    return rc;
+                it = arena.maps.emplace(key, map).first;
+            }
+            act_map[e] = &it->second;
+        }
+        for (size_t i = 0; i < count; i++) {
+            const Act& act = acts[act_of[i]];
+            jobs[i].pre = *act_map[act_of[i]];
+            jobs[i].pre_sfb = arena.buf + act.offset + lexb::matmul_q_pieces_bytes(m, act.k);
+            jobs[i].pre_amax = reinterpret_cast<const uint32_t*>(jobs[i].pre_sfb + lexb::matmul_q_sfb_total(m, act.k));
+        }
+        for (size_t e0 = 0; e0 < acts.size(); e0 += lexb::MQ_PIECES_LIST) {
+            const size_t e1 = std::min<size_t>(acts.size(), e0 + lexb::MQ_PIECES_LIST);
+            lexb::MqPiecesList list{};
+            uint32_t kb_most = 0;
+            for (size_t e = e0; e < e1; e++) {
+                list.job[e - e0] = lexb::MqPiecesJob{acts[e].x, nullptr, arena.buf + acts[e].offset, acts[e].k};
+                kb_most = std::max(kb_most, acts[e].k / lexb::MQ_STAGE_K);
+            }
+            cudaLaunchConfig_t pc{};
+            pc.gridDim = dim3(m, (kb_most + 31u) / 32u, static_cast<uint32_t>(e1 - e0));      // a warp per stage
+            pc.blockDim = dim3(1024);
+            pc.stream = g->stream;
+            pc.attrs = attr;
+            pc.numAttrs = pdl_next ? 1 : 0;
+            pdl_next = g->pdl;
+            LAUNCH_TRY(cudaLaunchKernelEx(&pc, pieces_kernel(p0->x_f32 ? 1 : 0), list, 0u));
+        }
     }
     const size_t table_bytes = sizeof(lexb::MqChainJob) * count;
     uint64_t h = 1469598103934665603ull;
     {
-        const unsigned char* bytes = reinterpret_cast<const unsigned char*>(jobs.data());
-        for (size_t i = 0; i < table_bytes; i++) h = (h ^ bytes[i]) * 1099511628211ull;
+        const uint64_t* words = reinterpret_cast<const uint64_t*>(jobs.data());      // (a job is whole 64-byte lines)
+        for (size_t i = 0; i < table_bytes / 8u; i++) {
+            h = (h ^ words[i]) * 0x9E3779B97F4A7C15ull;
+            h ^= h >> 32;
+        }
     }
-    lexb::MqChainJob* d_jobs = nullptr;
+    const lexb_gpu::ChainTable* table = nullptr;
     auto hit = g->chain_tables.equal_range(h);
-    for (auto it = hit.first; it != hit.second && !d_jobs; ++it)
-        if (it->second.host.size() == count && !memcmp(it->second.host.data(), jobs.data(), table_bytes)) d_jobs = it->second.dev;
-    if (!d_jobs) {
+    for (auto it = hit.first; it != hit.second && !table; ++it)
+        if (it->second.host.size() == count && !memcmp(it->second.host.data(), jobs.data(), table_bytes)) table = &it->second;
+    if (!table) {
         if (g->chain_tables.size() >= 4096) {
             // (tables of launches still in flight are freed only after them)
             CUDA_TRY(cudaStreamSynchronize(g->stream));
             for (auto& e : g->chain_tables) cudaFree(e.second.dev);
             g->chain_tables.clear();
         }
-        CUDA_TRY(x_malloc(&d_jobs, table_bytes));
-        auto it = g->chain_tables.emplace(h, lexb_gpu::ChainTable{std::move(jobs), d_jobs});
+        uint32_t grid = 0;
+        std::vector<lexb::MqChainTile> tiles = chain_tiles(steps, count, static_cast<uint32_t>(g->prop.multiProcessorCount), &grid);
+        const size_t tile_bytes = sizeof(lexb::MqChainTile) * tiles.size();
+        lexb::MqChainJob* d_jobs = nullptr;
+        CUDA_TRY(x_malloc(&d_jobs, table_bytes + tile_bytes));
+        auto it = g->chain_tables.emplace(h, lexb_gpu::ChainTable{std::move(jobs), std::move(tiles), grid, d_jobs});
+        table = &it->second;
         // (the source is the cache's own copy: it outlives the transfer)
-        CUDA_TRY_AT(SITE_COPY, cudaMemcpyAsync(d_jobs, it->second.host.data(), table_bytes, cudaMemcpyHostToDevice, g->stream));
+        auto copy = [&]() -> int {
+            CUDA_TRY_AT(SITE_COPY, cudaMemcpyAsync(d_jobs, table->host.data(), table_bytes, cudaMemcpyHostToDevice, g->stream));
+            CUDA_TRY_AT(SITE_COPY, cudaMemcpyAsync(d_jobs + count, table->tiles.data(), tile_bytes, cudaMemcpyHostToDevice, g->stream));
+            return LEXB_OK;
+        };
+        if ((rc = copy())) {                     // (a table that was not copied is not kept)
+            cudaStreamSynchronize(g->stream);
+            g->chain_tables.erase(it);
+            cudaFree(d_jobs);
+            return rc;
+        }
     }
     lexb::MqChainArgs a{};
-    a.jobs = d_jobs;
-    a.n_jobs = static_cast<uint32_t>(count);
-    a.n_tiles = tiles;
-    a.tiles_per_job = jobs_first_tiles;
-    a.m = p0->m; a.k = p0->k; a.stages = p0->stages; a.ws_pitch = p0->ws_pitch;
+    a.jobs = table->dev;
+    a.tiles = reinterpret_cast<const lexb::MqChainTile*>(table->dev + count);
+    a.m = m; a.stages = p0->stages;
     a.status = g->d_status;
     // blocks of this kernel do not wait for one another, and there is at most one per SM
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(std::min<uint32_t>(tiles, static_cast<uint32_t>(g->prop.multiProcessorCount)));
+    cfg.gridDim = dim3(table->grid);
     cfg.blockDim = dim3(pre ? lexb::MQC_THREADS_PRE : lexb::MQC_THREADS);
-    cfg.dynamicSmemBytes = lexb::matmul_q_chain_smem_bytes(p0->stages, p0->m);
+    cfg.dynamicSmemBytes = lexb::matmul_q_chain_smem_bytes(p0->stages, m);
     cfg.stream = g->stream;
     cfg.attrs = attr;
     cfg.numAttrs = pdl_next ? 1 : 0;
@@ -1185,8 +1293,8 @@ void lexb_close(lexb_gpu* g) {
     if (g->d_trace) cudaFree(g->d_trace);
     for (auto& e : g->chain_tables) cudaFree(e.second.dev);
     g->chain_tables.clear();
-    for (auto& e : g->chain_pre) cudaFree(e.second.buf);
-    g->chain_pre.clear();
+    for (auto& e : g->chain_arenas) cudaFree(e.second.buf);
+    for (uint8_t* b : g->retired_arenas) cudaFree(b);
     delete g;
 }
 
@@ -1377,6 +1485,7 @@ int lexb_gemm_fp4_plan(lexb_gpu* g, uint32_t m, uint32_t n, uint32_t k, int resi
         const uint32_t per = (kb_all + splits - 1u) / splits;
         splits = (kb_all + per - 1u) / per;
         p->k_splits = splits; p->kb_per_split = per; p->stages = stages;
+        p->splits_asked = s.k_splits != 0u;
         p->ws_pitch = k / 16u < 16u * lexb::MQ_WS_GROUP ? k / 16u : 16u * lexb::MQ_WS_GROUP;
         // In order by default, as the reference's launches are (crates/lex-cuda/src/device.rs:629-672): wq/ws are
         // loaded ahead of the stream's order only when the caller declares them constant or a step list shows
@@ -1402,11 +1511,7 @@ int lexb_gemm_fp4_plan(lexb_gpu* g, uint32_t m, uint32_t n, uint32_t k, int resi
         const bool ahead = m > 4u || (p->x_q16 && m > 1u && walk > (m == 2u ? 150u : 95u));
         p->mq_pre = m > 16u || env_u32("LEXB_MQ_PRE", ahead ? 1u : 0u) != 0;
         if (p->mq_pre) {
-            const size_t pieces_bytes = static_cast<size_t>(m) * 8u * (k / 2u), sfb_bytes = static_cast<size_t>(kb_all) * lexb::matmul_q_sfb_bytes(m);
-            const size_t total = pieces_bytes + sfb_bytes + 4u * lexb::MQ_MAX_TOKENS;
-            cudaError_t e = x_malloc(&p->pre_buf, total);
-            if (e == cudaSuccess) e = cudaMemsetAsync(p->pre_buf, 0, total, g->stream);          // scale rows nobody writes stay zero
-            if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
+            cudaError_t e = x_malloc(&p->pre_buf, lexb::matmul_q_pre_bytes(m, k));
             if (e != cudaSuccess) return bail(fail(LEXB_ERR_CUDA, "allocating the digit-row buffers: %s", cudaGetErrorString(e)));
             int erc = encode_2d(p, &p->pre_map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, p->pre_buf, k / 2u, 8u * m, 128u, 8u * m,
                                 CU_TENSOR_MAP_SWIZZLE_128B, "digit rows");

@@ -1,14 +1,14 @@
-// A run of matmul_q steps of one step list (same t <= 8 and k; see matmul_q_fp4_sm100.cuh) as ONE persistent
+// A run of matmul_q steps of one step list (same t <= 8; see matmul_q_fp4_sm100.cuh) as ONE persistent
 // kernel.  The runtime issues a layer's dispatches as a list (`Gpu::run_launches`,
 // crates/lex-cuda/src/device.rs:650-672); consecutive steps of it often read the same activations against
 // different weights (gate and up of one MLP, the q/k/v projections).
 //
 // A kernel that allocates tensor memory gets an SM to itself, so separate launches cannot overlap on an SM:
 // every launch pays its set-up, the first bytes' trip from DRAM and its tail with the memory system idle.
-// Here the run's row tiles (128 rows of one step, all of K) are numbered through the steps and block b takes
-// tiles b, b + grid, b + 2 grid, ...: every SM has work whatever the steps' tile counts are (136 tiles of
-// n = 17408 leave 12 of 148 SMs idle in a launch of their own, 224 tiles of n = 28672 need two waves), and a
-// block's rings never drain: the copy engine is into the next tile's weights while this tile's last stages
+// Here the run's row tiles (128 rows of one step, all of K) are dealt out to the blocks by a table, the longest first and each
+// to the block with the fewest stages so far: every SM has work whatever the steps' tile counts are (136 tiles of
+// n = 17408 leave 12 of 148 SMs idle in a launch of their own, 224 tiles of n = 28672 need two waves), steps of several K
+// share a launch, and a block's rings never drain: the copy engine is into the next tile's weights while this tile's last stages
 // are multiplied and stored.  Nothing orders the tiles of different blocks, so the host only puts a step into a
 // run if nothing it reads (x, r) is written, and nothing it writes (y) read or written, by a step already in the
 // run (it compares the buffers' address ranges); a step that does depend on the run starts a new launch, and
@@ -25,8 +25,9 @@
 // the same digit rows, which bounds the kernel from 3 tokens on; PRE = true (448 threads) has them derived once
 // per run and activation buffer by matmul_q_pieces_kernel, launched ahead, and the copy engine brings each
 // stage's digit rows and scale blocks with the weights (nothing of a run writes its activations).  Two sets of
-// accumulators (by the parity of the block's tile count) let a tile's MMAs start while the tile before is being
-// stored.
+// accumulators (by the parity of the block's count of parts) let a tile's MMAs start while the tile before is being
+// stored.  A step whose plan splits K over blocks has its parts here one behind the other in one block, each in accumulators
+// of its own, and their results added in the same order: the same bits without partial products in memory.
 #pragma once
 #include "matmul_q_fp4_sm100.cuh"
 
@@ -38,21 +39,30 @@ struct alignas(64) MqChainJob {
     const float* wg;         // [n]
     const float* r;          // [m, n] or null
     float* y;                // [m, n]
-    uint32_t n;              // rows of this step's weights
-    uint32_t tile_end;       // the run's tile count up to and including this step
+    uint32_t n, k;
     // PRE: what matmul_q_pieces_kernel wrote for this step's x
     const uint8_t* pre_sfb;  // [k / 256][2048] scale blocks of the digit rows
     const uint32_t* pre_amax;// [m] largest magnitudes, f32 bits
-    CUtensorMap pre;         // digit rows [8 m][k / 2]
     uint64_t pad[1];
+    CUtensorMap pre;         // digit rows [8 m][k / 2]
 };
 static_assert(sizeof(MqChainJob) % 64 == 0, "tensor maps of a job table sit on 64-byte boundaries");
 
+// One row tile of a run, as the table of tiles holds it: the block's i-th tile is entry i * gridDim.x + blockIdx.x, and the
+// entry behind its last one has job MQC_NO_JOB.
+struct alignas(16) MqChainTile {
+    uint32_t job, n0;        // its step, its first row
+    uint32_t kb_pitch;       // stages of K, and << 16 the bytes per row of a scale load
+    uint32_t per;            // stages per part of K (all of them, unless the step's plan splits K)
+    __device__ __forceinline__ uint32_t kb() const { return kb_pitch & 0xFFFFu; }
+    __device__ __forceinline__ uint32_t ws_pitch() const { return kb_pitch >> 16; }
+};
+constexpr uint32_t MQC_NO_JOB = ~0u;
+
 struct MqChainArgs {
     const MqChainJob* jobs;
-    uint32_t n_jobs, n_tiles;
-    uint32_t tiles_per_job;  // every step has this many row tiles, or 0: they differ and the table is walked
-    uint32_t m, k, stages, ws_pitch;
+    const MqChainTile* tiles;
+    uint32_t m, stages;
     uint32_t* status;
 };
 
@@ -106,20 +116,31 @@ __global__ void __launch_bounds__(PRE ? MQC_THREADS_PRE : MQC_THREADS, 1) matmul
     volatile uint8_t* const nan_rows = reinterpret_cast<volatile uint8_t*>(misc + 16);    // [2 sets][MQ_ROWS]
 
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
-    const uint32_t KB = a.k / MQ_STAGE_K;
-    const uint32_t GP = (KB + MQ_WS_GROUP - 1u) / MQ_WS_GROUP;             // scale-byte groups per step
     const uint32_t N = a.m * MQ_PIECES;
-    // this block's tiles: blockIdx.x + i * gridDim.x, i < T
-    const uint32_t T = blockIdx.x < a.n_tiles ? (a.n_tiles - blockIdx.x + gridDim.x - 1u) / gridDim.x : 0u;
-    // step and first row of the block's i-th tile; `j` is the caller's cursor into the steps (tiles ascend)
-    auto locate = [&](uint32_t i, uint32_t& j) -> uint32_t {
-        const uint32_t tile = blockIdx.x + i * gridDim.x;
-        if (a.tiles_per_job) {       // (a walk is one trip to L2 per step passed: with few tiles per step that is most of a tile's time)
-            j = tile / a.tiles_per_job;
-            return (tile - j * a.tiles_per_job) * MQ_ROWS;
+    // A role's way through this block's tiles: the entry behind the current one is on its way from memory while that one is
+    // worked on.
+    struct Tiles {
+        const MqChainTile* at;
+        uint32_t step;
+        MqChainTile cur, ahead;
+        __device__ __forceinline__ static MqChainTile load(const MqChainTile* p) {
+            const uint4 v = __ldg(reinterpret_cast<const uint4*>(p));
+            return MqChainTile{v.x, v.y, v.z, v.w};
         }
-        while (j + 1u < a.n_jobs && tile >= a.jobs[j].tile_end) j++;
-        return (tile - (j ? a.jobs[j - 1u].tile_end : 0u)) * MQ_ROWS;
+        __device__ __forceinline__ Tiles(const MqChainTile* table) : at(table + blockIdx.x), step(gridDim.x) {
+            cur = load(at);
+            fetch();
+        }
+        __device__ __forceinline__ void fetch() {
+            ahead.job = MQC_NO_JOB;
+            if (cur.job != MQC_NO_JOB) ahead = load(at += step);
+        }
+        __device__ __forceinline__ bool more() const { return cur.job != MQC_NO_JOB; }
+        __device__ __forceinline__ bool last() const { return ahead.job == MQC_NO_JOB; }
+        __device__ __forceinline__ void next() {
+            cur = ahead;
+            fetch();
+        }
     };
 
     if (warp == 0) {
@@ -153,10 +174,9 @@ __global__ void __launch_bounds__(PRE ? MQC_THREADS_PRE : MQC_THREADS, 1) matmul
         // ---------------------------------------------------------------- copy engine: every step's weights, in order
         if (lane == 0) {
             RingPos ps;
-            uint32_t g_issued = 0;                    // scale-byte groups requested so far (flat over the block's tiles)
-            const uint32_t TG = T * GP;
-            uint32_t gj = 0, g_tile = ~0u, g_n0 = 0;  // the scale bytes' own cursor (they run ahead of the codes); the job
-                                                      // table is read once per tile, not per group
+            uint32_t g_issued = 0, g_begun = 0;       // scale-byte groups requested, and those whose codes have been asked for (over the block's tiles)
+            Tiles gt(a.tiles);                        // the scale bytes' own cursor (they run ahead of the codes)
+            uint32_t g = 0;
             // Nothing is waited for until the rings are full.  Before its first real wait this warp joins the
             // stream's order: the warps that free the slots wait for the launch ahead, and a bounded wait must
             // not run against that launch's time.
@@ -168,32 +188,29 @@ __global__ void __launch_bounds__(PRE ? MQC_THREADS_PRE : MQC_THREADS, 1) matmul
                     in_order = true;
                 }
             };
-            auto issue_group = [&](uint32_t G) -> bool {
-                const uint32_t r = G % MQ_WS_SLOTS, wph = (G / MQ_WS_SLOTS) & 1u;
-                if (G >= MQ_WS_SLOTS) join_order();
+            auto issue_group = [&]() -> bool {
+                const uint32_t r = g_issued % MQ_WS_SLOTS, wph = (g_issued / MQ_WS_SLOTS) & 1u;
+                if (g_issued >= MQ_WS_SLOTS) join_order();
                 if (!mbar_wait(ws_empty(r), wph ^ 1u, abort_flag)) return false;
-                const uint32_t i = G / GP, g = G - i * GP;
-                if (i != g_tile) {
-                    g_tile = i;
-                    g_n0 = locate(i, gj);
+                mbar_arrive_expect_tx(ws_full(r), gt.cur.ws_pitch() * MQ_ROWS);
+                tma_load_2d(ws_base + r * MQ_WS_SLOT_BYTES, &a.jobs[gt.cur.job].ws, (int)(g * MQ_WS_GROUP * (MQ_STAGE_K / 16)), (int)gt.cur.n0, ws_full(r));
+                g_issued++;
+                if (++g * MQ_WS_GROUP >= gt.cur.kb()) {
+                    g = 0;
+                    gt.next();
                 }
-                const uint32_t gn0 = g_n0;
-                mbar_arrive_expect_tx(ws_full(r), a.ws_pitch * MQ_ROWS);
-                tma_load_2d(ws_base + r * MQ_WS_SLOT_BYTES, &a.jobs[gj].ws, (int)(g * MQ_WS_GROUP * (MQ_STAGE_K / 16)), (int)gn0, ws_full(r));
                 return true;
             };
             bool ok = true;
-            uint32_t j = 0, filled = 0;
-            uint32_t b_issued = 0, bj = 0;            // PRE: stages whose digit rows have been requested, and their cursor
+            uint32_t filled = 0;
+            uint32_t b_issued = 0;                    // PRE: stages whose digit rows have been requested, and their cursor
             const uint32_t b_bytes = PRE ? N * 128u : 0u;
-            uint32_t b_tile = 0, b_kb = 0;
-            const uint8_t* b_sfb = nullptr;
-            if (PRE) {
-                locate(0, bj);
-                b_sfb = a.jobs[bj].pre_sfb;
-            }
-            for (uint32_t ti = 0; ti < T && ok; ti++) {
-                const uint32_t n0 = locate(ti, j);
+            Tiles bt(a.tiles);
+            uint32_t b_kb = 0;
+            auto sfb_of_job = [&](uint32_t job) -> const uint8_t* { return PRE && job != MQC_NO_JOB ? a.jobs[job].pre_sfb : nullptr; };
+            const uint8_t *b_sfb = sfb_of_job(bt.cur.job), *b_sfb_ahead = sfb_of_job(bt.ahead.job);
+            for (Tiles ct(a.tiles); ct.more() && ok; ct.next()) {
+                const uint32_t KB = ct.cur.kb();
                 for (uint32_t kb = 0; kb < KB; kb++, ps.advance(S), filled++) {
                     const uint32_t s = ps.s;
                     if (filled >= S) join_order();
@@ -203,25 +220,26 @@ __global__ void __launch_bounds__(PRE ? MQC_THREADS_PRE : MQC_THREADS, 1) matmul
                     }
                     if ((kb & (MQ_WS_GROUP - 1u)) == 0u) {
                         // scale bytes one group ahead of the codes (two at the very start)
-                        const uint32_t want = ti * GP + kb / MQ_WS_GROUP + 2u;
-                        while (g_issued < want && g_issued < TG && ok) ok = issue_group(g_issued++);
+                        g_begun++;
+                        while (g_issued < g_begun + 1u && gt.more() && ok) ok = issue_group();
                         if (!ok) break;
                     }
                     mbar_arrive_expect_tx(raw_full(s), MQ_CODE_BYTES + (PRE ? b_bytes + MQ_SF_BYTES : 0u));
-                    tma_load_2d(codes_of(s), &a.jobs[j].wq, (int)(kb * (MQ_STAGE_K / 2)), (int)n0, raw_full(s));
+                    tma_load_2d(codes_of(s), &a.jobs[ct.cur.job].wq, (int)(kb * (MQ_STAGE_K / 2)), (int)ct.cur.n0, raw_full(s));
                     if (PRE) {
                         // The digit rows are written by the launch ahead: the first ring of weights goes out
                         // before that launch is waited for, the digit rows of those stages (slot = stage) after.
-                        if (filled + 1u == S || (ti + 1u == T && kb + 1u == KB)) join_order();
+                        if (filled + 1u == S || (ct.last() && kb + 1u == KB)) join_order();
                         if (in_order) {
                             for (; b_issued <= filled; b_issued++, b_kb++) {
-                                if (b_kb == KB) {            // the next tile of this block (the job table is not read per stage)
+                                if (b_kb == bt.cur.kb()) {   // the next tile of this block
                                     b_kb = 0;
-                                    locate(++b_tile, bj);
-                                    b_sfb = a.jobs[bj].pre_sfb;
+                                    bt.next();
+                                    b_sfb = b_sfb_ahead;
+                                    b_sfb_ahead = sfb_of_job(bt.ahead.job);
                                 }
                                 const uint32_t bs = b_issued % S;
-                                tma_load_2d(b_of(bs), &a.jobs[bj].pre, (int)(b_kb * (MQ_STAGE_K / 2)), 0, raw_full(bs));
+                                tma_load_2d(b_of(bs), &a.jobs[bt.cur.job].pre, (int)(b_kb * (MQ_STAGE_K / 2)), 0, raw_full(bs));
                                 tma_load_1d(sfb_of(bs), b_sfb + (size_t)b_kb * MQ_SF_BYTES, MQ_SF_BYTES, raw_full(bs));
                             }
                         }
@@ -245,17 +263,22 @@ __global__ void __launch_bounds__(PRE ? MQC_THREADS_PRE : MQC_THREADS, 1) matmul
         const uint32_t idesc = umma_idesc_mxf4nvf4(128u, N);
         bool ok = true;
         RingPos ps;
-        for (uint32_t ti = 0; ti < T && ok; ti++) {
-            const uint32_t set = ti & 1u, use = ti >> 1;
-            // the accumulators of this set must have been stored (the block's tile before last)
-            if (use > 0u && !__all_sync(0xFFFFFFFFu, mbar_wait(acc_empty(set), (use - 1u) & 1u, abort_flag))) {
-                atomicOr(a.status, ST_WAIT_ACC);
-                *abort_flag = 1;
-                ok = false;
-                break;
-            }
-            tc_fence_after_sync();
+        uint32_t sub = 0;                                 // parts of K over the block's tiles: the accumulator sets alternate by it
+        for (Tiles ct(a.tiles); ct.more() && ok; ct.next()) {
+            const uint32_t KB = ct.cur.kb(), per = ct.cur.per;
+            uint32_t kl = 0;                              // stage within the part
             for (uint32_t kb = 0; kb < KB; kb++, ps.advance(S)) {
+                const uint32_t set = sub & 1u, use = sub >> 1;
+                if (kl == 0u) {
+                    // the accumulators of this set must have been stored (the part before last)
+                    if (use > 0u && !__all_sync(0xFFFFFFFFu, mbar_wait(acc_empty(set), (use - 1u) & 1u, abort_flag))) {
+                        atomicOr(a.status, ST_WAIT_ACC);
+                        *abort_flag = 1;
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after_sync();
+                }
                 const uint32_t s = ps.s, ph = ps.ph;
                 if (!__all_sync(0xFFFFFFFFu, mbar_wait(raw_full(s), ph, abort_flag)) ||
                     !__all_sync(0xFFFFFFFFu, mbar_wait(prep_full(s), ph, abort_flag))) {
@@ -267,7 +290,8 @@ __global__ void __launch_bounds__(PRE ? MQC_THREADS_PRE : MQC_THREADS, 1) matmul
                 tc_fence_after_sync();
                 const uint32_t a_lo = umma_desc_lo(codes_of(s)), b_lo = umma_desc_lo(b_of(s));
                 const uint32_t sfa_t = tmem_base + TMEM_SFA + 16u * s, sfb_t = tmem_base + TMEM_SFB + 16u * s;
-                const uint32_t d = tmem_base + set * TMEM_SET + ((kb & 1u) ? ACC : 0u);
+                const uint32_t d = tmem_base + set * TMEM_SET + ((kl & 1u) ? ACC : 0u);
+                const bool part_ends = kl + 1u == per || kb + 1u == KB;
                 if (elect_one()) {
 #pragma unroll
                     for (uint32_t q = 0; q < 4; q++) {
@@ -277,11 +301,16 @@ __global__ void __launch_bounds__(PRE ? MQC_THREADS_PRE : MQC_THREADS, 1) matmul
 #pragma unroll
                     for (uint32_t q = 0; q < 4; q++)
                         umma1_mxf4nvf4(d, a_lo + 2u * q, b_lo + 2u * q, idesc, sfa_t + 4u * q, sfb_t + 4u * q,
-                                       (kb >= 2u || q > 0u) ? 1u : 0u);
+                                       (kl >= 2u || q > 0u) ? 1u : 0u);
                     umma_commit(empty(s));
-                    if (kb + 1u == KB) umma_commit(acc_full(set));
+                    if (part_ends) umma_commit(acc_full(set));
                 }
                 __syncwarp();
+                kl++;
+                if (part_ends) {
+                    kl = 0;
+                    sub++;
+                }
             }
         }
         __syncwarp();
@@ -292,11 +321,20 @@ __global__ void __launch_bounds__(PRE ? MQC_THREADS_PRE : MQC_THREADS, 1) matmul
         bool ok = true;
         RingPos ps;
         uint32_t gs = 0;                                  // stage index over the block's tiles
-        for (uint32_t ti = 0; ti < T && ok; ti++) {
-            const uint32_t set = ti & 1u, use = ti >> 1;
-            bool flags_free = use == 0u;                  // this set's NaN flags are cleared by the epilogue of the tile before last
+        uint32_t G0 = 0;                                  // ... and of scale-byte groups
+        uint32_t sub = 0;                                 // ... and of parts of K
+        for (Tiles ct(a.tiles); ct.more() && ok; ct.next(), sub++) {
+            const uint32_t KB = ct.cur.kb(), per = ct.cur.per, ws_pitch = ct.cur.ws_pitch();
+            uint32_t part_end = per;
+            bool flags_free = false;                      // this set's NaN flags are cleared by the epilogue of the part before last
             for (uint32_t kb = 0; kb < KB; kb++, ps.advance(S), gs++) {
+                if (kb == part_end) {
+                    part_end += per;
+                    sub++;
+                    flags_free = false;
+                }
                 if ((gs & 1u) != par) continue;
+                const uint32_t set = sub & 1u, use = sub >> 1;
                 const uint32_t s = ps.s, ph = ps.ph;
                 if (!__all_sync(0xFFFFFFFFu, mbar_wait(empty(s), ph ^ 1u, abort_flag))) {
                     atomicOr(a.status, ST_WAIT_EMPTY_DEQ);
@@ -304,14 +342,14 @@ __global__ void __launch_bounds__(PRE ? MQC_THREADS_PRE : MQC_THREADS, 1) matmul
                     ok = false;
                     break;
                 }
-                const uint32_t G = ti * GP + kb / MQ_WS_GROUP, wr = G % MQ_WS_SLOTS, wph = (G / MQ_WS_SLOTS) & 1u;
+                const uint32_t G = G0 + kb / MQ_WS_GROUP, wr = G % MQ_WS_SLOTS, wph = (G / MQ_WS_SLOTS) & 1u;
                 if (!__all_sync(0xFFFFFFFFu, mbar_wait(ws_full(wr), wph, abort_flag))) {
                     atomicOr(a.status, ST_WAIT_X_FULL);
                     *abort_flag = 1;
                     ok = false;
                     break;
                 }
-                const uint4 sc = *reinterpret_cast<const uint4*>(smem + (ws_base - base) + wr * MQ_WS_SLOT_BYTES + row * a.ws_pitch +
+                const uint4 sc = *reinterpret_cast<const uint4*>(smem + (ws_base - base) + wr * MQ_WS_SLOT_BYTES + row * ws_pitch +
                                                                  16u * (kb & (MQ_WS_GROUP - 1u)));
                 // this warp's last stage of the group: the stages of a group alternate between the two sets
                 // of warps by the parity of the list-wide stage index
@@ -346,6 +384,7 @@ __global__ void __launch_bounds__(PRE ? MQC_THREADS_PRE : MQC_THREADS, 1) matmul
                     if ((z - 0x01010101u) & ~z & 0x80808080u) {
                         for (uint32_t i = 0; i < 4; i++) {
                             if (((v >> (8u * i)) & 0xFFu) == 0x7Fu) {
+                                if (!flags_free && use == 0u) flags_free = true;
                                 if (!flags_free) {
                                     flags_free = mbar_wait(acc_empty(set), (use - 1u) & 1u, abort_flag);
                                     if (!flags_free) {
@@ -364,6 +403,7 @@ __global__ void __launch_bounds__(PRE ? MQC_THREADS_PRE : MQC_THREADS, 1) matmul
                 __syncwarp();
                 if (lane == 0) mbar_arrive(prep_full(s));
             }
+            G0 += (KB + MQ_WS_GROUP - 1u) / MQ_WS_GROUP;
         }
         __syncwarp();
     } else if (warp < MQC_WARP_PIECE) {
@@ -371,72 +411,83 @@ __global__ void __launch_bounds__(PRE ? MQC_THREADS_PRE : MQC_THREADS, 1) matmul
         const uint32_t row = 32u * (warp & 3u) + lane;
         const uint32_t lane_base = tmem_base + ((32u * (warp & 3u)) << 16);
         bool alive = true;
-        uint32_t j = 0;
-        for (uint32_t ti = 0; ti < T && alive; ti++) {
-            const uint32_t set = ti & 1u, use = ti >> 1;
-            const uint32_t n0 = locate(ti, j);
-            uint32_t go = 0;
-            if (alive && lane == 0) go = mbar_wait(acc_full(set), use & 1u, abort_flag);
-            go = __shfl_sync(0xFFFFFFFFu, go, 0);
-            if (alive && !go) {
-                if (lane == 0) {
-                    atomicOr(a.status, ST_WAIT_ACC);
-                    *abort_flag = 1;
-                }
-                alive = false;
-            }
-            if (!alive) break;
-            tc_fence_after_sync();
-            const MqChainJob& job = a.jobs[j];
-            const bool in_n = n0 + row < job.n;
+        uint32_t sub = 0;
+        for (Tiles ct(a.tiles); ct.more() && alive; ct.next()) {
+            const uint32_t KB = ct.cur.kb(), per = ct.cur.per, n0 = ct.cur.n0;
+            const MqChainJob& job = a.jobs[ct.cur.job];
+            // what is read from global memory goes out before the accumulators are waited for
+            const uint32_t n = job.n;
+            const bool in_n = n0 + row < n;
+            const float* const r_p = job.r;
+            float* const y_p = job.y;
             const float g = in_n ? __ldg(job.wg + n0 + row) : 0.0f;
-            const bool row_nan = nan_rows[set * MQ_ROWS + row] != 0;
-            for (uint32_t t = 0; t < a.m; t++) {
-                uint32_t d0[8], d1[8];
-                tmem_ld_32x32b_x8(lane_base + set * TMEM_SET + 8u * t, d0);
-                if (KB > 1u) tmem_ld_32x32b_x8(lane_base + set * TMEM_SET + ACC + 8u * t, d1);
-                tmem_ld_wait();
-                float v = 0.0f;
+            const uint32_t te_lane = PRE && lane < a.m ? __ldg(job.pre_amax + lane) >> 23 : 0u;
+            float res[MQC_MAX_TOKENS], total[MQC_MAX_TOKENS];
 #pragma unroll
-                for (int pc = 7; pc >= 0; pc--) {
-                    float c = __uint_as_float(d0[pc]);
-                    if (KB > 1u) c += __uint_as_float(d1[pc]);
-                    v += c;
-                }
-                const uint32_t te = (PRE ? __ldg(job.pre_amax + t) : tok_amax[set * 4u + t]) >> 23;
-                const float tscale = te >= 16u ? __uint_as_float((te - 8u) << 23) : 0.0f;
-                v = v * tscale * g;
-                if (row_nan || te == 255u) v = __uint_as_float(0x7FC00000u);
-                const size_t o = (size_t)t * job.n + n0 + row;
-                if (in_n) {
-                    if (job.r) v += __ldcg(job.r + o);   // may be an earlier step's output
-                    job.y[o] = v;
-                }
+            for (uint32_t t = 0; t < MQC_MAX_TOKENS; t++) {
+                res[t] = t < a.m && in_n && r_p ? __ldcg(r_p + (size_t)t * n + n0 + row) : 0.0f;
+                total[t] = 0.0f;
             }
-            nan_rows[set * MQ_ROWS + row] = 0;
-            // the accumulators (and this set's flags) are free for the block's tile after next
-            tc_fence_before_sync();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(acc_empty(set));
-
+            // A plan that splits K has its parts summed in their order, as the blocks of a launch of its own sum them.
+            for (uint32_t kb = 0; kb < KB && alive; kb += per, sub++) {
+                const uint32_t set = sub & 1u, use = sub >> 1, len = min(per, KB - kb);
+                uint32_t go = 0;
+                if (lane == 0) go = mbar_wait(acc_full(set), use & 1u, abort_flag);
+                go = __shfl_sync(0xFFFFFFFFu, go, 0);
+                if (!go) {
+                    if (lane == 0) {
+                        atomicOr(a.status, ST_WAIT_ACC);
+                        *abort_flag = 1;
+                    }
+                    alive = false;
+                    break;
+                }
+                tc_fence_after_sync();
+                const bool row_nan = nan_rows[set * MQ_ROWS + row] != 0;
+#pragma unroll
+                for (uint32_t t = 0; t < MQC_MAX_TOKENS; t++) {
+                    if (t >= a.m) break;
+                    uint32_t d0[8], d1[8];
+                    tmem_ld_32x32b_x8(lane_base + set * TMEM_SET + 8u * t, d0);
+                    if (len > 1u) tmem_ld_32x32b_x8(lane_base + set * TMEM_SET + ACC + 8u * t, d1);
+                    tmem_ld_wait();
+                    float v = 0.0f;
+#pragma unroll
+                    for (int pc = 7; pc >= 0; pc--) {
+                        float c = __uint_as_float(d0[pc]);
+                        if (len > 1u) c += __uint_as_float(d1[pc]);
+                        v += c;
+                    }
+                    const uint32_t te = PRE ? __shfl_sync(0xFFFFFFFFu, te_lane, t) : tok_amax[set * 4u + t] >> 23;
+                    const float tscale = te >= 16u ? __uint_as_float((te - 8u) << 23) : 0.0f;
+                    v = v * tscale * g;
+                    if (row_nan || te == 255u) v = __uint_as_float(0x7FC00000u);
+                    total[t] = per < KB ? total[t] + v : v;
+                    if (kb + per >= KB && in_n) y_p[(size_t)t * n + n0 + row] = r_p ? total[t] + res[t] : total[t];
+                }
+                nan_rows[set * MQ_ROWS + row] = 0;
+                // the accumulators (and this set's flags) are free for the part after next
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(acc_empty(set));
+            }
         }
     } else if (!PRE) {
         // ---------------------------------------------------------------- piece warps 14-17
         const uint32_t xw = warp - MQC_WARP_PIECE;
         const uint32_t xt = tid - 32u * MQC_WARP_PIECE;
-        const uint32_t items = KB * a.m;
+        // (the steps of a run without digit rows from ahead have one K and one part of it: a part is a tile)
         const uint32_t PW = (S * a.m < MQC_PIECE_WARPS) ? S * a.m : MQC_PIECE_WARPS;
         for (uint32_t i = xt; i < S * (MQ_SF_BYTES / 16u); i += 32u * MQC_PIECE_WARPS) {
             const uint32_t s = i / (MQ_SF_BYTES / 16u), o = i % (MQ_SF_BYTES / 16u);
             *reinterpret_cast<uint4*>(smem + (sfb_of(s) - base) + 16u * o) = make_uint4(0, 0, 0, 0);
         }
         bool ok = true;          // a warp that gave up keeps walking the steps: barrier 4 below needs all four warps
-        uint32_t j = 0;
         const void* prev_x = nullptr;
-        for (uint32_t ti = 0; ti < T; ti++) {
-            const uint32_t set = ti & 1u;
-            locate(ti, j);
-            const MqChainJob& job = a.jobs[j];
+        uint32_t ti = 0;
+        for (Tiles ct(a.tiles); ct.more(); ct.next(), ti++) {
+            const uint32_t set = ti & 1u, KB = ct.cur.kb(), items = KB * a.m;
+            const MqChainJob& job = a.jobs[ct.cur.job];
             // this block's epilogue of the tile before last is done with this set's slots (token maxima)
             if (ok && (ti >> 1) > 0u && !__all_sync(0xFFFFFFFFu, mbar_wait(acc_empty(set), ((ti >> 1) - 1u) & 1u, abort_flag))) {
                 if (lane == 0) {
@@ -457,7 +508,7 @@ __global__ void __launch_bounds__(PRE ? MQC_THREADS_PRE : MQC_THREADS, 1) matmul
             if (ok && !same_x) {
                 uint32_t mx[4] = {0, 0, 0, 0};
                 const uint4* xr = reinterpret_cast<const uint4*>(job.x);
-                const uint32_t row_chunks = XF32 ? a.k / 4u : a.k / 8u;
+                const uint32_t row_chunks = XF32 ? job.k / 4u : job.k / 8u;
 #pragma unroll 4
                 for (uint32_t i = xt; i < row_chunks; i += 32u * MQC_PIECE_WARPS) {
                     uint4 v[4];
@@ -496,12 +547,12 @@ __global__ void __launch_bounds__(PRE ? MQC_THREADS_PRE : MQC_THREADS, 1) matmul
                 const uint32_t gs = ti * KB + kb, s = gs % S, ph = (gs / S) & 1u;
                 uint4 lo, hi = make_uint4(0, 0, 0, 0);
                 if (XF32) {
-                    const uint4* p4 = reinterpret_cast<const uint4*>(static_cast<const float*>(job.x) + (size_t)tok * a.k) +
+                    const uint4* p4 = reinterpret_cast<const uint4*>(static_cast<const float*>(job.x) + (size_t)tok * job.k) +
                                       (size_t)kb * (MQ_STAGE_K / 4u) + 2u * lane;
                     lo = __ldcg(p4);
                     hi = __ldcg(p4 + 1);
                 } else {
-                    lo = __ldcg(reinterpret_cast<const uint4*>(static_cast<const __half*>(job.x) + (size_t)tok * a.k) +
+                    lo = __ldcg(reinterpret_cast<const uint4*>(static_cast<const __half*>(job.x) + (size_t)tok * job.k) +
                                 (size_t)kb * (MQ_STAGE_K / 8u) + lane);
                 }
                 const uint32_t te8 = tok_amax[set * 4u + tok] >> 23;

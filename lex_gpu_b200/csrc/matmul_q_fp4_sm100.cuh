@@ -754,18 +754,38 @@ matmul_q_fp4_kernel(const __grid_constant__ CUtensorMap tmap_wq, const __grid_co
 // each finds the token's largest magnitude itself and takes every gridDim.y-th set of 32 stages.
 //   pieces [8 m][k / 2] bytes: row 8 t + p holds piece p of token t, packed like wq (a tensor map with the
 //                              128-byte swizzle brings 8 m x 128 bytes of it per stage);
-//   sfb    [k / 256][2048 or 4096] bytes: per stage the scale blocks of B (rows past 8 m stay zero);
+//   sfb    [k / 256][2048 or 4096] bytes: per stage the scale blocks of B (zeros in the rows past 8 m);
 //   amax   [m]: the token's largest magnitude as f32 bits.
 // It follows the previous launch of the same pipeline in the stream, which may still be reading these
 // buffers: nothing is written before grid_dependency_wait().  With `fence` the launch behind it starts only once everything
 // ahead of this one is done, and may then load what this one does not write (the weights) at once.
 // XMODE: 0 = f16 activations, 1 = f32, 2 = int16 activations with one f32 scale per 16 values (`xs`), as
 // lex_msl::int8::quant16 leaves them (crates/lex-msl/src/int8.rs:47-114): the value is q * xs in f32.
+// A run of steps has all its activation buffers done by one launch: blocks (t, *, i) take buffer i of the list.
+struct MqPiecesJob {
+    const void* x;
+    const float* xs;
+    uint8_t* out;            // pieces, then sfb, then amax
+    uint32_t k;
+};
+__host__ __device__ constexpr size_t matmul_q_pieces_bytes(uint32_t m, uint32_t k) { return (size_t)m * MQ_PIECES * (k / 2u); }
+__host__ __device__ constexpr size_t matmul_q_sfb_total(uint32_t m, uint32_t k) { return (size_t)(k / MQ_STAGE_K) * matmul_q_sfb_bytes(m); }
+__host__ __device__ constexpr size_t matmul_q_pre_bytes(uint32_t m, uint32_t k) { return matmul_q_pieces_bytes(m, k) + matmul_q_sfb_total(m, k) + 4u * MQ_MAX_TOKENS; }
+constexpr uint32_t MQ_PIECES_LIST = 32;
+struct MqPiecesList {
+    MqPiecesJob job[MQ_PIECES_LIST];
+};
 template <int XMODE>
 __global__ void __launch_bounds__(1024, 1)
-matmul_q_pieces_kernel(const void* __restrict__ x, uint32_t k, uint8_t* __restrict__ pieces, uint8_t* __restrict__ sfb,
-                       uint32_t* __restrict__ amax, const float* __restrict__ xs, uint32_t fence) {
+matmul_q_pieces_kernel(const __grid_constant__ MqPiecesList list, uint32_t fence) {
     constexpr bool XF32 = XMODE == 1, Q16 = XMODE == 2;
+    const MqPiecesJob& job = list.job[blockIdx.z];
+    const void* const x = job.x;
+    const float* const xs = job.xs;
+    const uint32_t k = job.k;
+    uint8_t* const pieces = job.out;
+    uint8_t* const sfb = pieces + matmul_q_pieces_bytes(gridDim.x, k);
+    uint32_t* const amax = reinterpret_cast<uint32_t*>(sfb + matmul_q_sfb_total(gridDim.x, k));
     const bool wide = gridDim.x > 16u;                        // tokens = gridDim.x
     const uint32_t sfb_stage = matmul_q_sfb_bytes(gridDim.x);
     __shared__ uint32_t s_amax;
@@ -774,6 +794,7 @@ matmul_q_pieces_kernel(const void* __restrict__ x, uint32_t k, uint8_t* __restri
     if (!fence) allow_dependents();
     grid_dependency_wait();
     if (fence) allow_dependents();
+    if (blockIdx.y * 32u >= k / MQ_STAGE_K) return;           // (another buffer of the list has a longer K)
     __syncthreads();
     const uint4* xr = XF32 ? reinterpret_cast<const uint4*>(static_cast<const float*>(x) + (size_t)tok * k)
                            : reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(x) + (size_t)tok * k);
@@ -831,6 +852,13 @@ matmul_q_pieces_kernel(const void* __restrict__ x, uint32_t k, uint8_t* __restri
         for (uint32_t i = 0; i < 4; i++) {
             const uint32_t pc = 4u * (lane & 1u) + i;
             sfb[(size_t)kb * sfb_stage + mq_sfb_offset(tok * MQ_PIECES + pc, grp, wide)] = sv[i];
+        }
+        if (tok == 0) {                                       // the rows no token has hold zeros
+            uint32_t* const words = reinterpret_cast<uint32_t*>(sfb + (size_t)kb * sfb_stage);
+            for (uint32_t i = lane; i < sfb_stage / 4u; i += 32u) {
+                const uint32_t n = ((i >> 2) & 31u) + (i & 3u) * 32u + (wide ? ((i >> 7) & 1u) * 128u : 0u);
+                if (n >= gridDim.x * MQ_PIECES) words[i] = 0u;
+            }
         }
     }
 }

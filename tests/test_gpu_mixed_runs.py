@@ -1,0 +1,114 @@
+"""Runs of matmul_q steps of several K, and of plans that split K, as one persistent launch."""
+import numpy as np
+import pytest
+
+import lex_gpu_b200 as L
+from lex_gpu_b200 import inputs
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def gpu():
+    g = L.Gpu(0)
+    yield g
+    g.close()
+
+
+@pytest.mark.parametrize("m,xf32", [(1, False), (2, True), (4, False), (5, True), (8, False)])
+def test_steps_of_several_k_share_a_launch(gpu, m, xf32):
+    """K of 2 to 68 stages (groups of scale bytes that end inside), plans with 1, 2 and 8 parts of K, more tiles than SMs, a
+    residual, one activation buffer read with two K: each step's bits are those of its own launch."""
+    shapes = [(4096, 1024), (640, 17408), (1024, 512), (640, 8192), (2048, 2048), (8192, 1024), (128, 1536)]
+    ks = sorted({k for _, k in shapes})
+    xs = {k: inputs.make_x(m, k, seed_base=600 + k) for k in ks}
+    if xf32:
+        xs = {k: v.astype(np.float32) * np.float32(1.0009765625) for k, v in xs.items()}
+    xb = {k: gpu.upload(v) for k, v in xs.items()}
+    sets = [inputs.make_weights(n, k, seed_base=601, copy=i) for i, (n, k) in enumerate(shapes)]
+    r = np.random.Generator(np.random.PCG64(602)).standard_normal((m, 640)).astype(np.float32)
+    rb = gpu.upload(r)
+    xb[512] = xb[1024]                                            # the same buffer, its first half read as [m, 512]
+    xs[512] = xs[1024].reshape(-1)[:m * 512].reshape(m, 512)
+    pipes = [gpu.plan_matmul_fp4(m, n, k, residual=(i == 1), x_half=not xf32) for i, (n, k) in enumerate(shapes)]
+    assert {p.describe().k_splits for p in pipes} >= {1, 2, 8}
+    ys = [gpu.alloc(4 * m * n) for n, _ in shapes]
+    binds = [L.QBuf(gpu, *w).bind(xb[k], rb if i == 1 else None, ys[i]) for i, (w, (n, k)) in enumerate(zip(sets, shapes))]
+    alone = []
+    for i, (n, k) in enumerate(shapes):
+        gpu.run(pipes[i], binds[i])
+        gpu.sync()
+        alone.append(gpu.download(ys[i], np.float32, (m, n)))
+        err, scale, _ = O.err_of_scale(alone[i], O.matmul_q_x(xs[k], *sets[i], r=r if i == 1 else None))
+        assert scale > 1e-3 and err <= 1e-4
+    steps = L.StepList(list(zip(pipes, binds)))
+    assert gpu.list_runs(steps) == [len(shapes)] * len(shapes)
+    for _ in range(2):
+        for y in ys:
+            gpu.memset(y, 0xEE)
+        gpu.run_launches(steps)
+        for i, (n, _) in enumerate(shapes):
+            assert np.array_equal(gpu.download(ys[i], np.float32, (m, n)), alone[i]), shapes[i]
+    assert gpu.status_word() == 0
+
+
+def test_bad_scale_bytes_in_one_part_of_k(gpu):
+    """NaN scale bytes and negative ones in different parts of a split K: that row is NaN, no other is."""
+    m, n, k = 3, 640, 8192
+    x = inputs.make_x(m, k, seed_base=610)
+    wq, ws, wg = inputs.make_weights(n, k, seed_base=611)
+    ws = ws.copy()
+    for row, col, byte in ((3, 5, 0x7F), (200, k // 16 - 1, 0xFF), (639, 300, 0x7F)):
+        ws[row, col] = byte
+    ws[7, ::3] |= 0x80
+    other = inputs.make_weights(4096, 1024, seed_base=612)
+    pipe, first = gpu.plan_matmul_fp4(m, n, k), gpu.plan_matmul_fp4(m, 4096, 1024)
+    assert pipe.describe().k_splits > 1
+    y, ya = gpu.alloc(4 * m * n), gpu.alloc(4 * m * 4096)
+    xb, x1 = gpu.upload(x), gpu.upload(inputs.make_x(m, 1024, seed_base=613))
+    q = L.QBuf(gpu, wq, ws, wg)
+    gpu.run(pipe, q.bind(xb, None, y))
+    gpu.sync()
+    alone = gpu.download(y, np.float32, (m, n))
+    gpu.memset(y, 0)
+    steps = [(first, L.QBuf(gpu, *other).bind(x1, None, ya)), (pipe, q.bind(xb, None, y))]
+    assert gpu.list_runs(steps) == [2, 2]
+    gpu.run_launches(steps)
+    got = gpu.download(y, np.float32, (m, n))
+    assert np.array_equal(got, alone, equal_nan=True)
+    bad = np.isnan(got).any(axis=0)
+    assert set(np.flatnonzero(bad)) == {3, 200, 639} and np.isnan(got[:, bad]).all()
+    assert gpu.status_word() == 0
+
+
+def test_lists_of_growing_activations_on_two_streams(gpu):
+    """The digit rows of a run live in an arena per stream that grows with the lists: results stay right when a later list needs
+    more of it, an earlier one comes again, and another stream has its own."""
+    import torch
+    m = 4
+    lists = []
+    for ks in ((1024, 2048), (1024, 2048, 8192, 512), (4096, 1024, 17408, 2048, 512)):
+        steps, want = [], []
+        for i, k in enumerate(ks):
+            x, (wq, ws, wg) = inputs.make_x(m, k, seed_base=620 + i), inputs.make_weights(256, k, seed_base=621, copy=i)
+            y = gpu.alloc(4 * m * 256)
+            steps.append((gpu.plan_matmul_fp4(m, 256, k), L.QBuf(gpu, wq, ws, wg).bind(gpu.upload(x), None, y)))
+            want.append((y, O.matmul_q_x(x, wq, ws, wg)))
+        lists.append((steps, L.StepList(steps), want))
+    other = torch.cuda.Stream()
+    try:
+        for stream in (None, other.cuda_stream, None):
+            gpu.set_stream(stream)
+            for which in (0, 1, 0, 2, 1):
+                _, steps, want = lists[which]
+                for y, _ in want:
+                    gpu.memset(y, 0xEE)
+                gpu.sync()
+                gpu.run_launches(steps)
+                for y, w in want:
+                    err, scale, _ = O.err_of_scale(gpu.download(y, np.float32, w.shape), w)
+                    assert scale > 1e-3 and err <= 1e-4
+    finally:
+        gpu.set_stream(None)
+    assert gpu.status_word() == 0
