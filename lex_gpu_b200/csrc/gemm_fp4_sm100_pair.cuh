@@ -59,20 +59,24 @@ constexpr uint32_t PAIR_RAW_K = 256;                  // K columns per block of 
 constexpr uint32_t PAIR_RAW_WQ_BYTES = GEMM_TN * (PAIR_RAW_K / 2);          // 16 KiB
 constexpr uint32_t PAIR_RAW_WS_BYTES = GEMM_TN * (PAIR_RAW_K / 16);         // 2 KiB
 constexpr uint32_t PAIR_RAW_BYTES = PAIR_RAW_WQ_BYTES + PAIR_RAW_WS_BYTES;
+constexpr uint32_t PAIR_CLUSTER_SPLITS = 4;            // parts of K that a cluster (of at most 8 blocks) can hold
 constexpr uint32_t PAIR_RAW_STAGES = 2;                // default depth of the ring of packed-weight blocks
 
 // x ring, W ring (their depths are independent: the decoded W tiles may run further ahead of the
 // MMA than the x tiles), packed-weight blocks, barriers, TMEM slot + abort flag, alignment slack
 // (`w_in_tmem`: the decoded W tiles live in tensor memory and take no shared memory)
+__host__ __device__ constexpr uint32_t pair_ring_bytes(uint32_t tok_blocks, uint32_t sx, uint32_t sw, uint32_t sr, bool w_in_tmem, uint32_t k_sub, uint32_t x_rows) {
+    const uint32_t rings = sx * pair_x_stage_bytes(tok_blocks, k_sub, x_rows) + (w_in_tmem ? 0u : sw * GEMM_W_TILE_BYTES) + sr * PAIR_RAW_BYTES;
+    return rings > PAIR_STAGING_BYTES ? rings : PAIR_STAGING_BYTES;
+}
 __host__ __device__ constexpr uint32_t pair_smem_bytes(uint32_t tok_blocks, uint32_t sx, uint32_t sw, uint32_t sr = PAIR_RAW_STAGES,
                                                       bool w_in_tmem = false, uint32_t k_sub = 1, uint32_t x_rows = PAIR_XBLK_ROWS) {
-    const uint32_t rings = sx * pair_x_stage_bytes(tok_blocks, k_sub, x_rows) + (w_in_tmem ? 0u : sw * GEMM_W_TILE_BYTES) + sr * PAIR_RAW_BYTES;
-    return (rings > PAIR_STAGING_BYTES ? rings : PAIR_STAGING_BYTES) +
+    return pair_ring_bytes(tok_blocks, sx, sw, sr, w_in_tmem, k_sub, x_rows) +
            (2u * sx + 3u * sw + 1u + 2u * sr) * 8u + 16u + 1024u;
 }
 
 template <bool TRACE>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
+__global__ void __launch_bounds__(PAIR_THREADS, 1)
 gemm_fp4_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_wq,
                              const __grid_constant__ CUtensorMap tmap_ws, const GemmArgs a) {
     extern __shared__ uint8_t smem_raw[];
@@ -115,7 +119,8 @@ gemm_fp4_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const _
     volatile uint32_t* const abort_flag = tmem_slot + 1;
 
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
-    const uint32_t rank = cluster_ctarank();                 // 0 = leader
+    // A cluster is one pair, or - K split within it - the pairs of all parts of K of one tile.  Rank in the pair: 0 = leader.
+    const uint32_t cluster_rank = cluster_ctarank(), rank = cluster_rank & 1u, leader = cluster_rank & ~1u;
     const uint32_t pair = blockIdx.x >> 1;
     const uint32_t split = pair % a.k_splits, tile = pair / a.k_splits;
     const uint32_t m_tile = tile % a.m_tiles, n_pair = tile / a.m_tiles;
@@ -167,6 +172,8 @@ gemm_fp4_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const _
     // each joins the stream's order before its first wait on a ring slot (a bounded wait must not run
     // against another launch's time) and, for the decode warps, before the epilogue.
     const bool early_w = (a.flags & 2u) != 0u;
+    const bool in_cluster = (a.flags & 8u) != 0u;            // the parts of K are summed within the cluster (below)
+    bool acc_ok = false;                                     // (decode warps) the accumulator is complete
 
     const bool weight_role = warp == PAIR_WARP_RAW || warp < PAIR_DEQ_THREADS / 32u;
     if (!(early_w && weight_role)) grid_dependency_wait();
@@ -185,7 +192,7 @@ gemm_fp4_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const _
                     }
                     pe.advance(DN);
                 }
-                const uint32_t lead_bar = map_to_cta(full(pf.s), 0);
+                const uint32_t lead_bar = map_to_cta(full(pf.s), leader);
                 mbar_arrive_expect_tx_cluster(lead_bar, KS * TB * a.x_tx_bytes);
                 const uint32_t dst = base + s * XSB;
                 const uint32_t kb = kb0 + st * KS;
@@ -242,7 +249,7 @@ gemm_fp4_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const _
                     *abort_flag = 1;
                     break;
                 }
-                mbar_arrive_cluster(map_to_cta(full(pf.s), 0));
+                mbar_arrive_cluster(map_to_cta(full(pf.s), leader));
             }
         }
         // ---------------------------------------------------------------- MMA issuer (leader only)
@@ -252,6 +259,7 @@ gemm_fp4_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const _
             const uint32_t x_lo0 = umma_desc_lo(base), w_lo0 = umma_desc_lo(w_base);
             const uint32_t d0 = tmem_base, d1 = tmem_base + 256u;
             const bool reuse_a = (a.flags & 1u) != 0u;
+            const uint16_t both = static_cast<uint16_t>(3u << leader);
             bool ok = true;
             long long wait_full = 0, t_first = 0, t_issue = 0;
             RingPos px, pw, pf;
@@ -316,12 +324,12 @@ gemm_fp4_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const _
 #pragma unroll
                     for (uint32_t kk = 1; kk < GEMM_BK / 16; kk++) umma2_acc(d, aw + 2u * kk, b0 + 2u * kk, idesc);
                 }
-                umma_commit_pair(done(pf.s), 3);             // frees this K step's x stage and W stage in both CTAs
+                umma_commit_pair(done(pf.s), both);             // frees this K step's x stage and W stage in both CTAs
                 }
                 __syncwarp();
                 if (TRACE) t_issue += clock64() - ti0;
             }
-            if (ok && elect_one()) umma_commit_pair(acc_full, 3);
+            if (ok && elect_one()) umma_commit_pair(acc_full, both);
             __syncwarp();
             if (TRACE && a.trace && lane == 0) {
                 unsigned long long* tr = a.trace + 16ull * blockIdx.x;
@@ -444,13 +452,14 @@ gemm_fp4_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const _
             }
         }
         go = __shfl_sync(0xFFFFFFFFu, go, 0);
+        acc_ok = go != 0u;
         if (TRACE && a.trace && tid == 0) {
             a.trace[16ull * blockIdx.x + 0] = (unsigned long long)t_start;
             // block start on the global timer (ns): in the partner's record (the leader's slot 11 holds its MMA issue cycles)
             if (rank != 0u) a.trace[16ull * blockIdx.x + 11] = gt_start;
             a.trace[16ull * blockIdx.x + 6] = (unsigned long long)clock64();   // accumulator complete
         }
-        if (go && n0 < a.n) {
+        if (go && n0 < a.n && !in_cluster) {
             tc_fence_after_sync();
             const uint32_t quarter = warp & 3u, slice = warp >> 2;      // 4 lane quarters x 4 column slices
             const bool to_partial = a.k_splits > 1u;
@@ -537,6 +546,62 @@ gemm_fp4_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const _
                             }
                         }
                     }
+                }
+            }
+        }
+    }
+
+    if (in_cluster) {
+        // K split within the cluster (tiles of up to 256 tokens): every block leaves its sums in shared memory (the rings are idle:
+        // its accumulator is complete) as [token][128 rows]; then the blocks that hold the same rows share out the tokens, and add
+        // the parts, from one another's shared memory, in the order of the parts - the sums of splitk_reduce_kernel, bit for
+        // bit, without the partials' way through L2 and without a second launch (1024 x 2048 x 4096 in 2 parts: 21.1 -> 18.9 us;
+        // 201 x 6144 x 4096 in 2 parts: 19.9 -> 18.0).
+        const uint32_t tokens = min(a.m - m0, 2u * XR);
+        if (warp < PAIR_DEQ_THREADS / 32u && acc_ok) {
+            tc_fence_after_sync();
+            const uint32_t quarter = warp & 3u, slice = warp >> 2;
+            const bool two_acc = KB > 1u && !w_tmem;
+            float* const mine = reinterpret_cast<float*>(smem) + 32u * quarter + lane;
+            for (uint32_t c = 16u * slice; c < tokens; c += 64u) {
+                uint32_t v[16];
+                tmem_ld_32x32b_x16(tmem_base + ((32u * quarter) << 16) + c, v);
+                if (two_acc) {
+                    uint32_t v2[16];
+                    tmem_ld_32x32b_x16(tmem_base + ((32u * quarter) << 16) + 256u + c, v2);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (uint32_t j = 0; j < 16; j++) v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(v2[j]));
+                } else {
+                    tmem_ld_wait();
+                }
+#pragma unroll
+                for (uint32_t j = 0; j < 16; j++)
+                    if (c + j < tokens) mine[(c + j) * 128u] = __uint_as_float(v[j]);
+            }
+        }
+        cluster_sync_all();
+        if (warp < PAIR_DEQ_THREADS / 32u && acc_ok && n0 < a.n) {
+            const uint32_t S = a.k_splits;
+            // a warp takes a token's 128 rows, four rows a lane
+            for (uint32_t t = split + S * warp; t < tokens; t += S * (PAIR_DEQ_THREADS / 32u)) {
+                const uint32_t at = base + t * 512u + lane * 16u, tok = m0 + t;
+                float4 v[PAIR_CLUSTER_SPLITS];
+#pragma unroll
+                for (uint32_t p = 0; p < PAIR_CLUSTER_SPLITS; p++)
+                    if (p < S) v[p] = ld_shared_cluster_f32x4(map_to_cta(at, 2u * p + rank));
+                float4 s = v[0];
+                auto add = [&](const float4& o) { s.x += o.x; s.y += o.y; s.z += o.z; s.w += o.w; };
+#pragma unroll
+                for (uint32_t p = 1; p < PAIR_CLUSTER_SPLITS; p++)
+                    if (p < S) add(v[p]);
+                const uint32_t col = n0 + lane * 4u;
+                if (a.r) add(__ldg(reinterpret_cast<const float4*>(a.r + (size_t)tok * a.n + col)));
+                if (a.act != nullptr) {
+                    reinterpret_cast<uint32_t*>(a.act)[((size_t)tok * (a.n >> 1) + (col >> 1)) >> 1] =
+                        (uint32_t)f32_to_f16_bits(silu_mul_f32(s.x, s.y)) | ((uint32_t)f32_to_f16_bits(silu_mul_f32(s.z, s.w)) << 16);
+                } else {
+                    *reinterpret_cast<float4*>(a.y + (size_t)tok * a.n + col) = s;
                 }
             }
         }

@@ -178,6 +178,8 @@ struct lexb_pipeline {
     uint32_t k_sub = 1;         // two-CTA kernel: K steps per ring stage
     uint32_t x_rows = lexb::PAIR_XBLK_ROWS;     // two-CTA kernel: tokens per CTA and token block (tm / 2 for tiles below 512 tokens)
     uint32_t k_splits = 1, kb_per_split = 0, tok_blocks = 2;
+    double us = 1e30;           // ... what the planner expects a launch to take
+    bool cluster_split = false; // ... the parts of K summed within a cluster, but for a gather
     uint32_t ws_pitch = 0;      // block-scaled kernel: bytes per row of one scale load
     bool x_f32 = false;         // ... with f32 activations
     bool x_q16 = false;         // ... with int16 activations and one f32 scale per 16 (lexb_matmul_int8_plan): bindings [xq, xs, wq, ...]
@@ -568,21 +570,46 @@ uint32_t held_clusters(lexb_gpu* g, uint32_t c) {
     return held == ~0u ? 0u : held;
 }
 
+// What a launch of the two-CTA GEMM takes, us: `start`; per wave of tiles `wave` for a block's start and its store and `kstep` per K
+// step, for tiles of 512 / 256 / 128 / 64 tokens; `store` per MB of y; with K in parts, per MB of partial products and once,
+// `reduce` by the second launch, `cluster` in clusters.  At least `least` blocks of 256 columns in a part.
+struct PairPrices {
+    double start, kstep[4], wave[4], store, reduce, reduce_mb, cluster, cluster_mb;
+    uint32_t least;
+};
+// Fitted to 4,466 launches of 487 shapes (m = 9-2048, n = 128-28672, k = 256-17408) on a B200: rms error 5 %, the form chosen takes
+// 0.8 % more than the fastest in the mean, where the prices before (159 launches with the table decode) took 9 % more.  Past 60
+// GFLOP a launch runs into the power cap, which bursts of launches do not show: those prices stay there.
+const PairPrices& pair_prices(uint32_t m, uint32_t n, uint32_t k) {
+    static const PairPrices FITTED = {0.20, {0.598, 0.337, 0.319, 0.319}, {7.69, 5.85, 4.46, 3.70}, 0.157, 1.04, 0.288, 0.25, 0.271, 2u},
+                            LARGE = {4.51, {0.559, 0.311, 0.310, 0.304}, {8.05, 5.32, 4.02, 4.14}, 0.0, -1.12, 0.300, -1.12, 0.300, 4u};
+    return 2.0 * m * n * k < 6e10 ? FITTED : LARGE;
+}
+
 // The few-token kernel's launch for a pipeline, if it takes the shape.
 int plan_few(lexb_gpu* g, lexb_pipeline* p) {
     const uint32_t m = p->m, n = p->n, k = p->k;
+    if (p->kernel != KERNEL_TCGEN05_PAIR && !env_u32("LEXB_FEW_C", 0)) return LEXB_OK;      // (the matvec keeps m <= 8)
     if (m > lexb::FEW_MAX_TOKENS || n % lexb::FEW_ROWS || k % lexb::FEW_K) return LEXB_OK;
     const uint32_t tiles = n / lexb::FEW_ROWS, U = k / lexb::FEW_K;
+    // Fitted to 839 shapes (m = 9-64, clusters of 1, 2, 3, 4, 6 and 8; rms error 6 %, the cluster chosen takes 0.4 % more than the fastest
+    // in the mean), us: 2.45, 1.21 per block of weights of the longest share and a little less with wider MMAs, the cluster's
+    // barriers and sums, the segments' stores, y.
     const uint32_t forced = env_u32("LEXB_FEW_C", 0);
     uint32_t best_c = 0, best_clusters = 0;
-    double best = 1e30;
+    double best = forced ? 1e30 : p->us;
     for (uint32_t c = 1; c <= lexb::FEW_MAX_CLUSTER; c++) {
-        if (forced && c != forced) continue;
+        if (forced ? c != forced : c == 5u || c == 7u) continue;
         const uint32_t clusters = std::min(held_clusters(g, c), tiles);
         if (!clusters || (tiles / clusters) * U < c) continue;
-        const uint32_t blocks = ((tiles + clusters - 1u) / clusters * U + c - 1u) / c;
-        const double us = blocks * 0.4 + (c > 1u ? 1.0 : 0.0);
-        if (us < best) { best = us; best_c = c; best_clusters = clusters; }
+        const uint32_t blocks = ((tiles + clusters - 1u) / clusters * U + c - 1u) / c, segments = (blocks + U - 1u) / U;
+        const double us = 2.45 + blocks * (m <= 16u ? 1.21 : m <= 32u ? 1.195 : 1.154) + (c > 1u ? 1.88 + 0.005 * m : 0.0) + 0.0186 * segments * m +
+                          0.32e-5 * m * n;
+        if (us < best) {
+            best = us;
+            best_c = c;
+            best_clusters = clusters;
+        }
     }
     if (!best_c) return LEXB_OK;
     lexb_pipeline* f = new (std::nothrow) lexb_pipeline();
@@ -673,16 +700,22 @@ int launch_one(lexb_gpu* g, const lexb_pipeline* p, const lexb_buffer* x, const 
             cfg.blockDim = dim3(p->threads);
             cfg.dynamicSmemBytes = p->smem;
             cfg.stream = g->stream;
-            cudaLaunchAttribute attr[1];
-            attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-            attr[0].val.programmaticStreamSerializationAllowed = 1;
+            const bool in_cluster = p->cluster_split && !gather;
+            if (in_cluster) a.flags |= 8u;
+            cudaLaunchAttribute attr[2];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = in_cluster ? 2u * p->k_splits : 2u;
+            attr[0].val.clusterDim.y = 1;
+            attr[0].val.clusterDim.z = 1;
+            attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            attr[1].val.programmaticStreamSerializationAllowed = 1;
             cfg.attrs = attr;
-            cfg.numAttrs = pdl ? 1 : 0;
+            cfg.numAttrs = pdl ? 2 : 1;
             if (a.trace)
                 LAUNCH_TRY(cudaLaunchKernelEx(&cfg, lexb::gemm_fp4_tcgen05_pair_kernel<true>, maps.map, maps.map_wq, maps.map_ws, a));
             else
                 LAUNCH_TRY(cudaLaunchKernelEx(&cfg, lexb::gemm_fp4_tcgen05_pair_kernel<false>, maps.map, maps.map_wq, maps.map_ws, a));
-            if (p->k_splits > 1) {
+            if (p->k_splits > 1 && !in_cluster) {
                 CUDA_TRY(cudaGetLastError());
                 const size_t elems = static_cast<size_t>(p->m) * p->n;       // n % 128 == 0: a multiple of 4
                 const uint32_t blocks = static_cast<uint32_t>(std::min<size_t>((elems / 4 + 255) / 256, static_cast<size_t>(g->prop.multiProcessorCount) * 8u));
@@ -690,7 +723,7 @@ int launch_one(lexb_gpu* g, const lexb_pipeline* p, const lexb_buffer* x, const 
                 rc_cfg.gridDim = dim3(blocks);
                 rc_cfg.blockDim = dim3(256);
                 rc_cfg.stream = g->stream;
-                rc_cfg.attrs = attr;
+                rc_cfg.attrs = attr + 1;
                 rc_cfg.numAttrs = g->pdl ? 1 : 0;
                 const auto reduce = p->k_splits == 2u ? lexb::splitk_reduce_kernel<2> : p->k_splits == 3u ? lexb::splitk_reduce_kernel<3> : p->k_splits == 4u ? lexb::splitk_reduce_kernel<4> : lexb::splitk_reduce_kernel<0>;
                 LAUNCH_TRY(cudaLaunchKernelEx(&rc_cfg, reduce, static_cast<const float*>(p->partial), p->k_splits, elems,
@@ -1565,25 +1598,30 @@ int lexb_gemm_fp4_plan(lexb_gpu* g, uint32_t m, uint32_t n, uint32_t k, int resi
         // launch sums.  Smaller tiles: more of them; every weight is decoded once per tile of tokens, but a tile's
         // partial product and its store shrink with it and fewer splits are needed.  (Below 256 tokens a K step
         // costs about the same: it is the decode that bounds it, not the MMAs.)
-        // Every (tile, splits) pair is priced with figures fitted to 159 launches timed on a B200 (us): 4.5 overall; per
-        // wave of tiles 8.05 / 5.3 / 4.0 / 4.1 for a block's start and its store of a 512 / 256 / 128 / 64-token tile and
-        // 0.559 / 0.311 / 0.310 / 0.304 per K step; for the reduction launch its bytes at 3.33 TB/s minus 1.1.  The cheapest
-        // wins; a smaller tile or a further split must win by 2 %.  The fit (rms error 4 %) is that of the table decode: with
-        // the products a K step of the tiles up to 128 tokens takes 0.20-0.31 (17408 rows, k = 2048 to 8192), so they and
-        // their splits are priced up to a third too dear.
+        // Every (tile, splits) pair is priced (PairPrices), the cheapest wins; a smaller tile or a further split must win by 2 %.
         const uint32_t sm_pairs = static_cast<uint32_t>(g->prop.multiProcessorCount) / 2u;
         const uint32_t raw_blocks = k / lexb::PAIR_RAW_K;
         uint32_t splits = s.k_splits ? s.k_splits : 1u;
+        // The parts of K are summed in a cluster of their pairs where the device holds the clusters of all tiles at once - they are
+        // packed less tightly than pairs, and a second wave costs more than the reduction launch (m = 201, 6144 x 4096 in 3 parts:
+        // 24 clusters of 6, 18.2 us with the launch, 31.3 in clusters; in 2 parts 19.9 and 18.0) - and for tiles of up to 256
+        // tokens: those of 512 would take two turns of shared memory (512 x 5120 x 17408 in 3 parts: 84.0 and 86.5).  A split
+        // that the caller gives goes through the workspace.
+        auto in_cluster = [&](uint32_t tile_tokens, uint32_t tiles, uint32_t parts) {
+            return parts > 1u && parts <= lexb::PAIR_CLUSTER_SPLITS && tile_tokens <= 256u && tiles <= held_clusters(g, 2u * parts);
+        };
         {
-            // per tile size 512 / 256 / 128 / 64: us per K step, us per wave for a block's start and store
-            static const double kstep_us[4] = {0.559, 0.311, 0.310, 0.304}, wave_us[4] = {8.05, 5.32, 4.02, 4.14};
+            const PairPrices& price = pair_prices(m, n, k);
             auto model = [&](uint32_t ti, uint32_t c, uint32_t* eff_out) {
                 const uint32_t tt = 512u >> ti;
                 const uint32_t mt = (m + tt - 1u) / tt;
                 const uint32_t rbs = (raw_blocks + c - 1u) / c, eff = (raw_blocks + rbs - 1u) / rbs;
                 const double waves = static_cast<double>((mt * n_pairs * eff + sm_pairs - 1u) / sm_pairs);
-                double us = 4.51 + waves * (rbs * 4.0 * kstep_us[ti] + wave_us[ti]);
-                if (eff > 1u) us += -1.12 + static_cast<double>(eff) * m * n * 4.0 / 3.33e6;
+                const double mb = static_cast<double>(m) * n * 4e-6;                      // of y
+                double us = price.start + waves * (rbs * 4.0 * price.kstep[ti] + price.wave[ti]);
+                if (eff == 1u) us += price.store * mb;
+                else if (!s.k_splits && in_cluster(tt, mt * n_pairs, eff)) us += price.cluster + (price.cluster_mb * eff + price.store) * mb;
+                else us += price.reduce + price.reduce_mb * eff * mb;
                 *eff_out = eff;
                 return us;
             };
@@ -1592,7 +1630,7 @@ int lexb_gemm_fp4_plan(lexb_gpu* g, uint32_t m, uint32_t n, uint32_t k, int resi
             for (uint32_t ti = 0; ti < 4u; ti++) {
                 const uint32_t tt = 512u >> ti;
                 if (s.tm ? tt != s.tm : (tt != 64u && tt / 2u >= m)) continue;      // the caller's tile; or no tile more than half empty
-                for (uint32_t c = 1; c <= 8u && (c == 1u || raw_blocks / c >= 4u); c++) {
+                for (uint32_t c = 1; c <= 8u && (c == 1u || raw_blocks / c >= price.least); c++) {
                     if (s.k_splits && c != s.k_splits) continue;                    // the caller fixed the splits
                     uint32_t eff = 0;
                     const double us = model(ti, c, &eff);
@@ -1604,6 +1642,7 @@ int lexb_gemm_fp4_plan(lexb_gpu* g, uint32_t m, uint32_t n, uint32_t k, int resi
                     }
                 }
             }
+            p->us = best;
             splits = best_c;
             p->tm = best_tt;
             p->tok_blocks = best_tt == 512u ? 2u : 1u;
@@ -1646,6 +1685,9 @@ int lexb_gemm_fp4_plan(lexb_gpu* g, uint32_t m, uint32_t n, uint32_t k, int resi
         splits = (raw_blocks + rb_per_split - 1u) / rb_per_split;          // no empty split
         p->k_splits = splits;
         p->kb_per_split = rb_per_split * (lexb::PAIR_RAW_K / lexb::GEMM_BK);
+        // (a block's sums go where its rings were)
+        p->cluster_split = !s.k_splits && in_cluster(p->tm, tiles_final, splits) && env_u32("LEXB_CLUSTER_SPLIT", 1u) != 0u &&
+                           lexb::pair_ring_bytes(p->tok_blocks, stages, w_stages, raw_stages, w_tmem, k_sub, p->x_rows) >= p->tm * 512u;
         p->partial_borrowed = splits > 1u && t_plan_partial;
         if (p->partial_borrowed) {
             p->partial = t_plan_partial;
@@ -1676,7 +1718,7 @@ int lexb_gemm_fp4_plan(lexb_gpu* g, uint32_t m, uint32_t n, uint32_t k, int resi
         p->kc = v.kc; p->threads = 32u * v.warps; p->smem = v.smem; p->grid = v.clusters * v.cluster;
         snprintf(p->entry, sizeof p->entry, "%s_%u_%u_%u_%u_%u_%u", stem, m, n, k, m, lexb::MV_ROWS, lexb::MV_SLICE);
     }
-    if (!s.kernel && !s.tm && !s.stages && !s.kc && !s.w_stages && !s.k_splits && env_u32("LEXB_FEW", 0u) && (rc = plan_few(g, p))) return bail(rc);
+    if (!s.kernel && !s.tm && !s.stages && !s.kc && !s.w_stages && !s.k_splits && env_u32("LEXB_FEW", 1u) && (rc = plan_few(g, p))) return bail(rc);
     *out = p;
     return LEXB_OK;
 }
@@ -2248,7 +2290,19 @@ int lexb_gemm_fp4_splitk_static(lexb_gpu* g, uint32_t m, uint32_t n, uint32_t k,
     a.tmem_cols = p.tmem_cols; a.m_tiles = p.m_tiles; a.n_acc = 1;
     a.x_tx_bytes = lexb::PAIR_XBLK_BYTES;
     INJECT_LAUNCH();
-    lexb::gemm_fp4_tcgen05_pair_kernel<false><<<p.grid, p.threads, p.smem, g->stream>>>(map_x, map_wq, map_ws, a);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(p.grid);
+    cfg.blockDim = dim3(p.threads);
+    cfg.dynamicSmemBytes = p.smem;
+    cfg.stream = g->stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    CUDA_TRY(cudaLaunchKernelEx(&cfg, lexb::gemm_fp4_tcgen05_pair_kernel<false>, map_x, map_wq, map_ws, a));
     CUDA_TRY(cudaGetLastError());
     const size_t elems = mm * nn;
     const uint32_t blocks = static_cast<uint32_t>(std::min<size_t>((elems / 4 + 255) / 256, static_cast<size_t>(g->prop.multiProcessorCount) * 8u));

@@ -27,7 +27,6 @@ def check(got, want):
 def test_shares_that_cut_tiles(gpu, monkeypatch, m, cluster):
     """Every cluster size: shares that hold whole tiles and parts of two, that lie inside one tile, and tiles of one to several
     shares; one block of weights and odd numbers of them; with a residual."""
-    monkeypatch.setenv("LEXB_FEW", "1")
     monkeypatch.setenv("LEXB_FEW_C", str(cluster))
     for n, k in ((128, 256 * cluster), (640, 1280), (384, 256 * 17), (256, 512 * cluster)):
         x, wq, ws, wg = inputs.make_case(m, n, k, seed_base=700 + m)
