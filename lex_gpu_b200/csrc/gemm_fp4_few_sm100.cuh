@@ -12,8 +12,8 @@
 // Nothing of it passes through global memory, no block waits for another before that barrier, and a launch needs no
 // workspace.  The cuts depend on n, k and the cluster alone, so a token's bits do not depend on its batch.
 //
-// Roles (736 threads): warps 0-15 decode - four groups of four warps, of every block of weights group q has K step q (64
-// columns), a row a thread - into tensor memory, from where the MMAs take them as their A operand (M = 128 rows); warps
+// Roles (736 threads): warps 0-15 decode - eight take the even blocks of weights, eight the odd ones, a warp 32 rows and two of
+// the four K steps (64 columns each), a row a thread - into tensor memory, from where the MMAs take them as their A operand (M = 128 rows); warps
 // 16-19 the epilogue of a segment during the next one's main loop; warp 20 the copies of the packed weights, 21 of x, 22
 // the MMAs (N = 16, 32 or 64 tokens).
 //
@@ -108,8 +108,8 @@ gemm_fp4_few_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
         const uint32_t nbar = 2u * SR + 2u * SX + 2u * FEW_W_SLOTS + 4u, wb = 2u * SR + 2u * SX;
         for (uint32_t b = lane; b < nbar; b += 32u) {
             uint32_t count = 1;
-            if (b >= SR && b < 2u * SR) count = FEW_DEQ_WARPS;                       // raw_empty
-            if (b >= wb && b < wb + FEW_W_SLOTS) count = FEW_DEQ_WARPS;              // w_full
+            if (b >= SR && b < 2u * SR) count = FEW_DEQ_WARPS / FEW_W_SLOTS;         // raw_empty
+            if (b >= wb && b < wb + FEW_W_SLOTS) count = FEW_DEQ_WARPS / FEW_W_SLOTS;      // w_full
             if (b >= wb + 2u * FEW_W_SLOTS + 2u) count = 4u;                         // acc_empty: the epilogue warps
             mbar_init(bars + 8u * b, count);
         }
@@ -224,62 +224,79 @@ gemm_fp4_few_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
         }
         __syncwarp();
     } else if (warp < FEW_DEQ_WARPS) {
-        // ---------------------------------------------------------------- decode: K step q of every block of weights, a row a thread
-        const uint32_t r = tid & 127u, q = tid >> 7;
+        // ---------------------------------------------------------------- decode: half of every second block of weights, a row a thread
+        // Two sets of eight warps take the even and the odd blocks, each into a slot of its own; a warp has 32 rows and two of
+        // the four K steps, so that its waits, fences and arrivals - as long as the decode of a K step even where nothing is
+        // waited for - come once per two K steps.  (Its parity waits are right although it passes over every second block: before it
+        // stored the block before, the MMAs of the one before that were complete, so no barrier is two phases behind the one
+        // awaited as long as the ring of packed blocks has four.)
+        const uint32_t set = warp >> 3, half = (warp >> 2) & 1u, r = 32u * (warp & 3u) + lane;
         const uint32_t sw_xor = r & 7u;
         const uint8_t* const raw0 = smem + (raw_base - base) + r * 128u;
-        const uint32_t c0_off = ((2u * q) ^ sw_xor) << 4, c1_off = ((2u * q + 1u) ^ sw_xor) << 4;
-        const uint32_t sc_off = PAIR_RAW_WQ_BYTES - r * 128u + r * 16u + 4u * q;
-        const uint32_t tmem_row = tmem_base + ((32u * (warp & 3u)) << 16) + FEW_W_COL0 + 32u * q;
-        const float* wg_row = a.wg + (size_t)(t_lo + tile0) * FEW_ROWS + r;
-        RowScale g = make_row_scale(u0 < u1 ? __ldg(wg_row) : 0.0f);
-        uint32_t kb = kb0;
-        RingPos pr, pw;
-        for (uint32_t u = u0; u < u1; u++, pr.advance(SR), pw.advance(FEW_W_SLOTS)) {
-            float wg_next = 0.0f;
-            const bool tile_ends = kb + 1u == U;
-            if (tile_ends && u + 1u < u1) wg_next = __ldg(wg_row + FEW_ROWS);
+        const uint32_t sc_off = PAIR_RAW_WQ_BYTES - r * 128u + r * 16u + 8u * half;
+        const uint32_t dst = tmem_base + ((32u * (warp & 3u)) << 16) + FEW_W_COL0 + set * (STEPS * 32u) + 64u * half;
+        uint32_t kb = kb0 + set, tile = t_lo + tile0;
+        auto load_wg = [&](uint32_t t) { return t < tiles ? __ldg(a.wg + (size_t)t * FEW_ROWS + r) : 0.0f; };
+        float wg_now = load_wg(tile), wg_next = load_wg(tile + 1u);
+        RowScale g = make_row_scale(wg_now);
+        uint32_t turn = 0;                                                   // phase of this set's slot
+        RingPos pr;
+        pr.advance_by(set, SR);
+        for (uint32_t u = u0 + set; u < u1; u += FEW_W_SLOTS, kb += FEW_W_SLOTS, pr.advance_by(FEW_W_SLOTS, SR), turn ^= 1u) {
+            if (kb >= U) {                                                   // on to the tile that block is in
+                uint32_t over = 0;
+                do {
+                    kb -= U;
+                    over++;
+                } while (kb >= U);
+                tile += over;
+                g = make_row_scale(over == 1u ? wg_next : load_wg(tile));
+                wg_next = load_wg(tile + 1u);
+            }
             if (!__all_sync(0xFFFFFFFFu, mbar_wait(raw_full(pr.s), pr.ph, abort_flag))) {
                 atomicOr(a.status, ST_WAIT_X_FULL);
                 *abort_flag = 1;
                 break;
             }
             const uint8_t* const raw = raw0 + pr.s * PAIR_RAW_BYTES;
-            const uint4 c0 = *reinterpret_cast<const uint4*>(raw + c0_off);
-            const uint4 c1 = *reinterpret_cast<const uint4*>(raw + c1_off);
-            const uint32_t sc = *reinterpret_cast<const uint32_t*>(raw + sc_off);
-            __syncwarp();
-            if (lane == 0) mbar_arrive(raw_empty(pr.s));
-            uint4 o[8];
-            decode_row64(c0, c1, sc, g, o);
-            if (u >= u0 + FEW_W_SLOTS) {
-                if (early_w && u == u0 + FEW_W_SLOTS) grid_dependency_wait();      // first wait for a slot: join the stream's order
-                if (!__all_sync(0xFFFFFFFFu, mbar_wait(w_empty(pw.s), pw.ph ^ 1u, abort_flag))) {
-                    atomicOr(a.status, ST_WAIT_EMPTY_DEQ);
-                    *abort_flag = 1;
-                    break;
-                }
-                tc_fence_after_sync();
-            }
-            uint32_t v[32];
+            const uint2 sc = *reinterpret_cast<const uint2*>(raw + sc_off);
+            bool ok = true;
 #pragma unroll
-            for (uint32_t c = 0; c < 8; c++) {
-                v[4u * c + 0u] = o[c].x;
-                v[4u * c + 1u] = o[c].y;
-                v[4u * c + 2u] = o[c].z;
-                v[4u * c + 3u] = o[c].w;
+            for (uint32_t i = 0; i < 2; i++) {
+                const uint32_t q = 2u * half + i;
+                const uint4 c0 = *reinterpret_cast<const uint4*>(raw + (((2u * q) ^ sw_xor) << 4));
+                const uint4 c1 = *reinterpret_cast<const uint4*>(raw + (((2u * q + 1u) ^ sw_xor) << 4));
+                if (i == 1u) {
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(raw_empty(pr.s));
+                }
+                uint4 o[8];
+                decode_row64(c0, c1, i ? sc.y : sc.x, g, o);
+                if (i == 0u && u >= u0 + FEW_W_SLOTS) {
+                    if (early_w && u < u0 + 2u * FEW_W_SLOTS) grid_dependency_wait();      // first wait for a slot: join the stream's order
+                    if (!__all_sync(0xFFFFFFFFu, mbar_wait(w_empty(set), turn ^ 1u, abort_flag))) {
+                        atomicOr(a.status, ST_WAIT_EMPTY_DEQ);
+                        *abort_flag = 1;
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after_sync();
+                }
+                uint32_t v[32];
+#pragma unroll
+                for (uint32_t c = 0; c < 8; c++) {
+                    v[4u * c + 0u] = o[c].x;
+                    v[4u * c + 1u] = o[c].y;
+                    v[4u * c + 2u] = o[c].z;
+                    v[4u * c + 3u] = o[c].w;
+                }
+                tmem_st_32x32b_x32(dst + 32u * i, v);
             }
-            tmem_st_32x32b_x32(tmem_row + pw.s * (STEPS * 32u), v);
+            if (!ok) break;
             tmem_st_wait();
             tc_fence_before_sync();
             __syncwarp();
-            if (lane == 0) mbar_arrive(w_full(pw.s));
-            kb++;
-            if (tile_ends) {
-                kb = 0;
-                wg_row += FEW_ROWS;
-                g = make_row_scale(wg_next);
-            }
+            if (lane == 0) mbar_arrive(w_full(set));
         }
         __syncwarp();
         if (early_w) grid_dependency_wait();                                 // r and y belong to the stream's order

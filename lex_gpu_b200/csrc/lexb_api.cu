@@ -592,9 +592,9 @@ int plan_few(lexb_gpu* g, lexb_pipeline* p) {
     if (p->kernel != KERNEL_TCGEN05_PAIR && !env_u32("LEXB_FEW_C", 0)) return LEXB_OK;      // (the matvec keeps m <= 8)
     if (m > lexb::FEW_MAX_TOKENS || n % lexb::FEW_ROWS || k % lexb::FEW_K) return LEXB_OK;
     const uint32_t tiles = n / lexb::FEW_ROWS, U = k / lexb::FEW_K;
-    // Fitted to 839 shapes (m = 9-64, clusters of 1, 2, 3, 4, 6 and 8; rms error 6 %, the cluster chosen takes 0.4 % more than the fastest
-    // in the mean), us: 2.45, 1.21 per block of weights of the longest share and a little less with wider MMAs, the cluster's
-    // barriers and sums, the segments' stores, y.
+    // Fitted to 694 shapes (m = 9-64, clusters of 1, 2, 3, 4, 6 and 8; rms error 6.5 %, the cluster chosen takes 0.7 % more than the
+    // fastest in the mean), us: 2.95, 1.04 to 1.07 per block of weights of the longest share, the cluster's barriers and sums, the
+    // segments' stores, y.
     const uint32_t forced = env_u32("LEXB_FEW_C", 0);
     uint32_t best_c = 0, best_clusters = 0;
     double best = forced ? 1e30 : p->us;
@@ -603,8 +603,8 @@ int plan_few(lexb_gpu* g, lexb_pipeline* p) {
         const uint32_t clusters = std::min(held_clusters(g, c), tiles);
         if (!clusters || (tiles / clusters) * U < c) continue;
         const uint32_t blocks = ((tiles + clusters - 1u) / clusters * U + c - 1u) / c, segments = (blocks + U - 1u) / U;
-        const double us = 2.45 + blocks * (m <= 16u ? 1.21 : m <= 32u ? 1.195 : 1.154) + (c > 1u ? 1.88 + 0.005 * m : 0.0) + 0.0186 * segments * m +
-                          0.32e-5 * m * n;
+        const double us = 2.95 + blocks * (m <= 16u ? 1.039 : m <= 32u ? 1.045 : 1.07) + (c > 1u ? 1.76 + 0.0111 * m : 0.0) + 0.0085 * segments * m +
+                          0.376e-5 * m * n;
         if (us < best) {
             best = us;
             best_c = c;
@@ -619,7 +619,7 @@ int plan_few(lexb_gpu* g, lexb_pipeline* p) {
     f->m = m; f->n = n; f->k = k; f->tm = m;
     f->residual = p->residual; f->w_const = p->w_const; f->w_volatile = p->w_volatile;
     f->cluster = best_c; f->grid = best_c * best_clusters; f->threads = lexb::FEW_THREADS;
-    f->stages = env_u32("LEXB_FEW_SX", m <= 32u ? 4u : 3u); f->raw_stages = env_u32("LEXB_FEW_SR", m <= 32u ? 5u : 4u);
+    f->stages = env_u32("LEXB_FEW_SX", m <= 32u ? 4u : 3u); f->raw_stages = std::max(4u, env_u32("LEXB_FEW_SR", m <= 32u ? 5u : 4u));      // (four at least: see the decode)
     f->smem = lexb::few_smem_bytes(m, f->stages, f->raw_stages);
     if (f->smem > g->smem_optin) { delete f; return LEXB_OK; }
     p->few = f;
