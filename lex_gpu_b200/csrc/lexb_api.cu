@@ -779,7 +779,7 @@ int launch_one(lexb_gpu* g, const lexb_pipeline* p, const lexb_buffer* x, const 
         a.ws_pitch = p->ws_pitch;
         // a step on its own: the pieces kernel can be what it waits behind, and the weights are loaded beside that kernel
         const uint32_t pieces_fence = p->mq_pre && order.in_order ? 1u : 0u;
-        a.flags = order.early(p) || (pieces_fence && !p->w_volatile) ? 1u : 0u;
+        a.flags = (order.early(p) || (pieces_fence && !p->w_volatile) ? 1u : 0u) | (p->cluster > 1u ? 2u : 0u);
         lexb_pipeline::MapEntry nmaps = maps;         // placeholders when there is no hint (next_grid = 0)
         if (next && next->pipe && next->pipe->kernel == KERNEL_MATMUL_Q && next->pipe->gpu == g && next->wq && next->ws &&
             next->x && (a.flags & 1u) && get_maps(next->pipe, next->x->ptr, next->wq->ptr, next->ws->ptr, &nmaps) == LEXB_OK) {
@@ -792,11 +792,16 @@ int launch_one(lexb_gpu* g, const lexb_pipeline* p, const lexb_buffer* x, const 
         cfg.blockDim = dim3(p->threads);
         cfg.dynamicSmemBytes = p->smem;
         cfg.stream = g->stream;
-        cudaLaunchAttribute attr[1];
+        cudaLaunchAttribute attr[2];
         attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[0].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = (g->pdl && (!order.fence || p->mq_pre)) ? 1 : 0;      // (behind the pieces kernel, that one is the fence)
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = p->cluster;
+        attr[1].val.clusterDim.y = 1;
+        attr[1].val.clusterDim.z = 1;
+        const bool serial = !(g->pdl && (!order.fence || p->mq_pre));        // (behind the pieces kernel, that one is the fence)
+        cfg.attrs = serial ? attr + 1 : attr;
+        cfg.numAttrs = serial ? 1 : 2;
         a.trace = (g->d_trace && p->grid <= g->trace_ctas) ? g->d_trace : nullptr;
         const size_t pieces_bytes = lexb::matmul_q_pieces_bytes(p->m, p->k), sfb_bytes = lexb::matmul_q_sfb_total(p->m, p->k);
         if (p->mq_pre) {
@@ -1524,7 +1529,10 @@ int lexb_gemm_fp4_plan(lexb_gpu* g, uint32_t m, uint32_t n, uint32_t k, int resi
         // loaded ahead of the stream's order only when the caller declares them constant or a step list shows
         // that nothing in flight writes them (ListProof); never when the caller says they may change.
         p->flags = 0u;
-        if (splits > 1u) {
+        // The blocks of a row tile are a cluster and add up its splits there, where the device holds all of the launch's clusters at
+        // once (they are packed less tightly than blocks); else, and with a split that the caller gives, through a workspace.
+        if (splits > 1u && !s.k_splits && held_clusters(g, splits) >= tiles && env_u32("LEXB_CLUSTER_SPLIT", 1u) != 0u) p->cluster = splits;
+        if (splits > 1u && p->cluster == 1u) {
             // partial products [splits][m][n], then one arrival counter per row tile (zero between launches)
             const size_t pbytes = sizeof(float) * splits * static_cast<size_t>(m) * n;
             cudaError_t e = x_malloc(&p->partial, pbytes + sizeof(uint32_t) * tiles);

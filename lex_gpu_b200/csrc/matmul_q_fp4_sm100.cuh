@@ -95,6 +95,7 @@ struct MatmulQArgs {
     uint32_t k_splits, kb_per_split;   // in stages of 256
     uint32_t ws_pitch;                 // bytes per row of a scale load: min(64, k / 16)
     uint32_t flags;                    // bit 0: the weights are constant, load them before the launch ahead has finished
+                                       // bit 1: the blocks of a row tile are a cluster, which adds up its splits
     // The launch that follows this one in the step list, when it is of this kernel too (grid 0: none): its
     // blocks' first `next_stages` stages of weights are prefetched into L2 by this launch's blocks once
     // they have requested all of their own, so that DRAM keeps streaming through this launch's tail and the
@@ -241,6 +242,7 @@ matmul_q_fp4_kernel(const __grid_constant__ CUtensorMap tmap_wq, const __grid_co
     const uint32_t N = a.m * MQ_PIECES;
     const bool wide = N > 128u;                               // more than 16 tokens: one accumulator, two scale blocks of B per MMA
     const uint32_t sfb_bytes = matmul_q_sfb_bytes(a.m);
+    const bool in_cluster = (a.flags & 2u) != 0u;
     const long long t_start = clock64();
 
     if (warp == 0) {
@@ -470,48 +472,49 @@ matmul_q_fp4_kernel(const __grid_constant__ CUtensorMap tmap_wq, const __grid_co
         xv.lo = xv.hi = make_uint4(0, 0, 0, 0);
         xv.sc = 0.0f;
         if (xw < PW && xw < items) xv = load_chunk(xw / a.m, xw % a.m);
-        // largest magnitude of each token as f32 bits (its exponent gives the scale offset G); the
-        // tokens' loads go out together
-        for (uint32_t t0 = 0; t0 < a.m; t0 += 4u) {               // four tokens at a time (registers)
-            uint32_t mx[4] = {0, 0, 0, 0};
+        // Largest magnitude of each token as f32 bits (its exponent gives the scale offset G): up to four tokens at a time, the
+        // threads shared out over them and eight loads of each in flight - nothing can be multiplied before this is known, so
+        // the trips to L2 count (k = 17408, one token: two instead of three).
+        for (uint32_t t0 = 0; t0 < a.m; t0 += 4u) {
+            const uint32_t left = a.m - t0, lt = left == 1u ? 0u : left == 2u ? 1u : 2u;
+            const uint32_t share = (32u * MQ_PIECE_WARPS) >> lt, tok = t0 + xt / share, first = xt & (share - 1u);
             const uint4* xr = reinterpret_cast<const uint4*>(a.x);
             const uint32_t row_chunks = XF32 ? a.k / 4u : a.k / 8u;
-#pragma unroll 4
-            for (uint32_t i = xt; i < row_chunks; i += 32u * MQ_PIECE_WARPS) {
-                uint4 v[4];
+            uint32_t mx = 0;
+            constexpr uint32_t AHEAD = 8;
+            for (uint32_t i0 = tok < a.m ? first : row_chunks; i0 < row_chunks; i0 += AHEAD * share) {
+                uint4 v[AHEAD];
+                float sc[AHEAD];
 #pragma unroll
-                for (uint32_t t = 0; t < 4; t++)
-                    v[t] = t0 + t < a.m ? __ldg(xr + (size_t)(t0 + t) * row_chunks + i) : make_uint4(0, 0, 0, 0);
+                for (uint32_t e = 0; e < AHEAD; e++) {
+                    const uint32_t i = i0 + e * share;
+                    v[e] = i < row_chunks ? __ldg(xr + (size_t)tok * row_chunks + i) : make_uint4(0, 0, 0, 0);
+                    sc[e] = Q16 && i < row_chunks ? __ldg(a.xs + (size_t)tok * (a.k / 16u) + (i >> 1)) : 0.0f;
+                }
 #pragma unroll
-                for (uint32_t t = 0; t < 4; t++) {
+                for (uint32_t e = 0; e < AHEAD; e++) {
                     if (XF32) {
-                        mx[t] = max(max(mx[t], v[t].x & 0x7FFFFFFFu), v[t].y & 0x7FFFFFFFu);
-                        mx[t] = max(max(mx[t], v[t].z & 0x7FFFFFFFu), v[t].w & 0x7FFFFFFFu);
+                        mx = max(max(mx, v[e].x & 0x7FFFFFFFu), v[e].y & 0x7FFFFFFFu);
+                        mx = max(max(mx, v[e].z & 0x7FFFFFFFu), v[e].w & 0x7FFFFFFFu);
                     } else if (Q16) {
                         uint32_t fb[8];
-                        mq_q16_widen(v[t], t0 + t < a.m ? __ldg(a.xs + (size_t)(t0 + t) * (a.k / 16u) + (i >> 1)) : 0.0f, fb);
+                        mq_q16_widen(v[e], sc[e], fb);
 #pragma unroll
-                        for (uint32_t j = 0; j < 8; j++) mx[t] = max(mx[t], fb[j] & 0x7FFFFFFFu);
+                        for (uint32_t j = 0; j < 8; j++) mx = max(mx, fb[j] & 0x7FFFFFFFu);
                     } else {
-                        mx[t] = __vmaxu2(mx[t], v[t].x & 0x7FFF7FFFu);
-                        mx[t] = __vmaxu2(mx[t], v[t].y & 0x7FFF7FFFu);
-                        mx[t] = __vmaxu2(mx[t], v[t].z & 0x7FFF7FFFu);
-                        mx[t] = __vmaxu2(mx[t], v[t].w & 0x7FFF7FFFu);
+                        mx = __vmaxu2(mx, v[e].x & 0x7FFF7FFFu);
+                        mx = __vmaxu2(mx, v[e].y & 0x7FFF7FFFu);
+                        mx = __vmaxu2(mx, v[e].z & 0x7FFF7FFFu);
+                        mx = __vmaxu2(mx, v[e].w & 0x7FFF7FFFu);
                     }
                 }
             }
-#pragma unroll
-            for (uint32_t t = 0; t < 4; t++) {
-                if (t0 + t < a.m) {
-                    uint32_t r = mx[t];
-                    if (!XF32 && !Q16) {
-                        r = max(r & 0xFFFFu, r >> 16);
-                        r = __float_as_uint(__half2float(__ushort_as_half((unsigned short)r)));   // exact; inf and NaN stay so
-                    }
-                    r = __reduce_max_sync(0xFFFFFFFFu, r);
-                    if (lane == 0) atomicMax(tok_amax + t0 + t, r);
-                }
+            if (!XF32 && !Q16) {
+                mx = max(mx & 0xFFFFu, mx >> 16);
+                mx = __float_as_uint(__half2float(__ushort_as_half((unsigned short)mx)));   // exact; inf and NaN stay so
             }
+            mx = __reduce_max_sync(0xFFFFFFFFu, mx);              // (a warp's threads have one token)
+            if (lane == 0 && tok < a.m) atomicMax(tok_amax + tok, mx);
         }
         // B's scale blocks start as zeros: rows nobody writes must not hold stray NaN patterns
         for (uint32_t i = xt; i < S * (sfb_bytes / 16u); i += 32u * MQ_PIECE_WARPS) {
@@ -653,6 +656,7 @@ matmul_q_fp4_kernel(const __grid_constant__ CUtensorMap tmap_wq, const __grid_co
         // four tokens at a time, the first of it before the accumulators are complete.  So are the partial products below: one
         // trip to L2 each instead of one per value.
         const bool to_partial = a.k_splits > 1u;
+        float* const in_smem = reinterpret_cast<float*>(smem);         // (in a cluster: [token][128 rows], where the rings were)
         const uint32_t te_lane = PRE && lane < a.m ? __ldg(a.pre_amax + lane) >> 23 : 0u;      // (at most 32 tokens)
         float r4[4] = {0.f, 0.f, 0.f, 0.f};
         auto load4 = [&](uint32_t t0) {
@@ -700,11 +704,12 @@ matmul_q_fp4_kernel(const __grid_constant__ CUtensorMap tmap_wq, const __grid_co
                 if (row_nan || te == 255u) v = __uint_as_float(0x7FC00000u);
                 const size_t o = (size_t)t * a.n + n0 + row;
                 if (!to_partial && a.r) v += r_now[i];
-                out[o] = v;
+                if (in_cluster) in_smem[t * MQ_ROWS + row] = v;
+                else out[o] = v;
             }
             }
         }
-        if (a.k_splits > 1u) {
+        if (a.k_splits > 1u && !in_cluster) {
             // The last block of a row tile to get here adds up the splits, always in the order of the
             // splits, so the result does not depend on which block that is.  (A block that gave up
             // above still counts itself: the counter must be back at zero for the next launch.)
@@ -741,6 +746,31 @@ matmul_q_fp4_kernel(const __grid_constant__ CUtensorMap tmap_wq, const __grid_co
         }
     }
 
+    if (in_cluster) {
+        // Every split's sums are in its block's shared memory: added in the order of the splits, as above, without the trips
+        // through L2 (store, count, load); four rows a thread, shared out over the cluster.
+        const uint32_t i0 = split * NTHREADS + tid;
+        const size_t o0 = (size_t)(i0 >> 5) * a.n + n0 + (i0 & 31u) * 4u;
+        float4 r0 = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (warp != 0u && a.r && i0 < a.m * 32u) r0 = __ldg(reinterpret_cast<const float4*>(a.r + o0));
+        cluster_sync_all();
+        for (uint32_t i = i0; i < a.m * 32u; i += a.k_splits * NTHREADS) {
+            const uint32_t tok = i >> 5, quad = i & 31u;
+            const size_t o = (size_t)tok * a.n + n0 + quad * 4u;
+            float4 part[MQ_MAX_SPLITS];
+#pragma unroll
+            for (uint32_t sp = 0; sp < MQ_MAX_SPLITS; sp++)
+                if (sp < a.k_splits) part[sp] = ld_shared_cluster_f32x4(map_to_cta(base + tok * (MQ_ROWS * 4u) + quad * 16u, sp));
+            float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+            auto add = [&](const float4& v) { s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w; };
+#pragma unroll
+            for (uint32_t sp = 0; sp < MQ_MAX_SPLITS; sp++)
+                if (sp < a.k_splits) add(part[sp]);
+            if (a.r) add(i == i0 && warp != 0u ? r0 : __ldg(reinterpret_cast<const float4*>(a.r + o)));
+            *reinterpret_cast<float4*>(a.y + o) = s;
+        }
+        cluster_sync_all();                                   // a block's sums are read by the others until here
+    }
     tc_fence_before_sync();
     __syncthreads();
     if (TRACE && a.trace && tid == 0) a.trace[16ull * blockIdx.x + 10] = (unsigned long long)clock64();   // block done
