@@ -578,12 +578,13 @@ struct PairPrices {
     uint32_t least;
 };
 // Fitted to 4,466 launches of 487 shapes (m = 9-2048, n = 128-28672, k = 256-17408) on a B200: rms error 5 %, the form chosen takes
-// 0.8 % more than the fastest in the mean, where the prices before (159 launches with the table decode) took 9 % more.  Past 60
-// GFLOP a launch runs into the power cap, which bursts of launches do not show: those prices stay there.
+// 0.8 % more than the fastest in the mean, where the prices before (159 launches with the table decode) took 9 % more.  Past 10
+// GFLOP of more than 64 tokens a launch that is repeated runs into the power cap, which bursts of launches do not show (1572 x 6656 x
+// 1024 with down behind it: 62.4 us by the prices before, 64.6 by these), and these gain 1 % at most: those prices stay there.
 const PairPrices& pair_prices(uint32_t m, uint32_t n, uint32_t k) {
     static const PairPrices FITTED = {0.20, {0.598, 0.337, 0.319, 0.319}, {7.69, 5.85, 4.46, 3.70}, 0.157, 1.04, 0.288, 0.25, 0.271, 2u},
                             LARGE = {4.51, {0.559, 0.311, 0.310, 0.304}, {8.05, 5.32, 4.02, 4.14}, 0.0, -1.12, 0.300, -1.12, 0.300, 4u};
-    return 2.0 * m * n * k < 6e10 ? FITTED : LARGE;
+    return m <= 64u || 2.0 * m * n * k < 1e10 ? FITTED : LARGE;
 }
 
 // The few-token kernel's launch for a pipeline, if it takes the shape.
