@@ -34,7 +34,7 @@ def both_ways(gpu, plan, m, n, k, residual):
 
 
 @pytest.mark.parametrize("m,n,k,residual", [(65, 256, 1024, True), (100, 384, 2048, False), (130, 512, 2048, True), (257, 256, 2048, False),
-                                            (1024, 2048, 4096, True), (200, 640, 768, False)])
+                                            (1024, 2048, 4096, True), (200, 640, 1280, False)])
 def test_two_cta_gemm(gpu, m, n, k, residual):
     """Tiles of 64 to 256 tokens, a last tile of few tokens, an odd last pair of rows, parts of unequal length."""
     plan = lambda *a, **kw: gpu.plan_gemm_fp4(*a, kernel=3, **kw)
