@@ -95,7 +95,8 @@ typedef struct lexb_lowered {
     uint32_t m, n, k, residual;
     uint32_t bm, bn, bk, stages;
     uint32_t k_splits;           /* > 1: a second launch sums the partial products */
-    uint64_t scratch_bytes;      /* Lowered::scratch_bytes: the split-K workspace */
+    uint64_t scratch_bytes;      /* Lowered::scratch_bytes: the split-K workspace (launches that sum their parts within clusters,
+                                    and those of 9 to 64 tokens that run as one stream of weights per SM, do not use it) */
 } lexb_lowered;
 
 /* lex_cuda::Step, crates/lex-cuda/src/device.rs:314: a pipeline and its buffers in binding

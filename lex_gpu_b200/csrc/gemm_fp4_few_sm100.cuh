@@ -17,6 +17,10 @@
 // 16-19 the epilogue of a segment during the next one's main loop; warp 20 the copies of the packed weights, 21 of x, 22
 // the MMAs (N = 16, 32 or 64 tokens).
 //
+// What bounds it: the decode warps' turns, half decode (560 of 1450 clocks a K step when a turn was one K step) and half barriers,
+// stores and fences; without the decode 28672 x 4096 takes 21.6 us at 32 tokens, without the MMAs 29.3, with everything 32.0 and, with
+// two K steps a turn, 28.0 (the two-CTA kernel: 41.2; the bytes alone 10.7).  17408 x 5120 at 64 tokens: 24.9 -> 20.0 us.
+//
 // Tensor memory: columns 0-255 two sets of accumulators (segments alternate), 128 columns each: 8, 4 or 2 accumulators of N
 // columns that take the K steps in turn, so that each has an eighth, a quarter or half of the truncating additions; columns
 // 256-511 the decoded weights, two blocks.
