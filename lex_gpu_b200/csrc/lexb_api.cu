@@ -1658,9 +1658,9 @@ int lexb_gemm_fp4_plan(lexb_gpu* g, uint32_t m, uint32_t n, uint32_t k, int resi
             p->m_tiles = (m + p->tm - 1u) / p->tm;
         }
         p->x_rows = p->tm == 512u ? lexb::PAIR_XBLK_ROWS : p->tm / 2u;
-        // packed-weight blocks in flight: 2; 3 with tiles of 128 tokens or fewer, whose K step is short enough for the
-        // third block's trip to HBM to show (2-3 % per launch)
-        const uint32_t raw_stages = env_u32("LEXB_RAWSTAGES", p->tm <= 128u ? 3u : lexb::PAIR_RAW_STAGES);
+        // packed-weight blocks in flight: 2; 5 with tiles of 128 tokens or fewer, whose decode takes every second block (two more
+        // than the W ring's 3 stages: see the kernel's `paired`), or 3 beside ring depths that the caller gives
+        const uint32_t raw_stages = env_u32("LEXB_RAWSTAGES", p->tm > 128u ? lexb::PAIR_RAW_STAGES : s.stages || s.w_stages ? 3u : 5u);
         p->raw_stages = raw_stages;
         if (splits < 1u || splits > raw_blocks) return bail(fail(LEXB_ERR_ARG, "k_splits = %u outside [1, %u]", splits, raw_blocks));
         // Ring depths.  Tiles of 512 tokens: x ring of 4 stages of 32 KiB, W ring of 3 of 16 KiB, two packed-weight
