@@ -77,7 +77,7 @@ constexpr uint32_t MQC_MAX_TOKENS = 8;
 
 __host__ __device__ constexpr uint32_t matmul_q_chain_smem_bytes(uint32_t stages, uint32_t m) {
     return stages * matmul_q_stage_bytes(m <= 4u ? 4u : 8u) + MQ_WS_SLOTS * MQ_WS_SLOT_BYTES + (3u * stages + 4u + 2u * MQ_WS_SLOTS) * 8u + 64u +
-           2u * MQ_ROWS + 1024u;
+           4u * MQ_ROWS + 1024u;
 }
 
 constexpr uint32_t MQC_THREADS_PRE = 32u * MQC_WARP_PIECE;
@@ -113,7 +113,10 @@ __global__ void __launch_bounds__(PRE ? MQC_THREADS_PRE : MQC_THREADS, 1) matmul
     uint32_t* const tmem_slot = misc;
     volatile uint32_t* const abort_flag = misc + 1;
     uint32_t* const tok_amax = misc + 2;                                  // [2 sets][4 tokens]
-    volatile uint8_t* const nan_rows = reinterpret_cast<volatile uint8_t*>(misc + 16);    // [2 sets][MQ_ROWS]
+    // [MQ_ROWS]: a NaN scale byte seen, a bit per part of K, its count modulo 32.  The scale warps run ahead of the epilogue by more
+    // parts than there are accumulator sets: at a stage they have seen the MMAs of the one S before complete, so the part two
+    // before that one's is stored, and with parts of a single stage S + 2 of them are open - at most 10, of 32 bits.
+    uint32_t* const nan_parts = misc + 16;
 
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
     const uint32_t N = a.m * MQ_PIECES;
@@ -156,7 +159,7 @@ __global__ void __launch_bounds__(PRE ? MQC_THREADS_PRE : MQC_THREADS, 1) matmul
         __syncwarp();
         fence_mbar_init();
     }
-    for (uint32_t i = tid; i < 2u * MQ_ROWS; i += NTHREADS) nan_rows[i] = 0;
+    for (uint32_t i = tid; i < MQ_ROWS; i += NTHREADS) nan_parts[i] = 0;
     if (warp == 1) {
         tmem_alloc(smem_u32(tmem_slot), MQ_TMEM_COLS);
         tmem_relinquish();
@@ -326,15 +329,12 @@ __global__ void __launch_bounds__(PRE ? MQC_THREADS_PRE : MQC_THREADS, 1) matmul
         for (Tiles ct(a.tiles); ct.more() && ok; ct.next(), sub++) {
             const uint32_t KB = ct.cur.kb(), per = ct.cur.per, ws_pitch = ct.cur.ws_pitch();
             uint32_t part_end = per;
-            bool flags_free = false;                      // this set's NaN flags are cleared by the epilogue of the part before last
             for (uint32_t kb = 0; kb < KB; kb++, ps.advance(S), gs++) {
                 if (kb == part_end) {
                     part_end += per;
                     sub++;
-                    flags_free = false;
                 }
                 if ((gs & 1u) != par) continue;
-                const uint32_t set = sub & 1u, use = sub >> 1;
                 const uint32_t s = ps.s, ph = ps.ph;
                 if (!__all_sync(0xFFFFFFFFu, mbar_wait(empty(s), ph ^ 1u, abort_flag))) {
                     atomicOr(a.status, ST_WAIT_EMPTY_DEQ);
@@ -384,15 +384,7 @@ __global__ void __launch_bounds__(PRE ? MQC_THREADS_PRE : MQC_THREADS, 1) matmul
                     if ((z - 0x01010101u) & ~z & 0x80808080u) {
                         for (uint32_t i = 0; i < 4; i++) {
                             if (((v >> (8u * i)) & 0xFFu) == 0x7Fu) {
-                                if (!flags_free && use == 0u) flags_free = true;
-                                if (!flags_free) {
-                                    flags_free = mbar_wait(acc_empty(set), (use - 1u) & 1u, abort_flag);
-                                    if (!flags_free) {
-                                        atomicOr(a.status, ST_WAIT_ACC);
-                                        *abort_flag = 1;
-                                    }
-                                }
-                                nan_rows[set * MQ_ROWS + row] = 1;
+                                atomicOr(nan_parts + row, 1u << (sub & 31u));
                                 v &= ~(0xFFu << (8u * i));
                             }
                         }
@@ -443,7 +435,9 @@ __global__ void __launch_bounds__(PRE ? MQC_THREADS_PRE : MQC_THREADS, 1) matmul
                     break;
                 }
                 tc_fence_after_sync();
-                const bool row_nan = nan_rows[set * MQ_ROWS + row] != 0;
+                const uint32_t nan_bit = 1u << (sub & 31u);
+                const bool row_nan = (*static_cast<volatile uint32_t*>(nan_parts + row) & nan_bit) != 0u;
+                if (row_nan) atomicAnd(nan_parts + row, ~nan_bit);
 #pragma unroll
                 for (uint32_t t = 0; t < MQC_MAX_TOKENS; t++) {
                     if (t >= a.m) break;
@@ -465,8 +459,7 @@ __global__ void __launch_bounds__(PRE ? MQC_THREADS_PRE : MQC_THREADS, 1) matmul
                     total[t] = per < KB ? total[t] + v : v;
                     if (kb + per >= KB && in_n) y_p[(size_t)t * n + n0 + row] = r_p ? total[t] + res[t] : total[t];
                 }
-                nan_rows[set * MQ_ROWS + row] = 0;
-                // the accumulators (and this set's flags) are free for the part after next
+                // the accumulators are free for the part after next
                 tc_fence_before_sync();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(acc_empty(set));

@@ -82,6 +82,43 @@ def test_bad_scale_bytes_in_one_part_of_k(gpu):
     assert gpu.status_word() == 0
 
 
+@pytest.mark.parametrize("m,k,mixed", [(4, 512, True), (3, 512, True), (8, 512, True), (4, 512, False), (1, 512, True)])
+def test_bad_scale_bytes_in_later_tiles_of_few_stages(gpu, m, k, mixed):
+    """Tiles of two stages, five and more of them a block: the scale warps are several tiles ahead of the epilogue, and a
+    NaN scale byte still reaches its own row of its own tile and no other."""
+    shapes = ([(640, 17408)] if mixed else []) + [(16384, k)] * 6
+    xs = {kk: inputs.make_x(m, kk, seed_base=630) for _, kk in shapes}
+    xb = {kk: gpu.upload(x) for kk, x in xs.items()}
+    rng = np.random.Generator(np.random.PCG64(631))
+    sets, rows = [], []
+    for i, (n, kk) in enumerate(shapes):
+        wq, ws, wg = inputs.make_weights(n, kk, seed_base=632, copy=i)
+        bad = rng.choice(n, size=n // 100, replace=False)          # one row in a hundred: most tiles have one
+        ws = ws.copy()
+        ws[bad, rng.integers(0, kk // 16, size=bad.size)] = rng.choice(np.array([0x7F, 0xFF], dtype=np.uint8), size=bad.size)
+        sets.append((wq, ws, wg))
+        rows.append(set(bad.tolist()))
+    pipes = [gpu.plan_matmul_fp4(m, n, kk) for n, kk in shapes]
+    ys = [gpu.alloc(4 * m * n) for n, _ in shapes]
+    binds = [L.QBuf(gpu, *w).bind(xb[kk], None, y) for w, (_, kk), y in zip(sets, shapes, ys)]
+    alone = []
+    for pipe, bind, y, (n, _) in zip(pipes, binds, ys, shapes):
+        gpu.run(pipe, bind)
+        gpu.sync()
+        alone.append(gpu.download(y, np.float32, (m, n)))
+    steps = L.StepList(list(zip(pipes, binds)))
+    assert gpu.list_runs(steps) == [len(shapes)] * len(shapes)
+    for _ in range(3):
+        for y in ys:
+            gpu.memset(y, 0)
+        gpu.run_launches(steps)
+        for i, (n, _) in enumerate(shapes):
+            got = gpu.download(ys[i], np.float32, (m, n))
+            assert set(np.flatnonzero(np.isnan(got).any(axis=0)).tolist()) == rows[i]
+            assert np.array_equal(got, alone[i], equal_nan=True)
+    assert gpu.status_word() == 0
+
+
 def test_lists_of_growing_activations_on_two_streams(gpu):
     """The digit rows of a run live in an arena per stream that grows with the lists: results stay right when a later list needs
     more of it, an earlier one comes again, and another stream has its own."""
