@@ -221,18 +221,14 @@ __global__ void __launch_bounds__(PRE ? MQC_THREADS_PRE : MQC_THREADS, 1) matmul
                         ok = false;
                         break;
                     }
-                    if ((kb & (MQ_WS_GROUP - 1u)) == 0u) {
-                        // scale bytes one group ahead of the codes (two at the very start)
-                        g_begun++;
-                        while (g_issued < g_begun + 1u && gt.more() && ok) ok = issue_group();
-                        if (!ok) break;
-                    }
+                    const bool group_starts = (kb & (MQ_WS_GROUP - 1u)) == 0u;
+                    if (group_starts) g_begun++;
                     mbar_arrive_expect_tx(raw_full(s), MQ_CODE_BYTES + (PRE ? b_bytes + MQ_SF_BYTES : 0u));
                     tma_load_2d(codes_of(s), &a.jobs[ct.cur.job].wq, (int)(kb * (MQ_STAGE_K / 2)), (int)ct.cur.n0, raw_full(s));
                     if (PRE) {
                         // The digit rows are written by the launch ahead: the first ring of weights goes out
                         // before that launch is waited for, the digit rows of those stages (slot = stage) after.
-                        if (filled + 1u == S || (ct.last() && kb + 1u == KB)) join_order();
+                        if (filled + 1u == S || (ct.last() && kb + 1u == KB) || (group_starts && g_begun >= MQ_WS_SLOTS)) join_order();
                         if (in_order) {
                             for (; b_issued <= filled; b_issued++, b_kb++) {
                                 if (b_kb == bt.cur.kb()) {   // the next tile of this block
@@ -246,6 +242,13 @@ __global__ void __launch_bounds__(PRE ? MQC_THREADS_PRE : MQC_THREADS, 1) matmul
                                 tma_load_1d(sfb_of(bs), b_sfb + (size_t)b_kb * MQ_SF_BYTES, MQ_SF_BYTES, raw_full(bs));
                             }
                         }
+                    }
+                    if (group_starts) {
+                        // Scale bytes one group ahead of the codes (two at the very start), behind everything the stages so far are
+                        // made of: from the fourth group on this waits for scale warps, and one that has met a negative scale byte
+                        // waits for its stage to be whole - with tiles of 3, 6 or 7 stages before the first ring is full.
+                        while (g_issued < g_begun + 1u && gt.more() && ok) ok = issue_group();
+                        if (!ok) break;
                     }
                 }
             }

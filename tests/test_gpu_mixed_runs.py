@@ -119,6 +119,41 @@ def test_bad_scale_bytes_in_later_tiles_of_few_stages(gpu, m, k, mixed):
     assert gpu.status_word() == 0
 
 
+@pytest.mark.parametrize("m,ks", [(4, (768,)), (8, (768,)), (3, (1536, 768)), (4, (1792,)), (1, (1536, 512)), (6, (1792, 768, 512))])
+def test_negative_scale_bytes_in_tiles_of_few_stages(gpu, m, ks):
+    """Tiles of 2, 3, 6 and 7 stages: their groups of scale bytes fill the ring before the first stages' digit rows are due, and a
+    negative scale byte waits for its stage.  Signs and NaN bytes in every tile; each step's bits are those of its own launch."""
+    shapes = [(16384, k) for k in ks for _ in range(3)]
+    xb = {k: gpu.upload(inputs.make_x(m, k, seed_base=640)) for k in ks}
+    rng = np.random.Generator(np.random.PCG64(641))
+    pipes, binds, ys, rows = [], [], [], []
+    for i, (n, k) in enumerate(shapes):
+        wq, ws, wg = inputs.make_weights(n, k, seed_base=642, copy=i)
+        ws = np.where(rng.random(ws.shape) < 0.1, ws | 0x80, ws).astype(np.uint8)
+        bad = rng.choice(n, size=n // 100, replace=False)
+        ws[bad, rng.integers(0, k // 16, size=bad.size)] = rng.choice(np.array([0x7F, 0xFF], dtype=np.uint8), size=bad.size)
+        y = gpu.alloc(4 * m * n)
+        pipes.append(gpu.plan_matmul_fp4(m, n, k))
+        binds.append(L.QBuf(gpu, wq, ws, wg).bind(xb[k], None, y))
+        ys.append(y)
+        rows.append(set(bad.tolist()))
+    alone = []
+    for pipe, bind, y, (n, _) in zip(pipes, binds, ys, shapes):
+        gpu.run(pipe, bind)
+        gpu.sync()
+        alone.append(gpu.download(y, np.float32, (m, n)))
+    steps = L.StepList(list(zip(pipes, binds)))
+    assert gpu.list_runs(steps) == [len(shapes)] * len(shapes)
+    for y in ys:
+        gpu.memset(y, 0)
+    gpu.run_launches(steps)
+    for i, (n, _) in enumerate(shapes):
+        got = gpu.download(ys[i], np.float32, (m, n))
+        assert np.array_equal(got, alone[i], equal_nan=True)
+        assert set(np.flatnonzero(np.isnan(got).any(axis=0)).tolist()) == rows[i]
+    assert gpu.status_word() == 0
+
+
 def test_lists_of_growing_activations_on_two_streams(gpu):
     """The digit rows of a run live in an arena per stream that grows with the lists: results stay right when a later list needs
     more of it, an earlier one comes again, and another stream has its own."""

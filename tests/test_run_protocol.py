@@ -28,9 +28,10 @@ class Bar:
         return (self.done & 1) != parity
 
 
-def run(tiles, S, seed, negative=(), nan=(), flags="parts"):
+def run(tiles, S, seed, negative=(), nan=(), flags="parts", held_back=False):
     """`tiles`: (stages, stages per part of K); `negative`, `nan`: the stages with such a scale byte.  flags="sets": one flag per set
-    of accumulators behind a parity wait for the part two before.  -> parts found flagged, most parts open at once, errors."""
+    of accumulators behind a parity wait for the part two before.  `held_back`: the copy engine asks for a stage's scale bytes ahead of
+    its codes and digit rows.  -> parts found flagged, most parts open at once, errors."""
     rnd = random.Random(seed)
     stages, parts, groups = [], 0, 0                          # (part, first of a group, group, a tile's stage), ...
     group_stages = []
@@ -54,20 +55,25 @@ def run(tiles, S, seed, negative=(), nan=(), flags="parts"):
 
     def copy():
         issued = begun = digits = 0
+        ordered = False                                       # the launch ahead has been waited for
         for i, (_, _, g) in enumerate(stages):
             yield from wait(empty[i % S], i // S - 1, f"copy empty {i}")
-            if i == group_stages[g][0]:
-                begun += 1
-                while issued < min(begun + 1, groups):
+            starts = i == group_stages[g][0]
+            begun += starts
+            for what in ("groups", "stage") if held_back else ("stage", "groups"):
+                if what == "stage":
+                    raw_full[i % S].arrive()
+                    yield
+                    ordered |= i + 1 >= S or i + 1 == len(stages) or (starts and begun >= WS_SLOTS and not held_back)
+                    for d in range(digits, i + 1 if ordered else digits):
+                        raw_full[d % S].arrive()
+                        digits = d + 1
+                    continue
+                while starts and issued < min(begun + 1, groups):
+                    ordered |= issued >= WS_SLOTS
                     yield from wait(ws_empty[issued % WS_SLOTS], issued // WS_SLOTS - 1, f"copy ws_empty {issued}")
                     ws_full[issued % WS_SLOTS].arrive()
                     issued += 1
-            raw_full[i % S].arrive()
-            yield
-            if i + 1 >= S or i + 1 == len(stages) or issued > WS_SLOTS:      # the launch ahead has been waited for
-                for d in range(digits, i + 1):
-                    raw_full[d % S].arrive()
-                digits = i + 1
 
     def scale(par):
         for i, (p, _, g) in enumerate(stages):
@@ -155,3 +161,20 @@ def test_flags_per_accumulator_set_would_be_found_by_another_part():
         found, _, want, _ = run([(2, 2)] * 12, 8, seed, nan={8}, flags="sets")      # the block's fifth tile of two stages
         wrong += set(found) != want
     assert wrong
+
+
+@pytest.mark.parametrize("S", [7, 8])
+@pytest.mark.parametrize("tiles", SHAPES)
+def test_negative_scale_bytes_wait_for_nothing_that_is_held_back(tiles, S):
+    for seed in range(15):
+        rnd = random.Random(2000 + seed)
+        total = sum(kb for kb, _ in tiles)
+        negative = {0, 1} | set(rnd.sample(range(total), total // 3))
+        nan = set(rnd.sample(range(total), 2))
+        found, _, want, errors = run(tiles, S, seed, negative=negative, nan=nan)
+        assert not errors and set(found) == want
+
+
+@pytest.mark.parametrize("tiles", [[(3, 3)] * 10, [(6, 6)] * 5, [(7, 7)] * 4])
+def test_digit_rows_held_back_would_stop_a_run_of_few_stages(tiles):
+    assert run(tiles, 8, 0, negative={0}, held_back=True)[3] == ["nothing moves"]
