@@ -119,7 +119,7 @@ struct lexb_gpu {
     // Job tables of chained runs, kept by content: a decode loop issues the same lists token after token, and a
     // table found here needs no copy in front of its launch (a copy would put the launch behind the whole
     // kernel before it).  A table is never written again once copied.
-    // (the jobs, then the table of tiles, which follows from them and the device)
+    // (the jobs, then the table of tiles, which follows from them - their parts of K among them - and the device)
     struct ChainTable { std::vector<lexb::MqChainJob> host; std::vector<lexb::MqChainTile> tiles; uint32_t grid; lexb::MqChainJob* dev; };
     std::unordered_multimap<uint64_t, ChainTable> chain_tables;
     // Digit rows of a run's activations (matmul_q_pieces_kernel's output: [8 m][k / 2] digit rows, [k / 256][2048]
@@ -988,6 +988,9 @@ size_t chain_run(const lexb_gpu* g, const lexb_step* steps, size_t nsteps, size_
     return single && steps[i].pipeline->k_splits == 1u && tiles > static_cast<uint32_t>(g->prop.multiProcessorCount) ? 1 : 0;
 }
 
+// Stages per part of K of a step in a run.
+uint32_t chain_part(const lexb_pipeline* p) { return p->k_splits == 1u ? p->k / lexb::MQ_STAGE_K : p->kb_per_split; }
+
 // The table of a run's row tiles: block b works through entries b, b + grid, ...; a row of entries without a job ends it.  Tiles go
 // to the block with the fewest stages so far, the longest tiles first, so that steps of several K end together.
 std::vector<lexb::MqChainTile> chain_tiles(const lexb_step* steps, size_t count, uint32_t sms, uint32_t* grid_out) {
@@ -1019,7 +1022,7 @@ std::vector<lexb::MqChainTile> chain_tiles(const lexb_step* steps, size_t count,
                 b = l.second;
                 least.emplace(l.first + e.first, b);
             }
-            of[b].push_back(lexb::MqChainTile{e.second, n0, e.first | (p->ws_pitch << 16), p->k_splits == 1u ? e.first : p->kb_per_split});
+            of[b].push_back(lexb::MqChainTile{e.second, n0, e.first | (p->ws_pitch << 16), chain_part(p)});
         }
     }
     size_t rows = 0;
@@ -1067,6 +1070,7 @@ int launch_chain(lexb_gpu* g, const lexb_step* steps, size_t count, bool fence) 
         jobs[i].y = static_cast<float*>(y->ptr);
         jobs[i].n = p->n;
         jobs[i].k = p->k;
+        jobs[i].per = chain_part(p);
         if (pre) {
             size_t e = 0;
             while (e < acts.size() && (acts[e].x != x->ptr || acts[e].k != p->k)) e++;

@@ -43,7 +43,8 @@ struct alignas(64) MqChainJob {
     // PRE: what matmul_q_pieces_kernel wrote for this step's x
     const uint8_t* pre_sfb;  // [k / 256][2048] scale blocks of the digit rows
     const uint32_t* pre_amax;// [m] largest magnitudes, f32 bits
-    uint64_t pad[1];
+    uint32_t per;            // stages per part of K (the host's: tables are told apart by it; blocks have it in their tiles)
+    uint32_t pad;
     CUtensorMap pre;         // digit rows [8 m][k / 2]
 };
 static_assert(sizeof(MqChainJob) % 64 == 0, "tensor maps of a job table sit on 64-byte boundaries");

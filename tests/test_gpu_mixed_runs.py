@@ -154,6 +154,36 @@ def test_negative_scale_bytes_in_tiles_of_few_stages(gpu, m, ks):
     assert gpu.status_word() == 0
 
 
+@pytest.mark.parametrize("m", [1, 4])
+def test_plans_of_other_splits_over_the_same_buffers(gpu, m):
+    """A list planned with K whole and one with the planner's split, over the same buffers and in either order: each is summed as its
+    own launches are."""
+    shapes = [(640, 17408), (384, 8192)]
+    xb = {k: gpu.upload(inputs.make_x(m, k, seed_base=650)) for _, k in shapes}
+    plans = {which: [gpu.plan_matmul_fp4(m, n, k, k_splits=which) for n, k in shapes] for which in (0, 1)}
+    assert all(p.describe().k_splits > 1 for p in plans[0]) and all(p.describe().k_splits == 1 for p in plans[1])
+    for order in ((1, 0), (0, 1)):
+        sets = [L.QBuf(gpu, *inputs.make_weights(n, k, seed_base=651, copy=i + 2 * order[0])) for i, (n, k) in enumerate(shapes)]
+        ys = [gpu.alloc(4 * m * n) for n, _ in shapes]
+        binds = [q.bind(xb[k], None, y) for q, (_, k), y in zip(sets, shapes, ys)]
+
+        def results():
+            return [gpu.download(y, np.float32, (m, n)) for y, (n, _) in zip(ys, shapes)]
+
+        alone = {}
+        for which in order:
+            for pipe, bind in zip(plans[which], binds):
+                gpu.run(pipe, bind)
+            gpu.sync()
+            alone[which] = results()
+        assert not np.array_equal(alone[0][0], alone[1][0])        # (or the test tells nothing)
+        for which in order:
+            for y in ys:
+                gpu.memset(y, 0xEE)
+            gpu.run_launches(list(zip(plans[which], binds)))
+            assert all(np.array_equal(a, b) for a, b in zip(results(), alone[which])), (order, which)
+
+
 def test_lists_of_growing_activations_on_two_streams(gpu):
     """The digit rows of a run live in an arena per stream that grows with the lists: results stay right when a later list needs
     more of it, an earlier one comes again, and another stream has its own."""
