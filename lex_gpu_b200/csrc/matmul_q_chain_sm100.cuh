@@ -229,7 +229,7 @@ __global__ void __launch_bounds__(PRE ? MQC_THREADS_PRE : MQC_THREADS, 1) matmul
                     if (PRE) {
                         // The digit rows are written by the launch ahead: the first ring of weights goes out
                         // before that launch is waited for, the digit rows of those stages (slot = stage) after.
-                        if (filled + 1u == S || (ct.last() && kb + 1u == KB) || (group_starts && g_begun >= MQ_WS_SLOTS)) join_order();
+                        if (!in_order && (filled + 1u == S || (group_starts && g_begun >= MQ_WS_SLOTS) || (ct.last() && kb + 1u == KB))) join_order();
                         if (in_order) {
                             for (; b_issued <= filled; b_issued++, b_kb++) {
                                 if (b_kb == bt.cur.kb()) {   // the next tile of this block
