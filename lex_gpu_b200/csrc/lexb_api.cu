@@ -13,6 +13,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <initializer_list>
 #include <mutex>
 #include <new>
 #include <queue>
@@ -150,11 +151,13 @@ struct lexb_gpu {
     } host;
 };
 
+// (`device`: buffers and pipelines may be freed after their handle was closed, which must not be read then)
 struct lexb_buffer {
     lexb_gpu* gpu;
     void* ptr;
     size_t bytes;
     bool owned;
+    int device = 0;
 };
 
 // How the matvec's launch is laid out (plan_matvec).
@@ -169,6 +172,7 @@ struct MatvecShape {
 
 struct lexb_pipeline {
     lexb_gpu* gpu;
+    int device = 0;
     uint32_t kernel;
     uint32_t m, n, k;
     bool residual;
@@ -219,6 +223,16 @@ int use(lexb_gpu* g) {
     if (!g) return fail(LEXB_ERR_ARG, "null gpu handle");
     CUDA_TRY(cudaSetDevice(g->device));
     return LEXB_OK;
+}
+
+// Device memory of a buffer or a pipeline.  A failure is this call's: it does not stay behind as the next launch's error.
+cudaError_t free_on(int device, std::initializer_list<void*> memory) {
+    cudaError_t e = cudaSetDevice(device);
+    if (e == cudaSuccess)
+        for (void* p : memory)
+            if (cudaError_t f = cudaFree(p)) e = f;
+    if (e != cudaSuccess) cudaGetLastError();
+    return e;
 }
 
 int check_buf(const lexb_buffer* b, const lexb_gpu* g, size_t need, const char* what) {
@@ -1379,7 +1393,7 @@ int lexb_alloc(lexb_gpu* g, size_t bytes, lexb_buffer** out) {
     *out = nullptr;
     void* p = nullptr;
     CUDA_TRY(x_malloc(&p, bytes ? bytes : 1));
-    lexb_buffer* b = new (std::nothrow) lexb_buffer{g, p, bytes, true};
+    lexb_buffer* b = new (std::nothrow) lexb_buffer{g, p, bytes, true, g->device};
     if (!b) {
         cudaFree(p);
         return fail(LEXB_ERR_ARG, "out of host memory");
@@ -1406,7 +1420,7 @@ int lexb_zeroed(lexb_gpu* g, size_t bytes, lexb_buffer** out) {
 int lexb_wrap(lexb_gpu* g, void* device_ptr, size_t bytes, lexb_buffer** out) {
     if (!g || !out) return fail(LEXB_ERR_ARG, "lexb_wrap: null argument");
     if (!device_ptr && bytes) return fail(LEXB_ERR_ARG, "lexb_wrap: null device pointer");
-    lexb_buffer* b = new (std::nothrow) lexb_buffer{g, device_ptr, bytes, false};
+    lexb_buffer* b = new (std::nothrow) lexb_buffer{g, device_ptr, bytes, false, g->device};
     if (!b) return fail(LEXB_ERR_ARG, "out of host memory");
     *out = b;
     return LEXB_OK;
@@ -1416,8 +1430,7 @@ int lexb_free(lexb_buffer* b) {
     if (!b) return LEXB_OK;
     int rc = LEXB_OK;
     if (b->owned && b->ptr) {
-        cudaSetDevice(b->gpu->device);
-        cudaError_t e = cudaFree(b->ptr);
+        const cudaError_t e = free_on(b->device, {b->ptr});
         if (e != cudaSuccess) rc = fail(LEXB_ERR_CUDA, "cudaFree: %s", cudaGetErrorString(e));
     }
     delete b;
@@ -1498,6 +1511,7 @@ int lexb_gemm_fp4_plan(lexb_gpu* g, uint32_t m, uint32_t n, uint32_t k, int resi
     lexb_pipeline* p = new (std::nothrow) lexb_pipeline();
     if (!p) return fail(LEXB_ERR_ARG, "out of host memory");
     p->gpu = g;
+    p->device = g->device;
     p->kernel = kernel;
     p->m = m; p->n = n; p->k = k;
     p->residual = residual != 0;
@@ -1796,11 +1810,7 @@ void lexb_pipeline_free(lexb_pipeline* p) {
     if (!p) return;
     for (lexb_pipeline* part : p->host_pipes) lexb_pipeline_free(part);
     delete p->few;
-    if (p->partial || p->pre_buf) {
-        cudaSetDevice(p->gpu->device);
-        if (!p->partial_borrowed) cudaFree(p->partial);
-        cudaFree(p->pre_buf);
-    }
+    if (p->partial || p->pre_buf) free_on(p->device, {p->partial_borrowed ? nullptr : p->partial, p->pre_buf});
     delete p;
 }
 

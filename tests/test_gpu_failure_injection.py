@@ -204,3 +204,26 @@ def test_disarming_and_argument_checks(gpu):
     with pytest.raises(L.LexbError):
         D.debug_fail_next(9)
     parity_still_holds(gpu, seed=4)
+
+
+def test_what_a_handle_made_may_outlive_it(gpu):
+    """Pipelines and buffers freed after their handle was closed read nothing of it and leave no error behind for the next launch: the
+    closed handle's memory is handed out again and overwritten first."""
+    import ctypes
+    libc = ctypes.CDLL(None)
+    libc.malloc.restype, libc.malloc.argtypes, libc.free.argtypes = ctypes.c_void_p, [ctypes.c_size_t], [ctypes.c_void_p]
+    before = free_bytes()
+    other = L.Gpu(0)
+    made = [other.plan_gemm_fp4(512, 5120, 17408), other.plan_matmul_fp4(8, 1024, 4096), other.plan_gemm_fp4(32, 4096, 4096),
+            other.alloc(1 << 20), other.zeroed(4096)]
+    other.close()
+    blocks = [libc.malloc(size) for size in range(512, 8192, 16) for _ in range(2)]
+    for block, size in zip(blocks, (size for size in range(512, 8192, 16) for _ in range(2))):
+        ctypes.memset(block, 0x7F, size)
+    for thing in made:
+        thing.close()
+    for block in blocks:
+        libc.free(block)
+    parity_still_holds(gpu, m=4, n=256, k=512)
+    parity_still_holds(gpu)
+    assert free_bytes() >= before - (4 << 20)                    # (the workspaces and the buffers are back)
