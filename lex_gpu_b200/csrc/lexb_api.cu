@@ -961,6 +961,74 @@ bool chain_pre(const lexb_step* steps, size_t count) {
     return false;
 }
 
+// Stages per part of K of a step in a run.
+uint32_t chain_part(const lexb_pipeline* p) { return p->k_splits == 1u ? p->k / lexb::MQ_STAGE_K : p->kb_per_split; }
+
+// Of the first `len` steps of a list, which one launch can take: how many it should.  Steps whose plans keep K whole always share it.
+// The parts of a split K stay in one block of a run, where the step's own launch spreads them: two steps of 640 x 17408 are 10 blocks
+// of 68 stages there and 40 blocks of 9 alone (48 us and 30), three 27B layers 106 us and 160.  So a run with split plans is priced
+// against its steps' own launches, with the number of steps with which it and what is left cost least.  Fitted to 150 lists timed both ways (2-6
+// steps, t = 1-8, n = 128-20480, k = 512-17408; median error 3 % and 6 %), us: a run 12.4 and 0.546 per stage of its fullest block; a
+// list 5.2, a step of it 3.2, 0.536 per stage of each wave of blocks, 1.2 for a split, the walk over the tokens for their digits, in
+// front of the product past 4 tokens.  A run is given up where it costs a tenth more.  On 100 other lists the way taken takes 0.997 of
+// the faster of the two whole ways in the mean and 1.06 at most; every run taken, 1.02 and 1.9.  LEXB_CHAIN_SPLITS=1: it is taken
+// whatever it costs.
+size_t run_that_pays(const lexb_step* steps, size_t len, uint32_t sms) {
+    size_t unsplit = 0;
+    while (unsplit < len && steps[unsplit].pipeline->k_splits == 1u) unsplit++;
+    if (unsplit == len || env_u32("LEXB_CHAIN_SPLITS", 0) != 0u) return len;
+    using Tiles = std::vector<std::pair<uint32_t, uint32_t>>;    // (stages of a row tile, tiles), longest first
+    auto add = [](Tiles& tiles, uint32_t stages, uint32_t count) {
+        auto at = std::find_if(tiles.begin(), tiles.end(), [&](const auto& e) { return e.first <= stages; });
+        if (at != tiles.end() && at->first == stages) at->second += count;
+        else tiles.insert(at, {stages, count});
+    };
+    auto fullest = [&](const Tiles& tiles) {                     // stages of the fullest block, dealt out as well as can be
+        uint64_t total = 0, count = 0, most = 0;
+        for (const auto& e : tiles) count += e.second;
+        const uint64_t blocks = std::min<uint64_t>(count, sms);
+        count = 0;
+        for (const auto& e : tiles) {
+            count += e.second;
+            total += static_cast<uint64_t>(e.first) * e.second;
+            most = std::max(most, (count + blocks - 1u) / blocks * e.first);
+        }
+        return static_cast<double>(std::max(most, (total + blocks - 1u) / blocks));
+    };
+    constexpr double RUN = 12.4, RUN_STAGE = 0.546, LIST = 5.18, STEP = 3.17, STEP_STAGE = 0.536, STEP_SPLIT = 1.19, STEP_PIECES = 3.39, WALK = 0.0132;
+    // us of steps i, i + 1, ... in launches of their own, those that keep K whole as one run if that is less
+    std::vector<double> apart(len + 1u, 0.0);
+    Tiles tiles;
+    double split_alone = 0.0, whole_alone = 0.0;
+    for (size_t i = len, whole_steps = 0; i-- > 0;) {
+        const lexb_pipeline* p = steps[i].pipeline;
+        const uint32_t rows = p->n / lexb::MQ_ROWS, kb = p->k / lexb::MQ_STAGE_K, waves = (rows * p->k_splits + sms - 1u) / sms;
+        const double us = STEP + STEP_STAGE * waves * chain_part(p) + (p->m > 4u ? STEP_PIECES + WALK * kb : WALK * p->m * kb);
+        if (p->k_splits == 1u) {
+            add(tiles, kb, rows);
+            whole_alone += us;
+            whole_steps++;
+        } else {
+            split_alone += us + STEP_SPLIT;
+        }
+        apart[i] = split_alone + (whole_steps > 1u ? std::min(whole_alone, RUN - LIST + RUN_STAGE * fullest(tiles)) : whole_alone);
+    }
+    tiles.clear();
+    double without = LIST + apart[0], with = 1e30;
+    size_t best = 0;
+    for (size_t i = 0; i < len; i++) {
+        add(tiles, steps[i].pipeline->k / lexb::MQ_STAGE_K, steps[i].pipeline->n / lexb::MQ_ROWS);
+        if (i == 0 || i + 1u < unsplit) continue;
+        const double us = RUN + RUN_STAGE * fullest(tiles) + apart[i + 1u];
+        if (i + 1u == unsplit) without = us;
+        else if (us <= with) {
+            with = us;
+            best = i + 1u;
+        }
+    }
+    return with <= 1.1 * without ? best : unsplit >= 2u ? unsplit : 0u;
+}
+
 // Length of the run of steps starting at i that one persistent kernel can take (0: step i is launched on its own).
 // The run's copy warp starts on the weights at once, so every member's weights must be declared constant or be
 // untouched by the steps of this call so far (`proof`) and by the run's own members.
@@ -994,16 +1062,14 @@ size_t chain_run(const lexb_gpu* g, const lexb_step* steps, size_t nsteps, size_
         in_run.push_back(c);
         len++;
     }
-    if (len >= 2) return len;
+    if (len >= 2) len = run_that_pays(steps + i, len, static_cast<uint32_t>(g->prop.multiProcessorCount));
+    if (len != 1) return len;
     // a single step with more row tiles than SMs: the persistent kernel takes them without a second wave of
     // block set-ups (n = 28672: 224 tiles)
     static const bool single = env_u32("LEXB_CHAIN_SINGLE", 1) != 0;
     const uint32_t tiles = (steps[i].pipeline->n + lexb::MQ_ROWS - 1u) / lexb::MQ_ROWS;
     return single && steps[i].pipeline->k_splits == 1u && tiles > static_cast<uint32_t>(g->prop.multiProcessorCount) ? 1 : 0;
 }
-
-// Stages per part of K of a step in a run.
-uint32_t chain_part(const lexb_pipeline* p) { return p->k_splits == 1u ? p->k / lexb::MQ_STAGE_K : p->kb_per_split; }
 
 // The table of a run's row tiles: block b works through entries b, b + grid, ...; a row of entries without a job ends it.  Tiles go
 // to the block with the fewest stages so far, the longest tiles first, so that steps of several K end together.

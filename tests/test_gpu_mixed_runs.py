@@ -16,6 +16,12 @@ def gpu():
     g.close()
 
 
+@pytest.fixture(autouse=True)
+def every_run_is_taken(monkeypatch):
+    """These lists are too narrow to pay as a run where plans split K; what a run computes is tested here, not when one is chosen."""
+    monkeypatch.setenv("LEXB_CHAIN_SPLITS", "1")
+
+
 @pytest.mark.parametrize("m,xf32", [(1, False), (2, True), (4, False), (5, True), (8, False)])
 def test_steps_of_several_k_share_a_launch(gpu, m, xf32):
     """K of 2 to 68 stages (groups of scale bytes that end inside), plans with 1, 2 and 8 parts of K, more tiles than SMs, a
@@ -213,4 +219,35 @@ def test_lists_of_growing_activations_on_two_streams(gpu):
                     assert scale > 1e-3 and err <= 1e-4
     finally:
         gpu.set_stream(None)
+    assert gpu.status_word() == 0
+
+
+@pytest.mark.parametrize("t,shapes,runs", [
+    (4, [(640, 17408)] * 2, [1, 1]),                                               # 10 blocks of 68 stages against 40 of 9
+    (1, [(512, 12800), (8704, 2816)], [1, 1]),
+    (1, [(19456, 2816), (19456, 2816), (640, 17408)], [2, 2, 1]),                  # the pair goes without the long narrow one
+    (1, [(640, 17408), (19456, 2816), (19456, 2816)], [1, 2, 2]),
+    (2, [(1024, 4096)] * 5 + [(256, 17408)], [5] * 5 + [1]),
+    (4, [(1024, 4096)] * 4, [4] * 4),
+    (4, [(17408, 5120), (17408, 5120), (5120, 17408)] * 3, [9] * 9)])
+def test_a_run_of_split_plans_is_taken_where_it_pays(gpu, monkeypatch, t, shapes, runs):
+    """... and the results are those of the steps' own launches either way."""
+    monkeypatch.delenv("LEXB_CHAIN_SPLITS")
+    gen = np.random.Generator(np.random.PCG64(660))
+    weights = {}
+    for n, k in set(shapes):
+        weights[n, k] = L.QBuf(gpu, gen.integers(0, 256, (n, k // 2), dtype=np.uint8), gen.integers(0x30, 0x48, (n, k // 16), dtype=np.uint8),
+                               np.ones(n, np.float32))
+    xb = {k: gpu.upload(inputs.make_x(t, k, seed_base=662)) for _, k in set(shapes)}
+    ys = [gpu.alloc(4 * t * n) for n, _ in shapes]
+    steps = [(gpu.plan_matmul_fp4(t, n, k), weights[n, k].bind(xb[k], None, y)) for (n, k), y in zip(shapes, ys)]
+    assert gpu.list_runs(steps) == runs
+    for pipe, bind in steps:
+        gpu.run(pipe, bind)
+    gpu.sync()
+    alone = [gpu.download(y, np.float32, (t, n)) for y, (n, _) in zip(ys, shapes)]
+    for y in ys:
+        gpu.memset(y, 0xEE)
+    gpu.run_launches(steps)
+    assert all(np.array_equal(gpu.download(y, np.float32, a.shape), a) for y, a in zip(ys, alone))
     assert gpu.status_word() == 0
