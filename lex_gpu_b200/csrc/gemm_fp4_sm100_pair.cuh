@@ -75,7 +75,14 @@ __host__ __device__ constexpr uint32_t pair_smem_bytes(uint32_t tok_blocks, uint
            (2u * sx + 3u * sw + 1u + 2u * sr) * 8u + 16u + 1024u;
 }
 
-template <bool TRACE>
+// PAIRED: ring stages of a whole block of packed weights, decoded two K steps a turn, even and odd blocks by two sets of eight warps
+// (see the decode).  A set passes over every second packed block: at the block before, two ago, it has seen the MMAs of the one SW
+// before that complete, so its parity waits are right if the ring of packed blocks has at least SW + 2.
+__host__ __device__ constexpr bool pair_paired(uint32_t k_sub, bool w_in_tmem, uint32_t sw, uint32_t sr) { return k_sub == 4u && w_in_tmem && sr >= sw + 2u; }
+
+// PAIRED and CLUSTER (K split within a cluster: below) are instances of their own: as branches of one kernel their code cost the tiles
+// that take neither 1 % (201 x 6144 x 4096 in 3 parts: 18.28 us, 18.12 with instances).
+template <bool TRACE, bool PAIRED, bool CLUSTER>
 __global__ void __launch_bounds__(PAIR_THREADS, 1)
 gemm_fp4_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_wq,
                              const __grid_constant__ CUtensorMap tmap_ws, const GemmArgs a) {
@@ -107,11 +114,7 @@ gemm_fp4_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const _
     // ring every fourth K step (every 4 / KS stage steps), and a parity wait is only right if the barrier cannot be
     // two phases behind the one awaited: the group's previous wait (step j - 4 / KS) guarantees phase (j - DN) only
     // if DN >= 4 / KS.
-    // `paired`: stages of a whole block are decoded two K steps a turn, even and odd blocks by two sets of eight warps (see the
-    // decode).  A set passes over every second packed block: at the block before, two ago, it has seen the MMAs of the one SW
-    // before that complete, so its parity waits are right if the ring of packed blocks has at least SW + 2.
-    const bool paired = KS == 4u && w_tmem && SR >= SW + 2u;
-    const uint32_t stage_warps = paired ? PAIR_DEQ_THREADS / 64u : KS * (PAIR_DEQ_THREADS / 128u);      // decode warps that fill a stage
+    const uint32_t stage_warps = PAIRED ? PAIR_DEQ_THREADS / 64u : KS * (PAIR_DEQ_THREADS / 128u);      // decode warps that fill a stage
     const uint32_t DN = (SX > SW ? SX : SW) > 4u ? (SX > SW ? SX : SW) : 4u;
     auto full = [&](uint32_t j) { return bars + 8u * j; };                        // leader only: all inputs of K step j
     auto done = [&](uint32_t j) { return bars + 8u * (DN + j); };                 // both CTAs: K step j's MMAs complete
@@ -125,7 +128,7 @@ gemm_fp4_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const _
 
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
     // A cluster is one pair, or - K split within it - the pairs of all parts of K of one tile.  Rank in the pair: 0 = leader.
-    const uint32_t cluster_rank = cluster_ctarank(), rank = cluster_rank & 1u, leader = cluster_rank & ~1u;
+    const uint32_t cluster_rank = cluster_ctarank(), rank = CLUSTER ? cluster_rank & 1u : cluster_rank, leader = CLUSTER ? cluster_rank & ~1u : 0u;
     const uint32_t pair = blockIdx.x >> 1;
     const uint32_t split = pair % a.k_splits, tile = pair / a.k_splits;
     const uint32_t m_tile = tile % a.m_tiles, n_pair = tile / a.m_tiles;
@@ -149,7 +152,7 @@ gemm_fp4_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const _
         for (uint32_t s = 0; s < SW; s++) mbar_init(w_part(s), stage_warps);
         for (uint32_t rs = 0; rs < SR; rs++) {
             mbar_init(raw_full(rs), 1);
-            mbar_init(raw_empty(rs), paired ? stage_warps : PAIR_DEQ_THREADS / 32u);
+            mbar_init(raw_empty(rs), PAIRED ? stage_warps : PAIR_DEQ_THREADS / 32u);
         }
         mbar_init(acc_full, 1);
         fence_mbar_init();
@@ -177,7 +180,6 @@ gemm_fp4_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const _
     // each joins the stream's order before its first wait on a ring slot (a bounded wait must not run
     // against another launch's time) and, for the decode warps, before the epilogue.
     const bool early_w = (a.flags & 2u) != 0u;
-    const bool in_cluster = (a.flags & 8u) != 0u;            // the parts of K are summed within the cluster (below)
     bool acc_ok = false;                                     // (decode warps) the accumulator is complete
 
     const bool weight_role = warp == PAIR_WARP_RAW || warp < PAIR_DEQ_THREADS / 32u;
@@ -373,7 +375,7 @@ gemm_fp4_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const _
         const uint32_t hop = 4u / KS;                                // stage steps between this group's K steps
         const uint32_t sub_col = (q % KS) * 32u;                     // this group's K step within a two-step stage
         bool joined = !early_w, pe_set = false;
-        if (paired) {
+        if (PAIRED) {
             // A warp has 32 rows and two of the four K steps of every second block: its waits, fences and arrivals, as long as the
             // decode of a K step even where nothing is waited for, come once per two K steps (17408 x 5120 in tiles of 128 tokens:
             // 27.1 -> 23.3 us).
@@ -436,7 +438,7 @@ gemm_fp4_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const _
                 if (lane == 0) mbar_arrive(rank == 0u ? full(pf.s) : w_part(pw.s));
             }
         }
-        for (uint32_t kb = paired ? KB : q; kb < KB; kb += 4u, pr.advance(SR), pw.advance_by(hop, SW), pf.advance_by(hop, DN)) {
+        for (uint32_t kb = PAIRED ? KB : q; kb < KB; kb += 4u, pr.advance(SR), pw.advance_by(hop, SW), pf.advance_by(hop, DN)) {
             const uint32_t rs = pr.s, rph = pr.ph;
             long long tq0 = 0;
             if (TRACE) tq0 = clock64();
@@ -527,7 +529,7 @@ gemm_fp4_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const _
             if (rank != 0u) a.trace[16ull * blockIdx.x + 11] = gt_start;
             a.trace[16ull * blockIdx.x + 6] = (unsigned long long)clock64();   // accumulator complete
         }
-        if (go && n0 < a.n && !in_cluster) {
+        if (!CLUSTER && go && n0 < a.n) {
             tc_fence_after_sync();
             const uint32_t quarter = warp & 3u, slice = warp >> 2;      // 4 lane quarters x 4 column slices
             const bool to_partial = a.k_splits > 1u;
@@ -619,7 +621,7 @@ gemm_fp4_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const _
         }
     }
 
-    if (in_cluster) {
+    if (CLUSTER) {
         // K split within the cluster (tiles of up to 256 tokens): every block leaves its sums in shared memory (the rings are idle:
         // its accumulator is complete) as [token][128 rows]; then the blocks that hold the same rows share out the tokens, and add
         // the parts, from one another's shared memory, in the order of the parts - the sums of splitk_reduce_kernel, bit for

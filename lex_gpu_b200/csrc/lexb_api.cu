@@ -445,6 +445,13 @@ struct Order {
     bool early(const lexb_pipeline* p) const { return !in_order && (p->w_const || (early_weights && !p->w_volatile)); }
 };
 
+using PairKernel = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const lexb::GemmArgs);
+template <bool TRACE>
+PairKernel pair_kernel(bool paired, bool cluster) {
+    return paired ? (cluster ? lexb::gemm_fp4_tcgen05_pair_kernel<TRACE, true, true> : lexb::gemm_fp4_tcgen05_pair_kernel<TRACE, true, false>)
+                  : (cluster ? lexb::gemm_fp4_tcgen05_pair_kernel<TRACE, false, true> : lexb::gemm_fp4_tcgen05_pair_kernel<TRACE, false, false>);
+}
+
 using FewKernel = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const lexb::FewArgs);
 FewKernel few_kernel(uint32_t m) {
     const uint32_t cols = lexb::few_cols(m);
@@ -716,7 +723,6 @@ int launch_one(lexb_gpu* g, const lexb_pipeline* p, const lexb_buffer* x, const 
             cfg.dynamicSmemBytes = p->smem;
             cfg.stream = g->stream;
             const bool in_cluster = p->cluster_split && !gather;
-            if (in_cluster) a.flags |= 8u;
             cudaLaunchAttribute attr[2];
             attr[0].id = cudaLaunchAttributeClusterDimension;
             attr[0].val.clusterDim.x = in_cluster ? 2u * p->k_splits : 2u;
@@ -726,10 +732,9 @@ int launch_one(lexb_gpu* g, const lexb_pipeline* p, const lexb_buffer* x, const 
             attr[1].val.programmaticStreamSerializationAllowed = 1;
             cfg.attrs = attr;
             cfg.numAttrs = pdl ? 2 : 1;
-            if (a.trace)
-                LAUNCH_TRY(cudaLaunchKernelEx(&cfg, lexb::gemm_fp4_tcgen05_pair_kernel<true>, maps.map, maps.map_wq, maps.map_ws, a));
-            else
-                LAUNCH_TRY(cudaLaunchKernelEx(&cfg, lexb::gemm_fp4_tcgen05_pair_kernel<false>, maps.map, maps.map_wq, maps.map_ws, a));
+            const bool paired = lexb::pair_paired(p->k_sub, (p->flags & 4u) != 0u, p->w_stages, p->raw_stages);
+            const PairKernel kernel = a.trace ? pair_kernel<true>(paired, in_cluster) : pair_kernel<false>(paired, in_cluster);
+            LAUNCH_TRY(cudaLaunchKernelEx(&cfg, kernel, maps.map, maps.map_wq, maps.map_ws, a));
             if (p->k_splits > 1 && !in_cluster) {
                 CUDA_TRY(cudaGetLastError());
                 const size_t elems = static_cast<size_t>(p->m) * p->n;       // n % 128 == 0: a multiple of 4
@@ -1371,8 +1376,14 @@ int lexb_open(int device, lexb_gpu** out) {
     g->encode_tiled = reinterpret_cast<EncodeTiledFn>(fn);
     const int max_smem = static_cast<int>(g->smem_optin);
     if (cudaFuncSetAttribute(lexb::gemm_fp4_tcgen05_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem) != cudaSuccess ||
-        cudaFuncSetAttribute(lexb::gemm_fp4_tcgen05_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem) != cudaSuccess ||
-        cudaFuncSetAttribute(lexb::gemm_fp4_tcgen05_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem) != cudaSuccess ||
+        cudaFuncSetAttribute(pair_kernel<true>(true, true), cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem) != cudaSuccess ||
+        cudaFuncSetAttribute(pair_kernel<true>(true, false), cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem) != cudaSuccess ||
+        cudaFuncSetAttribute(pair_kernel<true>(false, true), cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem) != cudaSuccess ||
+        cudaFuncSetAttribute(pair_kernel<true>(false, false), cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem) != cudaSuccess ||
+        cudaFuncSetAttribute(pair_kernel<false>(true, true), cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem) != cudaSuccess ||
+        cudaFuncSetAttribute(pair_kernel<false>(true, false), cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem) != cudaSuccess ||
+        cudaFuncSetAttribute(pair_kernel<false>(false, true), cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem) != cudaSuccess ||
+        cudaFuncSetAttribute(pair_kernel<false>(false, false), cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem) != cudaSuccess ||
         cudaFuncSetAttribute(lexb::gemm_fp4_few_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem) != cudaSuccess ||
         cudaFuncSetAttribute(lexb::gemm_fp4_few_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem) != cudaSuccess ||
         cudaFuncSetAttribute(lexb::gemm_fp4_few_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem) != cudaSuccess ||
@@ -1743,7 +1754,7 @@ int lexb_gemm_fp4_plan(lexb_gpu* g, uint32_t m, uint32_t n, uint32_t k, int resi
         }
         p->x_rows = p->tm == 512u ? lexb::PAIR_XBLK_ROWS : p->tm / 2u;
         // packed-weight blocks in flight: 2; 5 with tiles of 128 tokens or fewer, whose decode takes every second block (two more
-        // than the W ring's 3 stages: see the kernel's `paired`), or 3 beside ring depths that the caller gives
+        // than the W ring's 3 stages: pair_paired), or 3 beside ring depths that the caller gives
         const uint32_t raw_stages = env_u32("LEXB_RAWSTAGES", p->tm > 128u ? lexb::PAIR_RAW_STAGES : s.stages || s.w_stages ? 3u : 5u);
         p->raw_stages = raw_stages;
         if (splits < 1u || splits > raw_blocks) return bail(fail(LEXB_ERR_ARG, "k_splits = %u outside [1, %u]", splits, raw_blocks));
@@ -2391,7 +2402,7 @@ int lexb_gemm_fp4_splitk_static(lexb_gpu* g, uint32_t m, uint32_t n, uint32_t k,
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    CUDA_TRY(cudaLaunchKernelEx(&cfg, lexb::gemm_fp4_tcgen05_pair_kernel<false>, map_x, map_wq, map_ws, a));
+    CUDA_TRY(cudaLaunchKernelEx(&cfg, pair_kernel<false>(false, false), map_x, map_wq, map_ws, a));
     CUDA_TRY(cudaGetLastError());
     const size_t elems = mm * nn;
     const uint32_t blocks = static_cast<uint32_t>(std::min<size_t>((elems / 4 + 255) / 256, static_cast<size_t>(g->prop.multiProcessorCount) * 8u));
