@@ -70,14 +70,14 @@ typedef struct lexb_sched {
 } lexb_sched;
 /* Block-scaled kernel and two-CTA GEMM.  Launches are in order on their stream, as the reference's are
  * (crates/lex-cuda/src/device.rs:629-672): every read waits for the kernel ahead.  The kernel can do
- * better when it knows that nothing in flight writes wq and ws - launched with programmatic stream
+ * better when it knows that nothing in flight writes wq, ws and wg - launched with programmatic stream
  * serialization, it then starts loading them while the kernel ahead of it is still running (x, r and y
  * wait as usual).  It knows in two ways:
  *   - inside one lexb_run_launches / lexb_time_launches call the library proves it from the step list (the
- *     call's first launch waits for all earlier work of the stream; a later step whose wq/ws meet no y of an
+ *     call's first launch waits for all earlier work of the stream; a later step whose wq/ws/wg meet no y of an
  *     earlier step of the call loads them early).  LEXB_SCHED_WEIGHTS_MAY_CHANGE turns that off for a pipeline
  *     whose weights something outside the list (another stream) rewrites;
- *   - LEXB_SCHED_WEIGHTS_CONSTANT is the caller's promise that nothing writes wq/ws while launches of
+ *   - LEXB_SCHED_WEIGHTS_CONSTANT is the caller's promise that nothing writes wq, ws and wg while launches of
  *     this pipeline are in flight, for launches made one at a time (lexb_gemm_fp4_launch). */
 #define LEXB_SCHED_WEIGHTS_MAY_CHANGE 1u
 #define LEXB_SCHED_WEIGHTS_CONSTANT 2u
@@ -226,7 +226,7 @@ LEXB_API int lexb_gemm_fp4_enqueue_host(lexb_gpu* gpu, const lexb_pipeline* p, c
  * The results are those of the steps run one after another.  Consecutive lexb_matmul_fp4_plan steps of t <= 8
  * tokens planned with k_splits = 1 (and without LEXB_SCHED_WEIGHTS_MAY_CHANGE), with the same t, k
  * and activation type, of which none reads or overwrites a buffer that an earlier one of them touches (x, r,
- * wq and ws not written, y neither read nor written: the address ranges are compared; wq and ws must also be
+ * wq, ws and wg not written, y neither read nor written: the address ranges are compared; wq, ws and wg must also be
  * untouched by every earlier step of the call, or declared constant), are run as ONE persistent kernel
  * over all their row tiles (the gate/up pair, q/k/v); each result is bit-identical to the step launched alone.
  * A step that depends on the run starts a new launch.  The environment variable LEXB_CHAIN=0 turns this off. */

@@ -905,7 +905,7 @@ static uint32_t chain_pre_min_m() {
 struct Range { const char *lo, *hi; };
 inline bool meet(Range a, Range b) { return a.lo < b.hi && b.lo < a.hi; }
 struct StepRanges {
-    Range x{}, wq{}, ws{}, r{}, y{};
+    Range x{}, wq{}, ws{}, wg{}, r{}, y{};
     bool valid = false;          // false: a null pipeline, buffer list or buffer (the step's own launch reports it)
 };
 
@@ -921,6 +921,7 @@ StepRanges step_ranges(const lexb_step& s) {
     out.x = range(s.buffers[0], m * k * (p->x_f32 ? 4 : 2));
     out.wq = range(s.buffers[1 + q], n * k / 2);
     out.ws = range(s.buffers[2 + q], n * k / 16);
+    out.wg = range(s.buffers[3 + q], n * 4);
     out.r = p->residual ? range(s.buffers[4 + q], out_bytes) : Range{nullptr, nullptr};
     out.y = range(s.buffers[(p->residual ? 5 : 4) + q], out_bytes);
     out.valid = true;
@@ -936,7 +937,7 @@ struct ListProof {
     std::vector<Range> written;      // distinct y ranges
     bool weights_untouched(const StepRanges& s) const {
         for (const Range& w : written)
-            if (meet(s.wq, w) || meet(s.ws, w)) return false;
+            if (meet(s.wq, w) || meet(s.ws, w) || meet(s.wg, w)) return false;
         return true;
     }
     void add(const StepRanges& s) {
@@ -1051,7 +1052,7 @@ size_t chain_run(const lexb_gpu* g, const lexb_step* steps, size_t nsteps, size_
         if (!declared_const && !proof.weights_untouched(c)) return true;
         for (const StepRanges& e : in_run) {
             if (meet(c.x, e.y) || meet(c.r, e.y) || meet(c.y, e.x) || meet(c.y, e.r) || meet(c.y, e.y)) return true;
-            if (meet(c.wq, e.y) || meet(c.ws, e.y) || meet(c.y, e.wq) || meet(c.y, e.ws)) return true;
+            if (meet(c.wq, e.y) || meet(c.ws, e.y) || meet(c.wg, e.y) || meet(c.y, e.wq) || meet(c.y, e.ws) || meet(c.y, e.wg)) return true;
         }
         return false;
     };

@@ -622,3 +622,41 @@ def test_a_list_of_one_step_waits_for_the_work_ahead_of_it(gpu, kind):
         gpu.run_launches(steps)
         assert np.array_equal(gpu.download(y, np.float32, (m, n)), want, equal_nan=True)
     assert gpu.status_word() == 0
+
+
+def test_row_scales_written_by_an_earlier_step(gpu):
+    """A step whose wg an earlier step of the list writes as its y, and one that overwrites an earlier step's wg: neither shares a
+    launch with that step or is decoded ahead of it."""
+    n, k = 256, 512
+    x, wq, ws, wg = inputs.make_case(1, n, k, seed_base=90)
+    wq2, ws2, _ = inputs.make_weights(n, k, seed_base=91)
+    q, xb, ya, yb = L.QBuf(gpu, wq, ws, wg), gpu.upload(x), gpu.alloc(4 * n), gpu.alloc(4 * n)
+    wq2b, ws2b = gpu.upload(wq2), gpu.upload(ws2)
+    pipe = gpu.plan_matmul_fp4(1, n, k, k_splits=1)
+    first, scaled = (pipe, q.bind(xb, None, ya)), (pipe, [xb, wq2b, ws2b, ya, yb])
+    other = (pipe, q.bind(xb, None, yb))
+    assert gpu.list_runs([first, other]) == [2, 2]
+    assert gpu.list_runs([first, scaled]) == [1, 1]
+    assert gpu.list_runs([scaled, first]) == [1, 1]
+    a = O.matmul_q_x(x, wq, ws, wg)
+    for _ in range(3):
+        gpu.memset(ya, 0)
+        gpu.run_launches([first, scaled])
+        got = gpu.download(yb, np.float32, (1, n))
+        err, scale, _ = O.err_of_scale(got, O.matmul_q_x(x, wq2, ws2, gpu.download(ya, np.float32, (n,))))
+        assert scale > 1e-3 and err <= 1e-4 and np.abs(gpu.download(ya, np.float32, (1, n)) - a).max() <= 1e-4 * np.abs(a).max()
+    # gemm_fp4: the few-token kernel and the two-CTA GEMM decode ahead of the stream's order, with wg
+    m, n, k = 32, 1024, 2048
+    x, wq, ws, wg = inputs.make_case(m, n, k, seed_base=92)
+    xb, wqb, wsb, wgb, y = gpu.upload(x), gpu.upload(wq), gpu.upload(ws), gpu.upload(wg), gpu.alloc(4 * m * n)
+    first_x, first_w = inputs.make_x(1, 512, seed_base=93), inputs.make_weights(n, 512, seed_base=93)
+    fresh = O.matmul_q_x(first_x, *first_w)[0]
+    first = (gpu.plan_matmul_fp4(1, n, 512), L.QBuf(gpu, *first_w).bind(gpu.upload(first_x), None, wgb))
+    for pipe in (gpu.plan_gemm_fp4(m, n, k), gpu.plan_gemm_fp4(m, n, k, kernel=3)):
+        gpu.memset(wgb, 0)
+        gpu.run_launches([(gpu.plan_matmul_fp4(1, n, 512), L.QBuf(gpu, *first_w).bind(gpu.upload(first_x), None, gpu.alloc(4 * n))),
+                          first, (pipe, [xb, wqb, wsb, wgb, y])])
+        err, scale, _ = O.err_of_scale(gpu.download(y, np.float32, (m, n)), O.gemm_fp4(x, wq, ws, gpu.download(wgb, np.float32, (n,))))
+        assert scale > 1e-3 and err <= 2e-5
+        assert np.abs(gpu.download(wgb, np.float32, (n,)) - fresh).max() <= 1e-4 * np.abs(fresh).max()
+    assert gpu.status_word() == 0
