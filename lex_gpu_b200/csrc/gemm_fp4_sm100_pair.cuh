@@ -80,12 +80,11 @@ __host__ __device__ constexpr uint32_t pair_smem_bytes(uint32_t tok_blocks, uint
 // before that complete, so its parity waits are right if the ring of packed blocks has at least SW + 2.
 __host__ __device__ constexpr bool pair_paired(uint32_t k_sub, bool w_in_tmem, uint32_t sw, uint32_t sr) { return k_sub == 4u && w_in_tmem && sr >= sw + 2u; }
 
-// PAIRED and CLUSTER (K split within a cluster: below) are instances of their own: as branches of one kernel their code cost the tiles
-// that take neither 1 % (201 x 6144 x 4096 in 3 parts: 18.28 us, 18.12 with instances).
+// PAIRED and CLUSTER (K split within a cluster: below) are instances of their own, and a pair alone has its cluster's size from the
+// kernel: with branches and a size per launch the tiles that take neither cost 1 % more (201 x 6144 x 4096 in 3 parts: 18.25 us,
+// 18.12 without the branches, 18.06 with the size fixed too).
 template <bool TRACE, bool PAIRED, bool CLUSTER>
-__global__ void __launch_bounds__(PAIR_THREADS, 1)
-gemm_fp4_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_wq,
-                             const __grid_constant__ CUtensorMap tmap_ws, const GemmArgs a) {
+__device__ __forceinline__ void pair_gemm(const CUtensorMap& tmap_x, const CUtensorMap& tmap_wq, const CUtensorMap& tmap_ws, const GemmArgs& a) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw_addr = smem_u32(smem_raw);
     const uint32_t base = (raw_addr + 1023u) & ~1023u;
@@ -690,6 +689,20 @@ gemm_fp4_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const _
         tc_fence_after_sync();
         tmem_dealloc_pair(tmem_base, PAIR_TMEM_COLS);
     }
+}
+
+template <bool TRACE, bool PAIRED>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
+gemm_fp4_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_wq,
+                             const __grid_constant__ CUtensorMap tmap_ws, const __grid_constant__ GemmArgs a) {
+    pair_gemm<TRACE, PAIRED, false>(tmap_x, tmap_wq, tmap_ws, a);
+}
+// ... in clusters of a tile's pairs, as many as K has parts
+template <bool TRACE, bool PAIRED>
+__global__ void __launch_bounds__(PAIR_THREADS, 1)
+gemm_fp4_tcgen05_pair_split_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_wq,
+                                   const __grid_constant__ CUtensorMap tmap_ws, const __grid_constant__ GemmArgs a) {
+    pair_gemm<TRACE, PAIRED, true>(tmap_x, tmap_wq, tmap_ws, a);
 }
 
 // y = sum over splits of partial[s] (+ r), four floats per thread step; the order of the sum is fixed.

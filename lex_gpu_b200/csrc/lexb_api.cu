@@ -448,8 +448,8 @@ struct Order {
 using PairKernel = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const lexb::GemmArgs);
 template <bool TRACE>
 PairKernel pair_kernel(bool paired, bool cluster) {
-    return paired ? (cluster ? lexb::gemm_fp4_tcgen05_pair_kernel<TRACE, true, true> : lexb::gemm_fp4_tcgen05_pair_kernel<TRACE, true, false>)
-                  : (cluster ? lexb::gemm_fp4_tcgen05_pair_kernel<TRACE, false, true> : lexb::gemm_fp4_tcgen05_pair_kernel<TRACE, false, false>);
+    return paired ? (cluster ? lexb::gemm_fp4_tcgen05_pair_split_kernel<TRACE, true> : lexb::gemm_fp4_tcgen05_pair_kernel<TRACE, true>)
+                  : (cluster ? lexb::gemm_fp4_tcgen05_pair_split_kernel<TRACE, false> : lexb::gemm_fp4_tcgen05_pair_kernel<TRACE, false>);
 }
 
 using FewKernel = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const lexb::FewArgs);
@@ -724,14 +724,14 @@ int launch_one(lexb_gpu* g, const lexb_pipeline* p, const lexb_buffer* x, const 
             cfg.stream = g->stream;
             const bool in_cluster = p->cluster_split && !gather;
             cudaLaunchAttribute attr[2];
-            attr[0].id = cudaLaunchAttributeClusterDimension;
-            attr[0].val.clusterDim.x = in_cluster ? 2u * p->k_splits : 2u;
-            attr[0].val.clusterDim.y = 1;
-            attr[0].val.clusterDim.z = 1;
-            attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-            attr[1].val.programmaticStreamSerializationAllowed = 1;
-            cfg.attrs = attr;
-            cfg.numAttrs = pdl ? 2 : 1;
+            attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            attr[0].val.programmaticStreamSerializationAllowed = 1;
+            attr[1].id = cudaLaunchAttributeClusterDimension;
+            attr[1].val.clusterDim.x = 2u * p->k_splits;
+            attr[1].val.clusterDim.y = 1;
+            attr[1].val.clusterDim.z = 1;
+            cfg.attrs = pdl ? attr : attr + 1;
+            cfg.numAttrs = (pdl ? 1u : 0u) + (in_cluster ? 1u : 0u);
             const bool paired = lexb::pair_paired(p->k_sub, (p->flags & 4u) != 0u, p->w_stages, p->raw_stages);
             const PairKernel kernel = a.trace ? pair_kernel<true>(paired, in_cluster) : pair_kernel<false>(paired, in_cluster);
             LAUNCH_TRY(cudaLaunchKernelEx(&cfg, kernel, maps.map, maps.map_wq, maps.map_ws, a));
@@ -743,7 +743,7 @@ int launch_one(lexb_gpu* g, const lexb_pipeline* p, const lexb_buffer* x, const 
                 rc_cfg.gridDim = dim3(blocks);
                 rc_cfg.blockDim = dim3(256);
                 rc_cfg.stream = g->stream;
-                rc_cfg.attrs = attr + 1;
+                rc_cfg.attrs = attr;
                 rc_cfg.numAttrs = g->pdl ? 1 : 0;
                 const auto reduce = p->k_splits == 2u ? lexb::splitk_reduce_kernel<2> : p->k_splits == 3u ? lexb::splitk_reduce_kernel<3> : p->k_splits == 4u ? lexb::splitk_reduce_kernel<4> : lexb::splitk_reduce_kernel<0>;
                 LAUNCH_TRY(cudaLaunchKernelEx(&rc_cfg, reduce, static_cast<const float*>(p->partial), p->k_splits, elems,
@@ -2391,19 +2391,7 @@ int lexb_gemm_fp4_splitk_static(lexb_gpu* g, uint32_t m, uint32_t n, uint32_t k,
     a.tmem_cols = p.tmem_cols; a.m_tiles = p.m_tiles; a.n_acc = 1;
     a.x_tx_bytes = lexb::PAIR_XBLK_BYTES;
     INJECT_LAUNCH();
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(p.grid);
-    cfg.blockDim = dim3(p.threads);
-    cfg.dynamicSmemBytes = p.smem;
-    cfg.stream = g->stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    CUDA_TRY(cudaLaunchKernelEx(&cfg, pair_kernel<false>(false, false), map_x, map_wq, map_ws, a));
+    lexb::gemm_fp4_tcgen05_pair_kernel<false, false><<<p.grid, p.threads, p.smem, g->stream>>>(map_x, map_wq, map_ws, a);
     CUDA_TRY(cudaGetLastError());
     const size_t elems = mm * nn;
     const uint32_t blocks = static_cast<uint32_t>(std::min<size_t>((elems / 4 + 255) / 256, static_cast<size_t>(g->prop.multiProcessorCount) * 8u));
