@@ -91,12 +91,15 @@ typedef struct lexb_lowered {
     uint32_t threadgroup_bytes;  /* dynamic shared memory */
     uint32_t nbind;
     uint8_t writes[8];           /* (7 bindings for lexb_matmul_int8_plan with a residual) */
-    uint32_t kernel;             /* 1 matvec, 2 tcgen05, 3 two-CTA tcgen05, 4 block-scaled FP4 */
+    uint32_t kernel;             /* 1 matvec, 2 tcgen05, 3 two-CTA tcgen05, 4 block-scaled FP4.  A plan of 9 to 64 tokens that nothing in
+                                    lexb_sched asked for is described as 3, what its gathers and traced launches run; its others run the
+                                    few-token kernel where that is the faster one (lexb_route: 736 threads a block) */
     uint32_t m, n, k, residual;
     uint32_t bm, bn, bk, stages;
-    uint32_t k_splits;           /* > 1: a second launch sums the partial products */
-    uint64_t scratch_bytes;      /* Lowered::scratch_bytes: the split-K workspace (launches that sum their parts within clusters,
-                                    and those of 9 to 64 tokens that run as one stream of weights per SM, do not use it) */
+    uint32_t k_splits;           /* > 1: the partial products are summed by a second launch, by a row tile's last block, or within
+                                    clusters (lexb_route.cluster) */
+    uint64_t scratch_bytes;      /* Lowered::scratch_bytes: the split-K workspace (the two-CTA GEMM's is there for its gathers also where
+                                    its other launches sum within clusters or run the few-token kernel) */
 } lexb_lowered;
 
 /* lex_cuda::Step, crates/lex-cuda/src/device.rs:314: a pipeline and its buffers in binding
@@ -154,11 +157,12 @@ LEXB_API int lexb_pipeline_describe(const lexb_pipeline* p, lexb_lowered* out);
 /* How a pipeline's work is laid out beyond its launch descriptor, for tests and for callers that want to see it; no
  * counterpart in the reference. */
 typedef struct lexb_route {
-    uint32_t cluster;        /* matvec: blocks that share a row block's K (1 otherwise) */
+    uint32_t cluster;        /* matvec: blocks that share a row block's K; few-token kernel: blocks that share a few row tiles; two-CTA GEMM
+                              * and block-scaled kernel: parts of K that are summed within a cluster (1 otherwise) */
     uint32_t parts;          /* matvec: parts K is summed in, a warp each */
     uint32_t groups;         /* matvec: groups of row blocks each block (cluster) works through */
     uint32_t kc;             /* matvec: K columns of x staged at a time, over the cluster's blocks; less than k: in chunks */
-    uint32_t blocks, threads;
+    uint32_t blocks, threads;  /* of a launch without a gather or phase timers */
     uint32_t host_part;      /* tokens of a part of lexb_gemm_fp4_run_host from pinned memory; 0: always whole */
 } lexb_route;
 LEXB_API int lexb_pipeline_route(const lexb_pipeline* p, lexb_route* out);
@@ -250,7 +254,7 @@ LEXB_API int lexb_status_word(lexb_gpu* gpu, uint32_t* out);
 LEXB_API int lexb_selftest_bounded_wait(lexb_gpu* gpu, uint32_t limit_us);
 #define LEXB_STATUS_WAIT_NEVER (1u << 16)
 
-/* In-kernel phase timers of the two-CTA GEMM (the counterpart of LEX_SYNC's per-call-site
+/* In-kernel phase timers of the two-CTA GEMM, which takes the few-token kernel's launches while its records fit (the counterpart of LEX_SYNC's per-call-site
  * attribution, crates/lex-rt/src/qwen_run.rs:2926-2960, one level down): with tracing enabled
  * for up to max_ctas blocks, each block of the next launch records 16 SM-clock values:
  * [0] start, [1] first K step ready, [2] all MMAs issued, [3] cycles the MMA warp waited for the

@@ -383,12 +383,15 @@ __device__ __forceinline__ void pair_gemm(const CUtensorMap& tmap_x, const CUten
             pw.seek(set, SW);
             pf.seek(set, DN);
             for (uint32_t st = set; st < stages && ok; st += 2u, pr.advance_by(2u, SR), pw.advance_by(2u, SW), pf.advance_by(2u, DN)) {
+                long long tq = 0;
+                if (TRACE) tq = clock64();
                 if (!__all_sync(0xFFFFFFFFu, mbar_wait(raw_full(pr.s), pr.ph, abort_flag))) {
                     atomicOr(a.status, ST_WAIT_X_FULL);
                     *abort_flag = 1;
                     ok = false;
                     break;
                 }
+                if (TRACE) dq_wait_raw += clock64() - tq;
                 const uint8_t* const raw = raw0 + pr.s * PAIR_RAW_BYTES;
                 const uint2 sc = *reinterpret_cast<const uint2*>(raw + PAIR_RAW_WQ_BYTES + r * 16u + 8u * half);
                 const uint32_t dst = tmem_base + ((32u * (warp & 3u)) << 16) + a_col0 + pw.s * 128u + 64u * half;
@@ -403,6 +406,7 @@ __device__ __forceinline__ void pair_gemm(const CUtensorMap& tmap_x, const CUten
                     }
                     uint4 o[8];
                     decode_row64(c0, c1, i ? sc.y : sc.x, g, o);
+                    if (TRACE && i == 0u) tq = clock64();
                     if (i == 0u && st >= SW) {
                         if (!joined) {                                       // first wait on a W stage: join the stream's order
                             grid_dependency_wait();
@@ -420,6 +424,7 @@ __device__ __forceinline__ void pair_gemm(const CUtensorMap& tmap_x, const CUten
                         }
                         pe.advance_by(2u, DN);
                     }
+                    if (TRACE && i == 0u) dq_wait_empty += clock64() - tq;
                     uint32_t v[32];
 #pragma unroll
                     for (uint32_t e = 0; e < 8; e++) {

@@ -658,7 +658,7 @@ int launch_one(lexb_gpu* g, const lexb_pipeline* p, const lexb_buffer* x, const 
     if (!p) return fail(LEXB_ERR_ARG, "null pipeline");
     if (p->gpu != g) return fail(LEXB_ERR_ARG, "pipeline was planned on another gpu handle");
     const bool fuses_silu = p->kernel == KERNEL_TCGEN05_PAIR && !p->residual;
-    if (p->few && !gather) p = p->few;
+    if (p->few && !gather && !(g->d_trace && p->grid <= g->trace_ctas)) p = p->few;      // (it has no phase timers)
     const size_t m = p->m, n = p->n, k = p->k;
     int rc;
     if ((rc = check_buf(x, g, m * k * (p->x_f32 ? 4 : 2), p->x_q16 ? "xq" : "x"))) return rc;
@@ -1929,9 +1929,11 @@ static lexb_route matvec_route(const MatvecShape& v) {
 int lexb_pipeline_route(const lexb_pipeline* p, lexb_route* out) {
     if (!p || !out) return fail(LEXB_ERR_ARG, "lexb_pipeline_route: null argument");
     *out = lexb_route{};
-    if (p->kernel == KERNEL_MATVEC) *out = matvec_route(p->mv);
+    const lexb_pipeline* l = p->few ? p->few : p;
+    if (l->kernel == KERNEL_MATVEC) *out = matvec_route(l->mv);
     else {
-        out->cluster = 1; out->blocks = p->grid; out->threads = p->threads;
+        out->cluster = l->cluster_split ? l->k_splits : l->cluster;
+        out->blocks = l->grid; out->threads = l->threads;
     }
     out->host_part = p->host_part;
     return LEXB_OK;
