@@ -12,7 +12,7 @@ def code(name):
     return re.sub(r"//[^\n]*", "", (CSRC / name).read_text())
 
 
-@pytest.mark.parametrize("name,barrier", [("gemm_fp4_sm100.cuh", "__syncthreads()"), ("gemm_fp4_sm100_pair.cuh", "cluster_sync_all()"),
+@pytest.mark.parametrize("name,barrier", [("gemm_fp4_sm100.cuh", "__syncthreads()"), ("gemm_fp4_sm100_pair.cuh", "cluster_sync_all()"), ("gemm_fp4_few_sm100.cuh", "__syncthreads()"),
                                           ("matmul_q_fp4_sm100.cuh", "bar.sync 2"), ("matmul_q_chain_sm100.cuh", "__syncthreads()")])
 def test_dependents_go_only_once_the_block_holds_its_tensor_memory(name, barrier):
     """A block that let the next launch start while it still waits for its columns could lose them to that launch, which
@@ -34,9 +34,24 @@ def test_dependents_go_only_once_the_block_holds_its_tensor_memory(name, barrier
 
 def test_the_cluster_barrier_brings_the_warp_together_first():
     """barrier.cluster.*.aligned must be executed by all lanes of a warp at once; the matvec meets it behind code whose lanes
-    part (tokens that do not exist, outputs that do not divide by the threads)."""
-    for name in ("sm100_ptx.cuh", "matvec_fp4_sm100.cuh", "gemm_fp4_sm100_pair.cuh"):
+    part (tokens that do not exist, outputs that do not divide by the threads), the kernels that sum within a cluster behind loops over
+    tokens: every barrier stands behind a __syncwarp of its own, or in cluster_sync_all, which has one."""
+    found = [path.name for path in sorted(CSRC.glob("*.cuh")) if "barrier.cluster" in code(path.name)]
+    assert "sm100_ptx.cuh" in found
+    for name in found:
         for at in re.finditer(r"barrier\.cluster\.(?:arrive|wait)[\w.]*\.aligned", code(name)):
             ahead = code(name)[:at.start()]
             last = max(ahead.rfind("__syncwarp()"), ahead.rfind("barrier.cluster"))
             assert last > ahead.rfind("__device__"), name
+
+
+@pytest.mark.parametrize("name", ["gemm_fp4_few_sm100.cuh", "matmul_q_fp4_sm100.cuh", "gemm_fp4_sm100_pair.cuh"])
+def test_a_block_whose_sums_others_read_waits_for_them(name):
+    """Sums in shared memory are read by the other blocks of a cluster: a barrier of the whole cluster before the first read and
+    one behind the last, before the block can end."""
+    text = code(name)
+    reads = [m.start() for m in re.finditer(r"ld_shared_cluster_f32x4\(", text)]
+    assert reads
+    before, behind = text.rfind("cluster_sync_all()", 0, reads[0]), text.find("cluster_sync_all()", reads[-1])
+    assert 0 < before and "tmem_ld_32x32b" not in text[before:reads[-1]]          # (all sums are stored by then)
+    assert reads[-1] < behind < text.index("tmem_dealloc", reads[-1])

@@ -13,7 +13,8 @@ import pytest
 import random
 
 
-def run(SX, SW, SR, KB, seed, DNmin, KS=1):
+def run(SX, SW, SR, KB, seed, DNmin, KS=1, paired=False):
+    """`paired`: the decode of two K steps a turn - eight warps take the even packed blocks, eight the odd ones (KS = 4)."""
     rnd = random.Random(seed)
     DN = max(SX, SW, DNmin)
     class Bar:
@@ -24,11 +25,13 @@ def run(SX, SW, SR, KB, seed, DNmin, KS=1):
             if s.pending == 0: s.pending = s.count; s.done += 1
         def test(s, parity): return (s.done & 1) != parity
     NST = KB // KS                       # stage steps: KS K steps of 64 columns each
-    full=[Bar(2+4*KS+1,f"full{j}") for j in range(DN)]
+    PW = 8 if paired else 4*KS           # decode warps that fill a stage
+    full=[Bar(2+PW+1,f"full{j}") for j in range(DN)]
     done=[[Bar(1,f"done{c}_{j}") for j in range(DN)] for c in range(2)]
-    wpart=[Bar(4*KS,f"wpart{j}") for j in range(SW)]
+    wpart=[Bar(PW,f"wpart{j}") for j in range(SW)]
     rawf=[[Bar(1,"rawf") for _ in range(SR)] for c in range(2)]
-    rawe=[[Bar(16,"rawe") for _ in range(SR)] for c in range(2)]
+    rawe=[[Bar(8 if paired else 16,"rawe") for _ in range(SR)] for c in range(2)]
+    in_flight=[[],[]]
     mma_done=[-1]      # highest K step whose MMAs completed
     errors=[]
     # ground-truth state for checking
@@ -50,14 +53,20 @@ def run(SX, SW, SR, KB, seed, DNmin, KS=1):
     def rawprod(c):
         for rb in range(KB//4):
             if rb >= SR:
-                yield from wait(rawe[c][rb%SR], ((rb-SR)//SR)&1, lambda: True, "rawe")
+                yield from wait(rawe[c][rb%SR], ((rb-SR)//SR)&1, lambda: rawe[c][rb%SR].done >= rb//SR, "rawe")
             yield
-            rawf[c][rb%SR].arrive()
+            in_flight[c].append(rb)
+    def land(c):                     # copies land in any order
+        for _ in range(KB//4):
+            while not in_flight[c]: yield
+            for _ in range(rnd.randint(0,8)): yield
+            rawf[c][in_flight[c].pop(rnd.randrange(len(in_flight[c])))%SR].arrive()
+            yield
     def dec(c, w):
         q = w>>2
-        for kb in range(q, KB, 4):
+        for kb in (range(4*(q>>1), KB, 8) if paired else range(q, KB, 4)):
             rb = kb//4
-            yield from wait(rawf[c][rb%SR], (rb//SR)&1, lambda: True, "rawf")
+            yield from wait(rawf[c][rb%SR], (rb//SR)&1, lambda: rawf[c][rb%SR].done > rb//SR, f"dec{c}.{w} rawf({rb})")
             yield
             rawe[c][rb%SR].arrive()
             for _ in range(rnd.randint(0,6)): yield
@@ -78,17 +87,17 @@ def run(SX, SW, SR, KB, seed, DNmin, KS=1):
                 wpart[st%SW].arrive()
     def relay():
         for kb in range(NST):
-            yield from wait(wpart[kb%SW], (kb//SW)&1, lambda kb=kb: wslot[1][kb%SW]==(kb,4*KS), f"relay kb={kb}")
+            yield from wait(wpart[kb%SW], (kb//SW)&1, lambda kb=kb: wslot[1][kb%SW]==(kb,PW), f"relay kb={kb}")
             yield
             full[kb%DN].arrive()
     def mma():
         for kb in range(NST):
-            yield from wait(full[kb%DN], (kb//DN)&1, lambda kb=kb: wslot[0][kb%SW]==(kb,4*KS) and wslot[1][kb%SW]==(kb,4*KS) and xslot[0][kb%SX]==kb and xslot[1][kb%SX]==kb, f"mma kb={kb}")
+            yield from wait(full[kb%DN], (kb//DN)&1, lambda kb=kb: wslot[0][kb%SW]==(kb,PW) and wslot[1][kb%SW]==(kb,PW) and xslot[0][kb%SX]==kb and xslot[1][kb%SX]==kb, f"mma kb={kb}")
             for _ in range(rnd.randint(0,3)): yield
             mma_done[0]=kb
             done[0][kb%DN].arrive(); done[1][kb%DN].arrive()
             yield
-    actors=[xprod(0),xprod(1),rawprod(0),rawprod(1),relay(),mma()]+[dec(c,w) for c in range(2) for w in range(16)]
+    actors=[xprod(0),xprod(1),rawprod(0),rawprod(1),land(0),land(1),relay(),mma()]+[dec(c,w) for c in range(2) for w in range(16)]
     weights=[rnd.random()+0.05 for _ in actors]
     live=list(range(len(actors)))
     steps=0
@@ -124,3 +133,17 @@ def test_protocol_is_safe_with_four_k_steps_per_stage(sx, sw):
 def test_a_shallower_barrier_ring_lets_a_parity_wait_pass_early():
     found = [e for seed in range(12) for e in run(2, 2, 2, 24, seed, 1)]
     assert any(e.startswith("false pass") for e in found)
+
+
+@pytest.mark.parametrize("sx,sw,sr", [(3, 3, 5), (2, 3, 5), (3, 2, 4), (2, 2, 4), (3, 3, 6)])
+@pytest.mark.parametrize("blocks", [1, 2, 7, 12])
+def test_protocol_is_safe_with_two_k_steps_a_turn(sx, sw, sr, blocks):
+    """Even and odd packed blocks by two sets of eight warps, packed blocks two more than W stages (pair_paired)."""
+    for seed in range(4):
+        assert run(sx, sw, sr, 4 * blocks, seed, 4, KS=4, paired=True) == []
+
+
+def test_fewer_packed_blocks_let_a_set_pass_a_parity_wait_early():
+    """A set passes over every second packed block; with three of them and three W stages it can find a barrier two phases behind."""
+    found = [e for seed in range(40) for e in run(3, 3, 3, 48, seed, 4, KS=4, paired=True)]
+    assert any(e.startswith("false pass: dec") for e in found)
