@@ -258,7 +258,7 @@ def run_ours(args):
 
     # ---- headline: m = 512 GEMM
     pipe = gpu.plan_gemm_fp4(M, n_local, K)
-    desc = pipe.describe()
+    desc, route = pipe.describe(), pipe.route()
 
     def gemm_step(i):
         _, bufs = weights[i % COPIES]
@@ -756,7 +756,8 @@ def run_ours(args):
                            "k_splits": desc.k_splits,
                            "l2": f"{COPIES} weight copies rotated per step ({COPIES * wbytes_local / 1e6:.0f} MB per GPU > L2)",
                            "schedule": {"bm": desc.bm, "bn": desc.bn, "bk": desc.bk, "stages": desc.stages,
-                                        "grid": desc.grid, "threads": desc.threads, "smem": desc.threadgroup_bytes}},
+                                        "grid": desc.grid, "threads": desc.threads, "smem": desc.threadgroup_bytes},
+                           "launch": {"blocks": route.blocks, "threads": route.threads, "cluster": route.cluster}},
                 "roofline": roofline, "cpu_baseline": info, "e2e": e2e, "gpu_launches": args.steps,
                 "clocks": clocks, "matvec": matvec, "allgather": allgather, "device_status": status,
                 "checksum": checksum, "only": args.only, "stack_m4096": stack, "parity": parity, "sustained": sustained,

@@ -228,11 +228,13 @@ LEXB_API int lexb_gemm_fp4_enqueue_host(lexb_gpu* gpu, const lexb_pipeline* p, c
 /* Gpu::run_launches, crates/lex-cuda/src/device.rs:650-672: all steps, one synchronise;
  * cpu_s = host time to enqueue, wall_s = host time until the device is idle.
  * The results are those of the steps run one after another.  Consecutive lexb_matmul_fp4_plan steps of t <= 8
- * tokens planned with k_splits = 1 (and without LEXB_SCHED_WEIGHTS_MAY_CHANGE), with the same t, k
- * and activation type, of which none reads or overwrites a buffer that an earlier one of them touches (x, r,
- * wq, ws and wg not written, y neither read nor written: the address ranges are compared; wq, ws and wg must also be
- * untouched by every earlier step of the call, or declared constant), are run as ONE persistent kernel
- * over all their row tiles (the gate/up pair, q/k/v); each result is bit-identical to the step launched alone.
+ * tokens with the same t and activation type (n and k may differ; without LEXB_SCHED_WEIGHTS_MAY_CHANGE), whose K
+ * is whole or split by the planner (not by the caller, unless k_splits = 1), and of which none reads or overwrites a
+ * buffer that an earlier one of them touches (x, r, wq, ws and wg not written, y neither read nor written: the address
+ * ranges are compared; wq, ws and wg must also be untouched by every earlier step of the call, or declared constant),
+ * are run as ONE persistent kernel over all their row tiles (gate/up, q/k/v, down of another layer).  Steps whose K the
+ * planner split join where that is the faster way by the library's prices: a run spreads no tile's K over blocks, so
+ * a few narrow steps with a long K are left to launches of their own.  Each result is bit-identical to the step launched alone.
  * A step that depends on the run starts a new launch.  The environment variable LEXB_CHAIN=0 turns this off. */
 LEXB_API int lexb_run_launches(lexb_gpu* gpu, const lexb_step* steps, size_t nsteps, double* cpu_s, double* wall_s);
 /* How lexb_run_launches would issue this list, without launching anything: run_len_out[i] = number of steps of

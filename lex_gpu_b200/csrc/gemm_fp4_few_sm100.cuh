@@ -10,7 +10,8 @@
 // boundary every share leaves its sums in shared memory, and after the last segment - one barrier across the cluster - the
 // blocks that have a part of it add the parts in the order of K, straight from one another's shared memory, and store y.
 // Nothing of it passes through global memory, no block waits for another before that barrier, and a launch needs no
-// workspace.  The cuts depend on n, k and the cluster alone, so a token's bits do not depend on its batch.
+// workspace.  The cuts depend on n, k and the cluster; the cluster, the number of accumulators (8, 4 or 2) and the choice of this kernel
+// depend on the number of tokens, so a token's last bits may depend on its batch, as in the two-CTA kernel's plans.
 //
 // Roles (736 threads): warps 0-15 decode - eight take the even blocks of weights, eight the odd ones, a warp 32 rows and two of
 // the four K steps (64 columns each), a row a thread - into tensor memory, from where the MMAs take them as their A operand (M = 128 rows); warps
@@ -18,8 +19,9 @@
 // the MMAs (N = 16, 32 or 64 tokens).
 //
 // What bounds it: the decode warps' turns, half decode (560 of 1450 clocks a K step when a turn was one K step) and half barriers,
-// stores and fences; without the decode 28672 x 4096 takes 21.6 us at 32 tokens, without the MMAs 29.3, with everything 32.0 and, with
-// two K steps a turn, 28.0 (the two-CTA kernel: 41.2; the bytes alone 10.7).  17408 x 5120 at 64 tokens: 24.9 -> 20.0 us.
+// stores and fences; without the decode 28672 x 4096 took 21.6 us at 32 tokens, without the MMAs 29.3, with everything 32.0 and, with
+// two K steps a turn, 29.4 in whole calls (the two-CTA kernel: 41.2; the bytes alone 10.7).  17408 x 5120 at 16 / 32 / 64 tokens: 18.9 /
+// 19.4 / 20.7 us (64 by the two-CTA kernel: 24.9).
 //
 // Tensor memory: columns 0-255 two sets of accumulators (segments alternate), 128 columns each: 8, 4 or 2 accumulators of N
 // columns that take the K steps in turn, so that each has an eighth, a quarter or half of the truncating additions; columns

@@ -598,10 +598,12 @@ struct PairPrices {
     double start, kstep[4], wave[4], store, reduce, reduce_mb, cluster, cluster_mb;
     uint32_t least;
 };
-// Fitted to 4,466 launches of 487 shapes (m = 9-2048, n = 128-28672, k = 256-17408) on a B200: rms error 5 %, the form chosen takes
-// 0.8 % more than the fastest in the mean, where the prices before (159 launches with the table decode) took 9 % more.  Past 10
-// GFLOP of more than 64 tokens a launch that is repeated runs into the power cap, which bursts of launches do not show (1572 x 6656 x
-// 1024 with down behind it: 62.4 us by the prices before, 64.6 by these), and these gain 1 % at most: those prices stay there.
+// Fitted to 4,466 launches of 487 shapes (m = 9-2048, n = 128-28672, k = 256-17408) on a B200, before tiles of 128 and 64 tokens were
+// decoded two K steps a turn: rms error 5 % then, the form chosen 0.8 % above the fastest in the mean (the prices before, 159 launches
+// with the table decode: 9 %).  A K step of those tiles now takes 0.23 us (17408 x 5120, m = 128: 23.3 us), not the 0.319 here, so they
+// and their splits are priced too dear against tiles of 256 tokens and the few-token kernel; not fitted again.  Past 10 GFLOP of more
+// than 64 tokens the prices of the table decode: a launch that is repeated runs into the power cap, which bursts do not show; the line
+// rests on one shape (1572 x 6656 x 1024 with down behind it: 62.4 us by them, 64.6 by FITTED), and plans jump across it.
 const PairPrices& pair_prices(uint32_t m, uint32_t n, uint32_t k) {
     static const PairPrices FITTED = {0.20, {0.598, 0.337, 0.319, 0.319}, {7.69, 5.85, 4.46, 3.70}, 0.157, 1.04, 0.288, 0.25, 0.271, 2u},
                             LARGE = {4.51, {0.559, 0.311, 0.310, 0.304}, {8.05, 5.32, 4.02, 4.14}, 0.0, -1.12, 0.300, -1.12, 0.300, 4u};
@@ -889,8 +891,8 @@ int launch_one(lexb_gpu* g, const lexb_pipeline* p, const lexb_buffer* x, const 
 }
 
 // Consecutive steps of a list that can run as one persistent kernel (matmul_q_chain_sm100.cuh): block-scaled
-// matmul_q of up to 8 tokens with the default ring depth and digit-row source of their token count, one K range per block, the same
-// t, k and activation type (n may differ), weights declared constant.  LEXB_CHAIN=0 turns it off.
+// matmul_q of up to 8 tokens with the default ring depth and digit-row source of their token count, the same t and activation type
+// (n and k may differ), K whole or split by the planner, weights declared constant or untouched by the list so far.  LEXB_CHAIN=0 turns it off.
 // (two accumulator sets of 2 x 64 columns: 8 tokens x 8 digit rows)
 static uint32_t chain_max_m() {
     static const uint32_t v = env_u32("LEXB_CHAIN_MAX_M", lexb::MQC_MAX_TOKENS);
@@ -1699,8 +1701,8 @@ int lexb_gemm_fp4_plan(lexb_gpu* g, uint32_t m, uint32_t n, uint32_t k, int resi
         p->m_tiles = (m + p->tm - 1) / p->tm;
         const uint32_t n_pairs = (n + 2u * lexb::GEMM_TN - 1) / (2u * lexb::GEMM_TN);
         // Two ways to fill the SM pairs when whole tiles fill them badly (few tiles, or a short last wave).  Split K:
-        // each split takes whole blocks of 256 columns (at least 4) and writes a partial product that a second
-        // launch sums.  Smaller tiles: more of them; every weight is decoded once per tile of tokens, but a tile's
+        // each split takes whole blocks of 256 columns (PairPrices' `least` of them, or more) and leaves a partial product, summed by a
+        // second launch or within a cluster.  Smaller tiles: more of them; every weight is decoded once per tile of tokens, but a tile's
         // partial product and its store shrink with it and fewer splits are needed.  (Below 256 tokens a K step
         // costs about the same: it is the decode that bounds it, not the MMAs.)
         // Every (tile, splits) pair is priced (PairPrices), the cheapest wins; a smaller tile or a further split must win by 2 %.

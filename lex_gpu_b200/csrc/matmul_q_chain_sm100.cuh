@@ -9,7 +9,8 @@
 // to the block with the fewest stages so far: every SM has work whatever the steps' tile counts are (136 tiles of
 // n = 17408 leave 12 of 148 SMs idle in a launch of their own, 224 tiles of n = 28672 need two waves), steps of several K
 // share a launch, and a block's rings never drain: the copy engine is into the next tile's weights while this tile's last stages
-// are multiplied and stored.  Nothing orders the tiles of different blocks, so the host only puts a step into a
+// are multiplied and stored.  (A tile's K stays in one block: a few narrow steps are left to launches of their own, run_that_pays.)
+// Nothing orders the tiles of different blocks, so the host only puts a step into a
 // run if nothing it reads (x, r) is written, and nothing it writes (y) read or written, by a step already in the
 // run (it compares the buffers' address ranges); a step that does depend on the run starts a new launch, and
 // the stream orders it as usual.  (A version that waited inside the kernel - every block counts itself in after
