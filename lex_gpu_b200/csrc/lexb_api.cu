@@ -975,12 +975,12 @@ uint32_t chain_part(const lexb_pipeline* p) { return p->k_splits == 1u ? p->k / 
 // Of the first `len` steps of a list, which one launch can take: how many it should.  Steps whose plans keep K whole always share it.
 // The parts of a split K stay in one block of a run, where the step's own launch spreads them: two steps of 640 x 17408 are 10 blocks
 // of 68 stages there and 40 blocks of 9 alone (48 us and 30), three 27B layers 106 us and 160.  So a run with split plans is priced
-// against its steps' own launches, with the number of steps with which it and what is left cost least.  Fitted to 150 lists timed both ways (2-6
-// steps, t = 1-8, n = 128-20480, k = 512-17408; median error 3 % and 6 %), us: a run 12.4 and 0.546 per stage of its fullest block; a
-// list 5.2, a step of it 3.2, 0.536 per stage of each wave of blocks, 1.2 for a split, the walk over the tokens for their digits, in
-// front of the product past 4 tokens.  A run is given up where it costs a tenth more.  On 100 other lists the way taken takes 0.997 of
-// the faster of the two whole ways in the mean and 1.06 at most; every run taken, 1.02 and 1.9.  LEXB_CHAIN_SPLITS=1: it is taken
-// whatever it costs.
+// against its steps' own launches, with the number of steps with which it and what is left cost least.  Fitted to 150 lists timed both
+// ways (2-6 steps, t = 1-8, n = 128-20480, k = 512-17408; median error 3 % and 6 %), us: a run 12.4 and 0.546 per stage of its fullest
+// block; a list 5.2, a step of it 3.2, 0.536 per stage of each wave of blocks, 1.2 for a split, the walk over the tokens for their
+// digits, in front of the product past 4 tokens.  A run is given up where it costs a tenth more.  On 100 other lists the way taken takes
+// 0.997 of the faster of the two whole ways in the mean and 1.06 at most; every run taken, 1.02 and 1.9.  LEXB_CHAIN_SPLITS=1: it is
+// taken whatever it costs.
 size_t run_that_pays(const lexb_step* steps, size_t len, uint32_t sms) {
     size_t unsplit = 0;
     while (unsplit < len && steps[unsplit].pipeline->k_splits == 1u) unsplit++;
